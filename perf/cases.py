@@ -224,3 +224,98 @@ def tolerance(case):
     the listed cases (batch reduced to 2, lengths to 8192): bf16 2.0e-3 to 2.8e-3 relative and at most 0.087 in one
     element, fp16 2.5e-4 to 3.1e-4 and at most 0.012."""
     return {"rel": 0.011, "max": 0.35} if case["dtype"] == "bf16" else {"rel": 0.00125, "max": 0.047}
+
+
+def _attend(q, k, v, causal, left, right, dout=None):
+    """One sequence in 64 bits, heads first: q (H, sq, D), k, v (Hk, sk, D).  out, and with dout also dq, dk, dv."""
+    H, sq, D = q.shape
+    Hk, sk, _ = k.shape
+    out, dq = torch.empty_like(q), torch.empty_like(q)
+    dk, dv = torch.zeros_like(k), torch.zeros_like(v)
+    cols, scale = torch.arange(sk, device=q.device), 1 / math.sqrt(D)
+    right = 0 if causal else right
+    step = max(1, (1 << 26) // max(1, sk))
+    for h in range(H):
+        g = h // (H // Hk)
+        for i in range(0, sq, step):
+            at = torch.arange(i, min(sq, i + step), device=q.device) + (sk - sq)
+            e = slice(i, i + len(at))
+            s = (q[h, e] @ k[g].T) * scale
+            if right >= 0:
+                s.masked_fill_(cols > at[:, None] + right, -math.inf)
+            if left >= 0:
+                s.masked_fill_(cols < at[:, None] - left, -math.inf)
+            p = torch.softmax(s, -1).nan_to_num_(0.0)  # a row without a key gives zero
+            del s
+            out[h, e] = p @ v[g]
+            if dout is not None:
+                dv[g] += p.T @ dout[h, e]
+                ds = dout[h, e] @ v[g].T
+                ds -= (dout[h, e] * out[h, e]).sum(-1, keepdim=True)
+                ds *= p
+                dq[h, e] = (ds @ k[g]) * scale
+                dk[g] += (ds.T @ q[h, e]) * scale
+                del ds
+            del p
+    return (out,) if dout is None else (out, dq, dk, dv)
+
+
+def _turn(x, cos, sin, pos):
+    """Rows of x (n, h, D) turned to the positions pos (n): the first half of a row against the second."""
+    c, s = cos[pos].double()[:, None], sin[pos].double()[:, None]
+    a, b = x.chunk(2, -1)
+    return torch.cat([a * c - b * s, a * s + b * c], -1)
+
+
+def exact(case, seed):
+    """What run() returns for these inputs, in 64 bits with plain torch.  The caches are left out where they are large:
+    all but their new rows is input."""
+    s = prepare(case, seed)
+    heads_first = lambda t: t.detach().double().transpose(0, 1)  # noqa: E731
+    left, right = s["window"]
+    if case["kind"] == "cache":
+        out, new, cap = torch.empty(s["q"].shape, dtype=torch.float64, device="cuda"), case["new"], case["sk"]
+        whole = s["kc"].numel() <= 1 << 26
+        kc, vc = (s["kc"].double(), s["vc"].double()) if whole else (None, None)
+        for b, n in enumerate(s["lens"].tolist()):
+            pos = torch.arange(n, n + new, device="cuda")
+            q, k, v = s["q"][b].double(), s["k"][b].double(), s["v"][b].double()
+            if s["cos"] is not None:
+                q, k = _turn(q, s["cos"], s["sin"], pos), _turn(k, s["cos"], s["sin"], pos)
+            if s["table"] is None:
+                old_k, old_v = s["kc"][b, :n], s["vc"][b, :n]
+            else:
+                pages = s["table"][b].long()
+                old_k, old_v = s["kc"][pages].flatten(0, 1)[:n], s["vc"][pages].flatten(0, 1)[:n]
+            if whole:
+                at = (b, pos) if s["table"] is None else (pages[pos // case["page"]], pos % case["page"])
+                kc[at], vc[at] = k, v
+            k, v = torch.cat([old_k.double(), k]), torch.cat([old_v.double(), v])
+            out[b] = _attend(q.transpose(0, 1), k.transpose(0, 1), v.transpose(0, 1), case["causal"], left, right)[0].transpose(0, 1)
+        return out, kc, vc
+    if case["kind"] == "varlen":
+        parts, ends = [], s["cu"].tolist()
+        for i, j in zip(ends, ends[1:]):
+            q, k, v, d = (heads_first(t[i:j]) for t in s["in"] + [s["dout"]])
+            parts.append([t.transpose(0, 1) for t in _attend(q, k, v, case["causal"], left, right, d)])
+        return tuple(torch.cat(t) for t in zip(*parts))
+    if case["pack"] == "qkv":
+        q, k, v = s["in"][0].unbind(2)
+    elif case["pack"] == "kv":
+        q, (k, v) = s["in"][0], s["in"][1].unbind(2)
+    else:
+        q, k, v = s["in"]
+    dout = s.get("dout")
+    parts = []
+    for b in range(case["batch"]):
+        d = None if dout is None else heads_first(dout[b])
+        parts.append([t.transpose(0, 1) for t in _attend(heads_first(q[b]), heads_first(k[b]), heads_first(v[b]), case["causal"], left, right, d)])
+    got = [torch.stack(t) for t in zip(*parts)]
+    if dout is None:
+        return got[0]
+    out, dq, dk, dv = got
+    if case["pack"] == "qkv":
+        return out, torch.stack([dq, dk, dv], 2)
+    if case["pack"] == "kv":
+        return out, dq, torch.stack([dk, dv], 2)
+    return out, dq, dk, dv
