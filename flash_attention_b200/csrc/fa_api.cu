@@ -126,6 +126,37 @@ static int refuse_if_device_failed() {
   return 0;
 }
 
+static int splits_by_wave_efficiency(int batch, int heads, int seqlen_q, int seqlen_k, int head_dim, int num_sms) {
+  // For the any-shape kernel: the search of num_splits_heuristic (flash_api.cpp:206-246) on work items of 256
+  // query rows (128 above head dim 128) and 128-key blocks: with enough items to fill 80 % of the SMs do not split; otherwise take the smallest
+  // split count within 85 % of the best wave efficiency.
+  const int rows = head_dim > 128 ? 128 : 256;
+  const int m_blocks = (seqlen_q + rows - 1) / rows, n_blocks = (seqlen_k + 127) / 128;
+  const int ctas = batch * heads * m_blocks;
+  if (ctas >= 0.8f * num_sms) return 1;
+  int max_splits = 128;
+  if (num_sms < max_splits) max_splits = num_sms;
+  if (n_blocks < max_splits) max_splits = n_blocks;
+  if (max_splits < 1) max_splits = 1;
+  auto blocks_per = [&](int s) { return (n_blocks + s - 1) / s; };
+  float best = 0.f;
+  float eff[129];
+  for (int s = 1; s <= max_splits; ++s) {
+    bool eligible = s == 1 || blocks_per(s) != blocks_per(s - 1);
+    if (!eligible) {
+      eff[s] = 0.f;
+      continue;
+    }
+    float waves = float(ctas) * s / num_sms;
+    float e = waves / ceilf(waves);
+    eff[s] = e;
+    if (e > best) best = e;
+  }
+  for (int s = 1; s <= max_splits; ++s)
+    if (eff[s] >= 0.85f * best && eff[s] > 0.f) return s;
+  return 1;
+}
+
 extern "C" {
 
 const char* fa_last_error(void) { return fa_host::g_err; }
@@ -164,36 +195,26 @@ int fa_abi_struct_size(int32_t which) {
 
 int fa_fwd_num_splits(int32_t batch, int32_t heads, int32_t seqlen_q, int32_t seqlen_k, int32_t head_dim,
                       int32_t num_sms) {
-  // Same search as num_splits_heuristic (flash_api.cpp:206-246) on this library's tile sizes (a work
-  // item of the tensor-core kernel is 256 query rows, 128 above head dim 128, and walks 128-key
-  // blocks): with enough items to fill 80 % of the SMs do not split; otherwise take the smallest
-  // split count within 85 % of the best wave efficiency.
+  // For the tensor-core kernel (a work item is 256 query rows, 128 above head dim 128, and walks 128-key blocks): the
+  // split count with the least estimated time.  A block takes about 2 us, a round of CTAs 5 us before and after its
+  // blocks, merging the parts 5 us and what writing and reading their fp32 rows takes at 5 TB/s.  On 2 x 512 x 8 x 64,
+  // where a split into single blocks fills the SMs, that split took 9.2 + 6.2 us.
   if (num_sms <= 0) num_sms = fa_host::sm_count();
   const int rows = head_dim > 128 ? 128 : 256;
-  const int m_blocks = (seqlen_q + rows - 1) / rows, n_blocks = (seqlen_k + 127) / 128;
-  const int ctas = batch * heads * m_blocks;
+  const int64_t ctas = (int64_t)batch * heads * ((seqlen_q + rows - 1) / rows);
+  const int n_blocks = (seqlen_k + 127) / 128;
   if (ctas >= 0.8f * num_sms) return 1;
-  int max_splits = 128;
-  if (num_sms < max_splits) max_splits = num_sms;
-  if (n_blocks < max_splits) max_splits = n_blocks;
-  if (max_splits < 1) max_splits = 1;
-  auto blocks_per = [&](int s) { return (n_blocks + s - 1) / s; };
-  float best = 0.f;
-  float eff[129];
-  for (int s = 1; s <= max_splits; ++s) {
-    bool eligible = s == 1 || blocks_per(s) != blocks_per(s - 1);
-    if (!eligible) {
-      eff[s] = 0.f;
-      continue;
+  const float part_us = (float)batch * heads * seqlen_q * head_dim * 8.f / 5e6f;
+  int best = 1;
+  float best_time = 5.f + 2.f * n_blocks;
+  for (int s = 2; s <= n_blocks && s <= 128; ++s) {
+    const float t = (float)((ctas * s + num_sms - 1) / num_sms) * (5.f + 2.f * ((n_blocks + s - 1) / s)) + 5.f + s * part_us;
+    if (t < best_time) {
+      best_time = t;
+      best = s;
     }
-    float waves = float(ctas) * s / num_sms;
-    float e = waves / ceilf(waves);
-    eff[s] = e;
-    if (e > best) best = e;
   }
-  for (int s = 1; s <= max_splits; ++s)
-    if (eff[s] >= 0.85f * best && eff[s] > 0.f) return s;
-  return 1;
+  return best;
 }
 
 int64_t fa_bwd_workspace_bytes(int32_t batch, int32_t seqlen_q, int32_t heads, int32_t head_dim, int32_t total_q,
@@ -322,7 +343,7 @@ int fa_kvcache_plan(const FaKvcacheArgs* a, int32_t num_sms, int64_t* lse_accum_
     splits = fa::decode_plan(*a, num_sms);
   } else {
     splits = a->num_splits;
-    if (splits == 0) splits = fa_fwd_num_splits(a->batch, a->heads, a->seqlen_q, a->seqlen_cache, a->head_dim, num_sms);
+    if (splits == 0) splits = splits_by_wave_efficiency(a->batch, a->heads, a->seqlen_q, a->seqlen_cache, a->head_dim, num_sms);
   }
   if (splits < 1) splits = 1;
   int64_t rows = (int64_t)a->batch * a->heads * a->seqlen_q;
