@@ -24,6 +24,8 @@ int kvcache_prep(const FaKvcacheArgs& a, int q_follows_rows, cudaStream_t st);
 // tcgen05 kernels (sm100/)
 bool fwd_tc_eligible(const FaFwdArgs& a);
 int fwd_tc(const FaFwdArgs& a, cudaStream_t st);
+bool fwd_tc_cache_eligible(const FaFwdArgs& a, int64_t kv_batches);
+int fwd_tc_cache(const FaFwdArgs& a, int64_t kv_batches, cudaStream_t st);
 bool bwd_tc_eligible(const FaBwdArgs& a);
 int bwd_tc_main(const FaBwdArgs& a, cudaStream_t st);
 // fused single-token decode
@@ -335,6 +337,65 @@ static int kvcache_checks(const FaKvcacheArgs* a) {
   return 0;
 }
 
+}  // extern "C"
+
+// The attention of a KV-cache call whose new tokens have been appended (and whose q has been rotated) by kvcache_prep.
+static FaFwdArgs cache_fwd_args(const FaKvcacheArgs& a, int splits) {
+  FaFwdArgs f;
+  memset(&f, 0, sizeof(f));
+  if (a.rotary_cos) {
+    f.q.ptr = a.q_rotated;
+    f.q.stride_h = a.head_dim;
+    f.q.stride_s = (int64_t)a.heads * a.head_dim;
+    f.q.stride_b = (int64_t)a.seqlen_q * a.heads * a.head_dim;
+  } else {
+    f.q = a.q;
+  }
+  f.k = a.kcache;
+  f.v = a.vcache;
+  f.out = a.out;
+  f.softmax_lse = a.softmax_lse;
+  f.lse_seqlen = a.seqlen_q;
+  f.batch = a.batch;
+  f.seqlen_q = a.seqlen_q;
+  f.seqlen_k = a.seqlen_cache;
+  f.heads = a.heads;
+  f.heads_k = a.heads_k;
+  f.head_dim = a.head_dim;
+  f.dtype = a.dtype;
+  f.softmax_scale = a.softmax_scale;
+  f.window_left = a.window_left;
+  f.window_right = a.window_right;
+  f.seqused_k = a.cache_seqlens;
+  f.seqused_k_extra = a.knew.ptr ? a.seqlen_new : 0;
+  f.kv_batch_idx = a.cache_batch_idx;
+  f.block_table = a.block_table;
+  f.block_table_stride = a.block_table_stride;
+  f.page_block_size = a.page_block_size;
+  f.num_splits = splits;
+  f.lse_accum = a.lse_accum;
+  f.out_accum = a.out_accum;
+  return f;
+}
+
+static bool cache_on_tensor_cores(const FaKvcacheArgs& a) {
+  return !fa_host::env_flag("FA_B200_FORCE_GENERIC") && fa::fwd_tc_cache_eligible(cache_fwd_args(a, 1), a.batch_cache);
+}
+
+// Splits of a multi-token call on the tensor-core kernel.  The lengths are on the device, so the plan knows the capacity
+// only: enough parts for about two rounds of CTAs over the SMs, so that a long sequence next to short ones does not set
+// the time alone, but no part under 4 key blocks of the capacity.
+static int cache_tc_splits(const FaKvcacheArgs& a, int num_sms) {
+  const int group = a.heads / a.heads_k, rows = a.head_dim > 128 ? 128 : 256;
+  const int64_t ctas = (int64_t)a.batch * a.heads_k * (((int64_t)a.seqlen_q * group + rows - 1) / rows);
+  int64_t s = (2 * num_sms + ctas - 1) / ctas;
+  const int64_t most = (a.seqlen_cache + 511) / 512;
+  s = s < most ? s : most;
+  return (int)(s < 1 ? 1 : s > 128 ? 128 : s);
+}
+
+extern "C" {
+
 int fa_kvcache_plan(const FaKvcacheArgs* a, int32_t num_sms, int64_t* lse_accum_bytes, int64_t* out_accum_bytes) {
   if (kvcache_checks(a)) return -1;
   if (num_sms <= 0) num_sms = fa_host::sm_count();
@@ -343,6 +404,7 @@ int fa_kvcache_plan(const FaKvcacheArgs* a, int32_t num_sms, int64_t* lse_accum_
     splits = fa::decode_plan(*a, num_sms);
   } else {
     splits = a->num_splits;
+    if (splits == 0 && cache_on_tensor_cores(*a)) splits = cache_tc_splits(*a, num_sms);
     if (splits == 0) splits = splits_by_wave_efficiency(a->batch, a->heads, a->seqlen_q, a->seqlen_cache, a->head_dim, num_sms);
   }
   if (splits < 1) splits = 1;
@@ -367,48 +429,16 @@ int fa_fwd_kvcache(const FaKvcacheArgs* a, fa_stream_t stream) {
     g_last_path = splits > 1 ? "decode+combine" : "decode";
     return fa::decode_run(*a, splits, st);
   }
-  g_last_path = splits > 1 ? "kvcache_prep+fwd_generic+combine" : "kvcache_prep+fwd_generic";
-
-  // General path: append/rotate in a first launch, then the any-shape forward on the cache.
+  // General path: append/rotate in a first launch, then the forward on the cache.
+  const bool tc = cache_on_tensor_cores(*a);
+  g_last_path = tc ? (splits > 1 ? "kvcache_prep+fwd_tc+combine" : "kvcache_prep+fwd_tc")
+                   : (splits > 1 ? "kvcache_prep+fwd_generic+combine" : "kvcache_prep+fwd_generic");
   const bool causal_or_local = a->window_left >= 0 || a->window_right >= 0;
   FA_REQUIRE(!a->rotary_cos || a->q_rotated, "rotary needs the q_rotated scratch buffer");
   int rc = fa::kvcache_prep(*a, (causal_or_local && !a->q_rows_share_position) ? 1 : 0, st);
   if (rc) return rc;
-  FaFwdArgs f;
-  memset(&f, 0, sizeof(f));
-  if (a->rotary_cos) {
-    f.q.ptr = a->q_rotated;
-    f.q.stride_h = a->head_dim;
-    f.q.stride_s = (int64_t)a->heads * a->head_dim;
-    f.q.stride_b = (int64_t)a->seqlen_q * a->heads * a->head_dim;
-  } else {
-    f.q = a->q;
-  }
-  f.k = a->kcache;
-  f.v = a->vcache;
-  f.out = a->out;
-  f.softmax_lse = a->softmax_lse;
-  f.lse_seqlen = a->seqlen_q;
-  f.batch = a->batch;
-  f.seqlen_q = a->seqlen_q;
-  f.seqlen_k = a->seqlen_cache;
-  f.heads = a->heads;
-  f.heads_k = a->heads_k;
-  f.head_dim = a->head_dim;
-  f.dtype = a->dtype;
-  f.softmax_scale = a->softmax_scale;
-  f.window_left = a->window_left;
-  f.window_right = a->window_right;
-  f.seqused_k = a->cache_seqlens;
-  f.seqused_k_extra = a->knew.ptr ? a->seqlen_new : 0;
-  f.kv_batch_idx = a->cache_batch_idx;
-  f.block_table = a->block_table;
-  f.block_table_stride = a->block_table_stride;
-  f.page_block_size = a->page_block_size;
-  f.num_splits = splits;
-  f.lse_accum = a->lse_accum;
-  f.out_accum = a->out_accum;
-  rc = fa::fwd_generic(f, st);
+  const FaFwdArgs f = cache_fwd_args(*a, splits);
+  rc = tc ? fa::fwd_tc_cache(f, a->batch_cache, st) : fa::fwd_generic(f, st);
   if (rc) return rc;
   if (splits > 1)
     return fa::combine(a->out_accum, a->lse_accum, a->out, a->softmax_lse, a->seqlen_q, splits, a->batch, a->heads,

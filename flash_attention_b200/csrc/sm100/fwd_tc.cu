@@ -58,7 +58,7 @@ constexpr int kBN = 128;  // keys per K/V tile
 constexpr int kChunkBytes = 128 * 128;  // [128 rows][64 x 16-bit]: one swizzled TMA box
 constexpr float kRescaleThreshold = 8.f;
 
-enum WaitCode { W_QFULL = 11, W_KVFULL = 12, W_KVEMPTY = 13, W_SFULL = 14, W_PFULL = 15, W_OFULL = 16 };
+enum WaitCode { W_QFULL = 11, W_KVFULL = 12, W_KVEMPTY = 13, W_SFULL = 14, W_PFULL = 15, W_OFULL = 16, W_VTAIL = 17 };
 
 template <int DH>
 struct Cfg {
@@ -69,7 +69,7 @@ struct Cfg {
   static constexpr int NT = DH > 128 ? 1 : 2;
   static constexpr int STAGES = DH > 128 ? 2 : (DH == 128 ? 4 : 8);
   static constexpr int SMEM_TILES = (NT + STAGES) * TILE_BYTES;
-  static constexpr int NBAR = 2 + 2 * STAGES + 8;
+  static constexpr int NBAR = 2 + 2 * STAGES + 10;
   static constexpr int SMEM_BYTES = SMEM_TILES + NBAR * 8 + 32 + 1024;  // + barriers, tmem ptr / abort block, align slack
   static constexpr int TMEM_COLS = 512;
   static constexpr int COL_S0 = 0, COL_S1 = 128, COL_O0 = 256, COL_O1 = 256 + DH;
@@ -79,7 +79,12 @@ struct FwdTcParams {
   CUtensorMap tq, tk, tv;
   FaFwdArgs a;
   StatusRef status;
-  int32_t num_splits, blocks_per_split;  // split-KV: key blocks [split * blocks_per_split, +blocks_per_split)
+  int32_t num_splits;  // split-KV: a sequence's key blocks are divided evenly
+  // A 128-row query tile holds `tile_pos` positions of `pack` neighbouring heads of one KV head's group, rows ordered
+  // (position, head): pack * tile_pos <= 128.  pack = 1: 128 positions of one head.
+  int32_t pack, pack_inv, tile_pos;
+  int32_t kv_box;  // rows of one K / V load: 128, or 64 where the pages of a paged cache are not a multiple of 128 rows
+  int32_t cache;   // K / V are a KV cache: the rows behind a sequence's keys hold anything, NaN patterns included
 };
 
 template <typename T>
@@ -93,7 +98,9 @@ struct Fmt<__nv_bfloat16> {
   static constexpr int kIdesc = 1;
 };
 
-template <typename T, int DH>
+// GROUPED: tiles shared by heads and / or keys in a KV cache (the plain instance keeps its geometry as constants: read from
+// the parameters it took 436 us instead of 397 on 16 x 2048 x 16 x 128 causal)
+template <typename T, int DH, bool GROUPED>
 __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ FwdTcParams P) {
   using C = Cfg<DH>;
   const FaFwdArgs& a = P.a;
@@ -110,6 +117,7 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
   auto bar_pfull = [&](int t) { return bar0 + 8 * (2 + 2 * C::STAGES + 2 + t); };
   auto bar_ofull = [&](int t) { return bar0 + 8 * (2 + 2 * C::STAGES + 4 + t); };
   auto bar_pfull_b = [&](int t) { return bar0 + 8 * (2 + 2 * C::STAGES + 6 + t); };
+  const uint32_t bar_vtail = bar0 + 8 * (2 + 2 * C::STAGES + 8), bar_vtail_go = bar0 + 8 * (2 + 2 * C::STAGES + 9);
   volatile uint32_t* tmem_ptr_smem = reinterpret_cast<volatile uint32_t*>(smem + C::SMEM_TILES + C::NBAR * 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + C::SMEM_TILES + C::NBAR * 8 + 4);
 
@@ -119,28 +127,32 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
     prefetch_tensormap(&P.tk);
     prefetch_tensormap(&P.tv);
   }
-  const int b = blockIdx.z, h = blockIdx.y, hk = h / (a.heads / a.heads_k);
-  const SeqInfo si = seq_info(a.cu_seqlens_q, a.cu_seqlens_k, nullptr, nullptr, a.seqlen_q, a.seqlen_k,
-                              a.use_mask_shift, a.mask_shift, b);
+  const int pack = GROUPED ? P.pack : 1, tile_pos = GROUPED ? P.tile_pos : kBM, pack_inv = GROUPED ? P.pack_inv : 65536;
+  const bool cache = GROUPED && P.cache;
+  const int b = blockIdx.z, h = blockIdx.y * pack, hk = h / (a.heads / a.heads_k);  // h: first head of the tile rows
+  SeqInfo si = seq_info(a.cu_seqlens_q, a.cu_seqlens_k, GROUPED ? a.seqused_k : nullptr, GROUPED ? a.kv_batch_idx : nullptr, a.seqlen_q,
+                        a.seqlen_k, a.use_mask_shift, a.mask_shift, b, GROUPED ? a.seqused_k_extra : 0);
+  if (cache) si.sk = min(si.sk, a.seqlen_k);
   // heaviest blocks (largest row index under a causal mask) first; with split-KV the splits of a row block are neighbours
   const int split = P.num_splits > 1 ? (int)blockIdx.x % P.num_splits : 0;
   const int mrank = P.num_splits > 1 ? (int)blockIdx.x / P.num_splits : (int)blockIdx.x;
   const int mblk = (int)gridDim.x / P.num_splits - 1 - mrank;
-  const int m_base = mblk * C::NT * kBM;
+  const int m_base = mblk * C::NT * tile_pos;
   if (m_base >= si.sq) return;  // uniform for the CTA
 
   // per-tile key block ranges
+  const int blocks_per_split = ((si.sk + kBN - 1) / kBN + P.num_splits - 1) / P.num_splits;
   int lo[2], hi[2];
   bool active[2];
 #pragma unroll
   for (int t = 0; t < 2; ++t) {
-    const int m0 = m_base + t * kBM;
+    const int m0 = m_base + t * tile_pos;
     active[t] = t < C::NT && m0 < si.sq;
     if (active[t]) {
-      key_block_range(m0, kBM, kBN, si.sk, si.shift, a.window_left, a.window_right, lo[t], hi[t]);
+      key_block_range(m0, tile_pos, kBN, si.sk, si.shift, a.window_left, a.window_right, lo[t], hi[t]);
       if (P.num_splits > 1) {
-        lo[t] = max(lo[t], split * P.blocks_per_split);
-        hi[t] = min(hi[t], (split + 1) * P.blocks_per_split);
+        lo[t] = max(lo[t], split * blocks_per_split);
+        hi[t] = min(hi[t], (split + 1) * blocks_per_split);
         if (hi[t] <= lo[t]) lo[t] = hi[t] = 0;
       }
     } else {
@@ -159,9 +171,44 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
     J_hi = hi[1];
   }
   const int nblk = J_hi - J_lo;  // may be 0
+  // Cache: block whose V rows past the last key are zeroed in shared memory (their P is 0, but 0 * NaN is not)
+  const int j_tail = cache && (si.sk % kBN) && (si.sk - 1) / kBN < J_hi && (si.sk - 1) / kBN >= J_lo ? (si.sk - 1) / kBN : -1;
 
+  auto load_q = [&](int t) {
+    if (!active[t] || hi[t] <= lo[t]) return;
+    mbar_expect_tx(bar_qfull(t), C::NCHUNK * 128 * pack * tile_pos);
+    const int r0 = (int)si.q_row0 + m_base + t * tile_pos;
+    for (int c = 0; c < C::NCHUNK; ++c)
+      tma_load_4d(sQ + t * C::TILE_BYTES + c * kChunkBytes, &P.tq, bar_qfull(t), c * 64, pack > 1 ? h : r0, pack > 1 ? r0 : h, (int)si.q_batch);
+  };
+  // Paged cache: the page of the block after the current one is looked up a block ahead, so that the producer does not
+  // stand in front of a free slot with a global load to wait for.  (With 64-row pages the second half is looked up.)
+  int page_key = -1, page_id = 0;
+  auto page_at = [&](int key) { return a.block_table[(int64_t)b * a.block_table_stride + key / a.page_block_size]; };
+  auto page_of = [&](int key) { return key == page_key ? page_id : page_at(key); };
+  // ring item idx: K of block J_lo + idx / 2 (idx even) or V (odd)
+  auto load_kv = [&](int idx) {
+    const int slot = idx % C::STAGES, j = J_lo + (idx >> 1);
+    const CUtensorMap* tm = (idx & 1) ? &P.tv : &P.tk;
+    const uint32_t dst = sKV + slot * C::TILE_BYTES;
+    if (GROUPED && a.block_table) {  // one lookup per load; rows past the last key are not loaded page by page
+      const int n_box = min((min(kBN, si.sk - j * kBN) + P.kv_box - 1) / P.kv_box, kBN / P.kv_box);
+      mbar_expect_tx(bar_full(slot), n_box * P.kv_box * C::NCHUNK * 128);
+      for (int i = 0; i < n_box; ++i) {
+        const int key = j * kBN + i * P.kv_box;
+        const int page = page_of(key);
+        for (int c = 0; c < C::NCHUNK; ++c)
+          tma_load_4d(dst + c * kChunkBytes + i * P.kv_box * 128, tm, bar_full(slot), c * 64, key % a.page_block_size, hk, page);
+      }
+    } else {
+      mbar_expect_tx(bar_full(slot), C::TILE_BYTES);
+      for (int c = 0; c < C::NCHUNK; ++c)
+        tma_load_4d(dst + c * kChunkBytes, tm, bar_full(slot), c * 64, (int)si.k_row0 + j * kBN, hk, (int)si.k_batch);
+    }
+  };
+
+  if (threadIdx.x == 32) abort_init(abort_flag, P.status);  // a read of global memory: not in front of the first loads
   if (threadIdx.x == 0) {
-    abort_init(abort_flag, P.status);
     for (int t = 0; t < 2; ++t) {
       mbar_init(bar_qfull(t), 1);
       mbar_init(bar_sfull(t), 1);
@@ -173,8 +220,18 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
       mbar_init(bar_full(s), 1);
       mbar_init(bar_empty(s), 1);
     }
+    mbar_init(bar_vtail, 1);
+    mbar_init(bar_vtail_go, 1);
     fence_barrier_init();
     fence_proxy_async();
+    if (nblk > 0) {
+      // This thread has made the barriers, so it can start the first block's loads while the CTA still sets itself up:
+      // what S of the first tile needs goes first
+      load_q(0);
+      load_kv(0);
+      if (C::NT > 1) load_q(1);
+      load_kv(1);
+    }
   }
   if (warp == 10) {
     tmem_alloc(smem_addr(const_cast<uint32_t*>(tmem_ptr_smem)), C::TMEM_COLS);
@@ -192,7 +249,11 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
     setmaxnreg_inc<216>();
     const int t = warp >> 2;
     const int row_in_tile = (warp & 3) * 32 + lane;
-    const int row = m_base + t * kBM + row_in_tile;
+    const int m0 = m_base + t * tile_pos;
+    const int pos_in_tile = (row_in_tile * pack_inv) >> 16;             // row_in_tile / pack
+    const int row = m0 + (GROUPED ? min(pos_in_tile, tile_pos - 1) : pos_in_tile);                  // query position of this thread's row
+    const int head = h + row_in_tile - pos_in_tile * pack;
+    const bool row_valid = pos_in_tile < tile_pos && row < si.sq;
     const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
     const uint32_t tS = tmem + lane_off + (t ? C::COL_S1 : C::COL_S0);
     const uint32_t tO = tmem + lane_off + (t ? C::COL_O1 : C::COL_O0);
@@ -202,7 +263,6 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
     int col_first = 0, col_last = si.sk - 1;
     if (a.window_right >= 0) col_last = min(col_last, row + si.shift + a.window_right);
     if (a.window_left >= 0) col_first = max(col_first, row + si.shift - a.window_left);
-    const int m0 = m_base + t * kBM;
 
     const uint64_t scale2 = pack2(scale_log2, scale_log2);
     uint64_t l_sum2 = pack2(0.f, 0.f);  // two running partial row sums (even / odd columns)
@@ -215,7 +275,7 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
       const int n0 = j * kBN;
       const bool need_mask = (n0 + kBN - 1 >= si.sk) ||
                              (a.window_right >= 0 && n0 + kBN - 1 > m0 + si.shift + a.window_right) ||
-                             (a.window_left >= 0 && n0 < m0 + kBM - 1 + si.shift - a.window_left);
+                             (a.window_left >= 0 && n0 < m0 + tile_pos - 1 + si.shift - a.window_left);
       // One block of the online softmax.  MASKED = false is the straight-line version for blocks that every row
       // sees entirely; MASKED = true classifies each 32-column chunk for the warp: bit q of `none` = no row of
       // this warp sees chunk q (no maximum, no exponentials, P = 0), bit q of `part` = the mask boundary crosses
@@ -343,11 +403,11 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
         const bool empty = !(l_sum > 0.f) || m_used == -INFINITY;
         const float inv = empty ? 0.f : 1.f / l_sum;
         const float lse = empty ? INFINITY : (m_used + log2f(l_sum)) * kLn2;
-        if (row < si.sq) {
+        if (row_valid) {
           if (P.num_splits > 1)  // the split workspaces are (split, batch, head, row): not packed, -inf marks an empty part
-            a.lse_accum[((int64_t)split * a.batch * a.heads + (int64_t)b * a.heads + h) * a.seqlen_q + row] = empty ? -INFINITY : lse;
+            a.lse_accum[((int64_t)split * a.batch * a.heads + (int64_t)b * a.heads + head) * a.seqlen_q + row] = empty ? -INFINITY : lse;
           else
-            a.softmax_lse[((int64_t)b * a.heads + h) * a.lse_seqlen + row] = lse;
+            a.softmax_lse[((int64_t)b * a.heads + head) * a.lse_seqlen + row] = lse;
         }
         unsigned char* stage = smem + t * C::TILE_BYTES;  // the Q tile of this warpgroup is no longer read
         constexpr int ROWB = DH * 2;
@@ -370,9 +430,9 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
           }
           const uint32_t(&o)[32] = ob[(c0 % OB) / 32];
           if (P.num_splits > 1) {  // normalised fp32 partial, straight from the registers (rows are contiguous)
-            if (row < si.sq) {
+            if (row_valid && have_o) {  // an empty part is not read: its weight is zero
               float* oa = a.out_accum +
-                          (((int64_t)split * a.batch * a.heads + (int64_t)b * a.heads + h) * a.seqlen_q + row) * a.head_dim;
+                          (((int64_t)split * a.batch * a.heads + (int64_t)b * a.heads + head) * a.seqlen_q + row) * a.head_dim;
 #pragma unroll
               for (int i = 0; i < 32; i += 4)
                 if (c0 + i < a.head_dim)
@@ -405,11 +465,13 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
 #pragma unroll 4
         for (int i = tid; i < kBM * CPR; i += 128) {
           const int r = i / CPR, chunk = i % CPR;
-          const int grow_ = m0 + r;
-          if (grow_ < si.sq) {
+          const int rp = (r * pack_inv) >> 16;  // r / pack
+          const int grow_ = m0 + rp;
+          if (rp < tile_pos && grow_ < si.sq) {
             const int phys = (chunk & ~7) | ((chunk ^ r) & 7);
             uint4 v = *reinterpret_cast<const uint4*>(stage + r * (DH * 2) + phys * 16);
-            if (chunk * 8 < a.head_dim) *reinterpret_cast<uint4*>(og + (int64_t)grow_ * a.out.stride_s + chunk * 8) = v;
+            if (chunk * 8 < a.head_dim) 
+              *reinterpret_cast<uint4*>(og + (int64_t)grow_ * a.out.stride_s + (r - rp * pack) * a.out.stride_h + chunk * 8) = v;
           }
         }
       }
@@ -419,25 +481,15 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
     if (warp == 8) {
       // ---------------------------------------------------------------- TMA producer
       if (lane == 0) {
-        const int qrow = (int)si.q_row0 + m_base;
-        const int qb = (int)si.q_batch, kb = (int)si.k_batch;
-        for (int t = 0; t < 2; ++t) {
-          if (!active[t] || hi[t] <= lo[t]) continue;
-          mbar_expect_tx(bar_qfull(t), C::TILE_BYTES);
-          for (int c = 0; c < C::NCHUNK; ++c)
-            tma_load_4d(sQ + t * C::TILE_BYTES + c * kChunkBytes, &P.tq, bar_qfull(t), c * 64, qrow + t * kBM, h, qb);
-        }
         bool ok = true;
-        for (int idx = 0; idx < 2 * nblk && ok; ++idx) {
+        for (int idx = 2; idx < 2 * nblk && ok; ++idx) {  // K and V of the first block are on their way
           const int slot = idx % C::STAGES, round = idx / C::STAGES;
+          if (GROUPED && a.block_table && !(idx & 1)) {
+            page_key = (J_lo + (idx >> 1)) * kBN;
+            page_id = page_at(page_key);
+          }
           ok = mbar_wait(bar_empty(slot), (round & 1) ^ 1, W_KVEMPTY, abort_flag);
-          if (!ok) break;
-          const int j = J_lo + (idx >> 1);
-          const CUtensorMap* tm = (idx & 1) ? &P.tv : &P.tk;
-          mbar_expect_tx(bar_full(slot), C::TILE_BYTES);
-          for (int c = 0; c < C::NCHUNK; ++c)
-            tma_load_4d(sKV + slot * C::TILE_BYTES + c * kChunkBytes, tm, bar_full(slot), c * 64,
-                        (int)si.k_row0 + j * kBN, hk, kb);
+          if (ok) load_kv(idx);
         }
       }
     } else if (warp == 9) {
@@ -482,22 +534,25 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
         // (Testing each barrier one MMA group ahead of its use, so that the answer travels while the group before
         // is being issued, was measured here and lost 3-5 %: the tests themselves take issue slots of this warp.)
         if (nblk > 0) {
-          for (int t = 0; t < C::NT && ok; ++t)
-            if (hi[t] > lo[t]) ok = mbar_wait_w(bar_qfull(t), 0, W_QFULL, abort_flag);
           // prologue: S_t(J_lo)
-          if (ok) ok = mbar_wait_w(bar_full(slot_of(0)), par_of(0), W_KVFULL, abort_flag);
-          if (ok) {
+          ok = mbar_wait_w(bar_full(slot_of(0)), par_of(0), W_KVFULL, abort_flag);
+          for (int t = 0; t < C::NT && ok; ++t) {
+            if (hi[t] > lo[t]) ok = mbar_wait_w(bar_qfull(t), 0, W_QFULL, abort_flag);
+            if (!ok) break;
             tc_fence_after();
-            for (int t = 0; t < C::NT; ++t)
-              if (in_range(t, J_lo)) issue_s(t, slot_of(0));
-            tc_commit_w(bar_empty(slot_of(0)));
+            if (in_range(t, J_lo)) issue_s(t, slot_of(0));
           }
+          if (ok) tc_commit_w(bar_empty(slot_of(0)));
           for (int j = J_lo; j < J_hi && ok; ++j) {
             const int iv = 2 * (j - J_lo) + 1;  // ring index of V(j)
             const int ik = iv + 1;              // ring index of K(j+1)
             const bool more = j + 1 < J_hi;
             ok = mbar_wait_w(bar_full(slot_of(iv)), par_of(iv), W_KVFULL, abort_flag);
             if (ok && more) ok = mbar_wait_w(bar_full(slot_of(ik)), par_of(ik), W_KVFULL, abort_flag);
+            if (GROUPED && ok && j == j_tail) {  // V has landed: warp 11 clears its rows behind the last key
+              if (lane == 0) mbar_arrive(bar_vtail_go);
+              ok = mbar_wait_w(bar_vtail, 0, W_VTAIL, abort_flag);
+            }
             if (!ok) break;
 #pragma unroll
             for (int t = 0; t < C::NT; ++t) {
@@ -521,6 +576,20 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
           }
         }
       }
+    } else if (GROUPED && warp == 11 && j_tail >= 0) {
+      // ---------------------------------------------------------------- zeroes the rows of the last V tile that hold no key
+      // (The MMA warp says when: a wait of this warp's own on the slot's barrier would have to pass all its earlier phases.)
+      const int iv = 2 * (j_tail - J_lo) + 1, slot = iv % C::STAGES;
+      if (mbar_wait_w(bar_vtail_go, 0, W_VTAIL, abort_flag)) {
+        const int first = si.sk - j_tail * kBN;
+        unsigned char* v = smem + (C::NT + slot) * C::TILE_BYTES + first * 128;
+        for (int i = lane; i < (kBN - first) * 8; i += 32)
+#pragma unroll
+          for (int c = 0; c < C::NCHUNK; ++c) *reinterpret_cast<uint4*>(v + c * kChunkBytes + i * 16) = make_uint4(0, 0, 0, 0);
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_vtail);
+      }
     }
   }
 
@@ -538,36 +607,53 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
   if (warp == 10) tmem_dealloc(tmem, C::TMEM_COLS);
 }
 
+// Heads of a KV head's group that share a query tile: the largest divisor of the group that leaves at least 120 of the
+// 128 rows in use.  With the group's heads in one tile the two tiles of a CTA end at the same key block of a causal mask
+// (a block in which only one tile works costs both tiles' time), and a few tokens per sequence fill a tile.
+int pack_heads(int group) {
+  for (int d = group < kBM ? group : kBM; d > 1; --d)
+    if (group % d == 0 && kBM / d * d >= 120) return d;
+  return 1;
+}
+
 template <typename T, int DH>
-int launch_fwd_tc(const FaFwdArgs& a, cudaStream_t st) {
+int launch_fwd_tc(const FaFwdArgs& a, int64_t kv_batches, cudaStream_t st) {
   using C = Cfg<DH>;
   FwdTcParams P;
   P.a = a;
   const bool varlen = a.cu_seqlens_q != nullptr;
   const int64_t q_rows = varlen ? a.total_q : a.seqlen_q, k_rows = varlen ? a.total_k : a.seqlen_k;
   const int64_t nb = varlen ? 1 : a.batch;
-  if (make_tmap_4d(&P.tq, a.q, a.dtype, q_rows, a.heads, nb, a.head_dim, kBM)) return 1;
-  if (make_tmap_4d(&P.tk, a.k, a.dtype, k_rows, a.heads_k, nb, a.head_dim, kBN)) return 1;
-  if (make_tmap_4d(&P.tv, a.v, a.dtype, k_rows, a.heads_k, nb, a.head_dim, kBN)) return 1;
+  P.cache = kv_batches > 0;
+  P.pack = pack_heads(a.heads / a.heads_k);
+  P.pack_inv = (65536 + P.pack - 1) / P.pack;
+  P.tile_pos = kBM / P.pack;
+  P.kv_box = a.block_table && a.page_block_size % kBN ? 64 : kBN;
+  if (P.pack > 1 ? make_tmap_4d_heads(&P.tq, a.q, a.dtype, q_rows, a.heads, nb, a.head_dim, P.pack, P.tile_pos)
+                 : make_tmap_4d(&P.tq, a.q, a.dtype, q_rows, a.heads, nb, a.head_dim, kBM))
+    return 1;
+  const int64_t kv_rows = a.block_table ? a.page_block_size : k_rows, kv_nb = P.cache ? kv_batches : nb;
+  if (make_tmap_4d(&P.tk, a.k, a.dtype, kv_rows, a.heads_k, kv_nb, a.head_dim, P.kv_box)) return 1;
+  if (make_tmap_4d(&P.tv, a.v, a.dtype, kv_rows, a.heads_k, kv_nb, a.head_dim, P.kv_box)) return 1;
   P.status = status_ref(true);
   P.num_splits = a.num_splits > 1 ? a.num_splits : 1;
-  const int n_blocks = (a.seqlen_k + kBN - 1) / kBN;
-  P.blocks_per_split = (n_blocks + P.num_splits - 1) / P.num_splits;
-  auto kern = fwd_tc_kernel<T, DH>;
-  static fa_host::DeviceOnce once;
-  if (int rc = fa_host::raise_smem_limit(once, reinterpret_cast<const void*>(kern), C::SMEM_BYTES, "fwd_tc_kernel")) return rc;
-  const int n_m = (a.seqlen_q + C::NT * kBM - 1) / (C::NT * kBM);
-  dim3 grid(n_m * P.num_splits, a.heads, a.batch);
+  const bool grouped = P.pack > 1 || P.cache;
+  auto kern = grouped ? fwd_tc_kernel<T, DH, true> : fwd_tc_kernel<T, DH, false>;
+  static fa_host::DeviceOnce once[2];
+  if (int rc = fa_host::raise_smem_limit(once[grouped], reinterpret_cast<const void*>(kern), C::SMEM_BYTES, "fwd_tc_kernel")) return rc;
+  const int n_m = (a.seqlen_q + C::NT * P.tile_pos - 1) / (C::NT * P.tile_pos);
+  dim3 grid(n_m * P.num_splits, a.heads / P.pack, a.batch);
   kern<<<grid, 384, C::SMEM_BYTES, st>>>(P);
   return fa_host::check_launch("fwd_tc_kernel");
 }
 
 }  // namespace
 
-bool fwd_tc_eligible(const FaFwdArgs& a) {
+// kv_batches: 0, or the number of sequence slots (pages) of a KV cache
+static bool fwd_tc_takes(const FaFwdArgs& a, int64_t kv_batches) {
   if (a.head_dim > 256 || a.p_dropout > 0.f || a.s_dmask) return false;
   if (a.num_splits > 1 && a.cu_seqlens_q) return false;
-  if (a.seqused_k || a.kv_batch_idx || a.block_table) return false;
+  if ((a.seqused_k || a.kv_batch_idx || a.block_table) && kv_batches <= 0) return false;
   if (a.seqlen_k <= 0) return false;
   if (!tma_compatible(a.q) || !tma_compatible(a.k) || !tma_compatible(a.v)) return false;
   if ((reinterpret_cast<uintptr_t>(a.out.ptr) & 15) || a.out.stride_s % 8 || a.out.stride_h % 8 || a.out.stride_b % 8)
@@ -576,11 +662,23 @@ bool fwd_tc_eligible(const FaFwdArgs& a) {
   return encode_tiled_fn() != nullptr;
 }
 
-int fwd_tc(const FaFwdArgs& a, cudaStream_t st) {
+static int fwd_tc_run(const FaFwdArgs& a, int64_t kv_batches, cudaStream_t st) {
   const bool bf = a.dtype == FA_DTYPE_BF16;
-  if (a.head_dim <= 64) return bf ? launch_fwd_tc<__nv_bfloat16, 64>(a, st) : launch_fwd_tc<__half, 64>(a, st);
-  if (a.head_dim <= 128) return bf ? launch_fwd_tc<__nv_bfloat16, 128>(a, st) : launch_fwd_tc<__half, 128>(a, st);
-  return bf ? launch_fwd_tc<__nv_bfloat16, 256>(a, st) : launch_fwd_tc<__half, 256>(a, st);
+  if (a.head_dim <= 64)
+    return bf ? launch_fwd_tc<__nv_bfloat16, 64>(a, kv_batches, st) : launch_fwd_tc<__half, 64>(a, kv_batches, st);
+  if (a.head_dim <= 128)
+    return bf ? launch_fwd_tc<__nv_bfloat16, 128>(a, kv_batches, st) : launch_fwd_tc<__half, 128>(a, kv_batches, st);
+  return bf ? launch_fwd_tc<__nv_bfloat16, 256>(a, kv_batches, st) : launch_fwd_tc<__half, 256>(a, kv_batches, st);
 }
+
+bool fwd_tc_eligible(const FaFwdArgs& a) { return fwd_tc_takes(a, 0); }
+int fwd_tc(const FaFwdArgs& a, cudaStream_t st) { return fwd_tc_run(a, 0, st); }
+
+// Several tokens per sequence against a KV cache.  Up to 32 rows (tokens x heads of a group) the 64-row any-shape kernel
+// stays, whose tiles such calls fill better.
+bool fwd_tc_cache_eligible(const FaFwdArgs& a, int64_t kv_batches) {
+  return (int64_t)a.seqlen_q * (a.heads / a.heads_k) > 32 && kv_batches > 0 && fwd_tc_takes(a, kv_batches);
+}
+int fwd_tc_cache(const FaFwdArgs& a, int64_t kv_batches, cudaStream_t st) { return fwd_tc_run(a, kv_batches, st); }
 
 }  // namespace fa

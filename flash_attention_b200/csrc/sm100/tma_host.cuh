@@ -30,30 +30,48 @@ static inline EncodeTiledFn encode_tiled_fn() {
   return fn;
 }
 
-// 4-D map with dims (dim, seq, head, batch), 128-byte swizzle, box = 64 elements x box_rows rows.
-// Out-of-range elements read as zero.  `rows`/`batches` describe the extent of the tensor: for
-// packed variable-length tensors rows = total tokens and batches = 1.
-static inline int make_tmap_4d(CUtensorMap* map, const FaTensor& t, int dtype, int64_t rows, int heads, int64_t batches,
-                               int head_dim, int box_rows) {
+static inline int make_tmap(CUtensorMap* map, const FaTensor& t, int dtype, int head_dim, const int64_t (&extent)[3],
+                            const int64_t (&stride)[3], const int (&box_of)[3]) {
   EncodeTiledFn fn = encode_tiled_fn();
   if (!fn) {
     fa_host::set_error("cuTensorMapEncodeTiled is not available from this driver");
     return 1;
   }
-  cuuint64_t dims[4] = {(cuuint64_t)head_dim, (cuuint64_t)rows, (cuuint64_t)heads, (cuuint64_t)batches};
+  cuuint64_t dims[4] = {(cuuint64_t)head_dim, (cuuint64_t)extent[0], (cuuint64_t)extent[1], (cuuint64_t)extent[2]};
   // strides of dims 1..3 in bytes; a degenerate dim still needs a legal (non-zero, 16 B multiple) stride
   auto legal = [](int64_t elems) { return (cuuint64_t)(elems > 0 ? elems : 8) * 2; };
-  cuuint64_t strides[3] = {legal(t.stride_s), legal(t.stride_h), legal(t.stride_b)};
-  cuuint32_t box[4] = {64, (cuuint32_t)box_rows, 1, 1};
+  cuuint64_t strides[3] = {legal(stride[0]), legal(stride[1]), legal(stride[2])};
+  cuuint32_t box[4] = {64, (cuuint32_t)box_of[0], (cuuint32_t)box_of[1], (cuuint32_t)box_of[2]};
   cuuint32_t estr[4] = {1, 1, 1, 1};
-  CUresult r = fn(map, dtype == FA_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4,
+  auto encode = [&]() { return fn(map, dtype == FA_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4,
                   t.ptr, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE); };
+  CUresult r = encode();
+  if (r == CUDA_ERROR_INVALID_CONTEXT) {  // a thread that has made no runtime call yet (autograd's): make its context current
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) r = encode();
+  }
   if (r != CUDA_SUCCESS) {
     fa_host::set_error("cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
     return 1;
   }
   return 0;
+}
+
+// 4-D map with dims (dim, seq, head, batch), 128-byte swizzle, box = 64 elements x box_rows rows.
+// Out-of-range elements read as zero.  `rows`/`batches` describe the extent of the tensor: for
+// packed variable-length tensors rows = total tokens and batches = 1.
+static inline int make_tmap_4d(CUtensorMap* map, const FaTensor& t, int dtype, int64_t rows, int heads, int64_t batches,
+                               int head_dim, int box_rows) {
+  return make_tmap(map, t, dtype, head_dim, {rows, heads, batches}, {t.stride_s, t.stride_h, t.stride_b}, {box_rows, 1, 1});
+}
+
+// The same tensor with dims (dim, head, seq, batch) and a box of box_heads heads of box_rows positions: the rows of a
+// box are ordered (position, head).
+static inline int make_tmap_4d_heads(CUtensorMap* map, const FaTensor& t, int dtype, int64_t rows, int heads, int64_t batches,
+                                     int head_dim, int box_heads, int box_rows) {
+  return make_tmap(map, t, dtype, head_dim, {heads, rows, batches}, {t.stride_h, t.stride_s, t.stride_b},
+                   {box_heads, box_rows, 1});
 }
 
 static inline bool tma_compatible(const FaTensor& t) {

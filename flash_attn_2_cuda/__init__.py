@@ -163,7 +163,8 @@ def fwd(q, k, v, out_, p_dropout, softmax_scale, is_causal, window_size_left, wi
             a.num_splits = 1
             keep = None
             if p_dropout == 0.0:  # flash_api.cpp:373-389
-                ns = lib().fa_fwd_num_splits(batch, heads, seqlen_q, seqlen_k, d, _sm_count(q.device))
+                # the heads of a group share the kernel's 128-row tiles
+                ns = lib().fa_fwd_num_splits(batch, heads_k, seqlen_q * (heads // heads_k), seqlen_k, d, _sm_count(q.device))
                 if os.environ.get("FA_B200_FWD_SPLITS"):  # test knob: pin the split count (1 = never split)
                     ns = max(1, min(128, int(os.environ["FA_B200_FWD_SPLITS"])))
                 if ns > 1:
