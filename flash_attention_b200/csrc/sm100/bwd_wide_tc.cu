@@ -38,7 +38,7 @@ constexpr int kChunkB = kN * 128;        // [64 rows][64 x 16-bit]
 constexpr int kTileA = 4 * kChunkA, kTileB = 4 * kChunkB;
 constexpr int kThreads = 384;
 constexpr int kWarpProducer = 8, kWarpMma = 9, kWarpTmem = 10, kWarpMmaX1 = 11;
-constexpr int kRegsCompute = 200, kRegsOther = 72;
+constexpr int kRegsCompute = 192, kRegsOther = 88;
 
 enum Pass { PASS_DV = 0, PASS_DK = 1, PASS_DQ = 2 };
 
@@ -109,13 +109,19 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_wide_tc_kernel(const __grid_c
   auto bar_b2_full = [&](int st) { return bar0 + 8 * (2 * NS1 + st); };
   auto bar_b2_empty = [&](int st) { return bar0 + 8 * (2 * NS1 + NS2 + st); };
   constexpr int kB0 = 2 * NS1 + 2 * NS2;
-  const uint32_t bar_x1 = bar0 + 8 * kB0, bar_x1read = bar0 + 8 * (kB0 + 1), bar_a = bar0 + 8 * (kB0 + 2),
+  const uint32_t bar_x1 = bar0 + 8 * kB0, bar_x1read = bar0 + 8 * (kB0 + 1), bar_a1 = bar0 + 8 * (kB0 + 2), bar_a2 = bar0 + 8 * (kB0 + 7),
                  bar_x2 = bar0 + 8 * (kB0 + 3), bar_x2read = bar0 + 8 * (kB0 + 4), bar_w = bar0 + 8 * (kB0 + 5),
                  bar_done = bar0 + 8 * (kB0 + 6);
   volatile uint32_t* tmem_ptr_smem = reinterpret_cast<volatile uint32_t*>(smem + C::OFF_BAR + C::NBAR * 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + C::OFF_BAR + C::NBAR * 8 + 4);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 32) {  // the TMA unit fetches the descriptors while the CTA sets itself up
+    prefetch_tensormap(&P.ta1);
+    if (C::NA == 2) prefetch_tensormap(&P.ta2);
+    prefetch_tensormap(&P.tb1);
+    prefetch_tensormap(&P.tb2);
+  }
   const int b = blockIdx.z;
   const int group = a.heads / a.heads_k;
   const SeqInfo si = seq_info(a.cu_seqlens_q, a.cu_seqlens_k, nullptr, nullptr, a.seqlen_q, a.seqlen_k,
@@ -138,9 +144,11 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_wide_tc_kernel(const __grid_c
     iters = (blk_hi - blk_lo) * group;
   }
 
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == 64) {  // reads global memory: not in front of the first loads
     abort_init(abort_flag, P.status);
     if (s_base & 1023u) abort_raise(abort_flag, W_W_ALIGN);  // the swizzled tiles need a 1024-byte aligned base
+  }
+  if (threadIdx.x == 0) {
     for (int s = 0; s < NS1; ++s) {
       mbar_init(bar_b1_full(s), 1);
       mbar_init(bar_b1_empty(s), 1);
@@ -151,13 +159,32 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_wide_tc_kernel(const __grid_c
     }
     mbar_init(bar_x1, 1);
     mbar_init(bar_x1read, 8);
-    mbar_init(bar_a, 1);
+    mbar_init(bar_a1, 1);
+    mbar_init(bar_a2, 1);
     mbar_init(bar_x2, 1);
     mbar_init(bar_x2read, 8);
     mbar_init(bar_w, 8);
     mbar_init(bar_done, 1);
     fence_barrier_init();
     fence_proxy_async();
+    if (iters > 0) {
+      // This thread has made the barriers, so it can start the first block's loads while the CTA still sets itself up,
+      // in the order in which the first products need them
+      auto load = [&](uint32_t dst, const CUtensorMap* tm, uint32_t bar, int chunk, int64_t row, int head, int64_t batch) {
+        mbar_expect_tx(bar, 4 * chunk);
+        for (int c = 0; c < 4; ++c) tma_load_4d(dst + c * chunk, tm, bar, c * 64, (int)row, head, (int)batch);
+      };
+      const int64_t arow = (kRowsAreQueries ? si.q_row0 : si.k_row0) + r0, ab = kRowsAreQueries ? si.q_batch : si.k_batch;
+      const int64_t brow = (kRowsAreQueries ? si.k_row0 : si.q_row0) + blk_lo * kN, bb = kRowsAreQueries ? si.k_batch : si.q_batch;
+      const int ahead = kRowsAreQueries ? hq_fixed : hk, bhead = kRowsAreQueries ? hk : hq_fixed;
+      if (C::NA == 2) {
+        load(s_base + C::OFF_A + kTileA, &P.ta2, bar_a2, kChunkA, arow, ahead, ab);
+        load(sB2(0), &P.tb2, bar_b2_full(0), kChunkB, brow, bhead, bb);
+      }
+      load(s_base + C::OFF_A, &P.ta1, bar_a1, kChunkA, arow, ahead, ab);
+      load(sB1(0), &P.tb1, bar_b1_full(0), kChunkB, brow, bhead, bb);
+      if (C::NA == 1) load(sB2(0), &P.tb2, bar_b2_full(0), kChunkB, brow, bhead, bb);
+    }
   }
   if (warp == kWarpTmem) {
     tmem_alloc(smem_addr(const_cast<uint32_t*>(tmem_ptr_smem)), C::TMEM_COLS);
@@ -322,15 +349,10 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_wide_tc_kernel(const __grid_c
     if (ok && iters > 0) ok = mbar_wait(bar_done, 0, W_W_DONE, abort_flag);
     tc_fence_after();
     ok = __all_sync(0xffffffffu, ok && *abort_flag == 0);  // the TMEM loads below are warp-wide instructions
+    const bool to_accum = !kRowsAreQueries && a.accumulate_dkv;
     if (ok) {
       const uint32_t tO = tmem + lane_off + C::COL_OUT + w * 128;
-      const bool valid = row < (kRowsAreQueries ? si.sq : si.sk);
       const float sc = PASS == PASS_DV ? 1.f : a.softmax_scale;
-      const FaTensor& tt = PASS == PASS_DQ ? a.dq : (PASS == PASS_DK ? a.dk : a.dv);
-      const int64_t tb = kRowsAreQueries ? si.q_batch : si.k_batch, trow = (kRowsAreQueries ? si.q_row0 : si.k_row0) + row;
-      const int th = kRowsAreQueries ? hq_fixed : hk;
-      const bool to_accum = !kRowsAreQueries && a.accumulate_dkv;
-      T* g = to_accum ? nullptr : reinterpret_cast<T*>(tt.ptr) + tb * tt.stride_b + trow * tt.stride_s + (int64_t)th * tt.stride_h;
       float* acc = to_accum ? (PASS == PASS_DK ? a.dk_accum : a.dv_accum) +
                                   (((int64_t)si.k_batch * a.seqlen_k + si.k_row0 + row) * a.heads_k + hk) * a.head_dim
                             : nullptr;
@@ -344,12 +366,11 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_wide_tc_kernel(const __grid_c
 #pragma unroll
           for (int i = 0; i < 32; ++i) o[i] = 0u;
         }
-        if (!valid) continue;
         const int col0 = w * 128 + c0;
         if (to_accum) {
 #pragma unroll
           for (int i = 0; i < 32; i += 4) {
-            if (col0 + i < a.head_dim) {
+            if (row < si.sk && col0 + i < a.head_dim) {
               float4 cur = *reinterpret_cast<float4*>(acc + col0 + i);
               cur.x += __uint_as_float(o[i]) * sc;
               cur.y += __uint_as_float(o[i + 1]) * sc;
@@ -359,40 +380,40 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_wide_tc_kernel(const __grid_c
             }
           }
         } else {
+          // 16-bit rows over the first stationary tile (every MMA is done), 16-byte pieces swizzled
 #pragma unroll
           for (int i = 0; i < 32; i += 8) {
-            if (col0 + i < a.head_dim) {
-              uint4 v;
-              v.x = Pack<T>::two(__uint_as_float(o[i]) * sc, __uint_as_float(o[i + 1]) * sc);
-              v.y = Pack<T>::two(__uint_as_float(o[i + 2]) * sc, __uint_as_float(o[i + 3]) * sc);
-              v.z = Pack<T>::two(__uint_as_float(o[i + 4]) * sc, __uint_as_float(o[i + 5]) * sc);
-              v.w = Pack<T>::two(__uint_as_float(o[i + 6]) * sc, __uint_as_float(o[i + 7]) * sc);
-              *reinterpret_cast<uint4*>(g + col0 + i) = v;
-            }
+            uint4 v;
+            v.x = Pack<T>::two(__uint_as_float(o[i]) * sc, __uint_as_float(o[i + 1]) * sc);
+            v.y = Pack<T>::two(__uint_as_float(o[i + 2]) * sc, __uint_as_float(o[i + 3]) * sc);
+            v.z = Pack<T>::two(__uint_as_float(o[i + 4]) * sc, __uint_as_float(o[i + 5]) * sc);
+            v.w = Pack<T>::two(__uint_as_float(o[i + 6]) * sc, __uint_as_float(o[i + 7]) * sc);
+            *reinterpret_cast<uint4*>(smem + C::OFF_A + r * (kDH * 2) + ((((col0 + i) / 8) ^ (r & 7)) << 4)) = v;
           }
         }
       }
+    }
+    named_bar_sync(1, 256);
+    if (ok && !to_accum) {  // whole rows by neighbouring threads: a store of a warp is one row, not 32 lines
+      const FaTensor& tt = PASS == PASS_DQ ? a.dq : (PASS == PASS_DK ? a.dk : a.dv);
+      const int64_t tb = kRowsAreQueries ? si.q_batch : si.k_batch, trow = (kRowsAreQueries ? si.q_row0 : si.k_row0) + r0;
+      T* g = reinterpret_cast<T*>(tt.ptr) + tb * tt.stride_b + trow * tt.stride_s + (int64_t)(kRowsAreQueries ? hq_fixed : hk) * tt.stride_h;
+      const int rows = min(kR, (kRowsAreQueries ? si.sq : si.sk) - r0);
+      if (lane * 8 < a.head_dim)
+        for (int i = warp; i < rows; i += 8)
+          *reinterpret_cast<uint4*>(g + i * tt.stride_s + lane * 8) =
+              *reinterpret_cast<const uint4*>(smem + C::OFF_A + i * (kDH * 2) + ((lane ^ (i & 7)) << 4));
     }
   } else {
     setmaxnreg_dec<kRegsOther>();
     if (warp == kWarpProducer) {
       // -------------------------------------------------------------- TMA producer
       if (lane == 0 && run) {
-        prefetch_tensormap(&P.ta1);
-        if (C::NA == 2) prefetch_tensormap(&P.ta2);
-        prefetch_tensormap(&P.tb1);
-        prefetch_tensormap(&P.tb2);
         const int kb = (int)si.k_batch, qb = (int)si.q_batch;
-        const int arow = (int)(kRowsAreQueries ? si.q_row0 : si.k_row0) + r0;
-        const int ahead = kRowsAreQueries ? hq_fixed : hk, ab = kRowsAreQueries ? qb : kb;
-        mbar_expect_tx(bar_a, C::NA * kTileA);
-        for (int c = 0; c < 4; ++c) {
-          tma_load_4d(s_base + C::OFF_A + c * kChunkA, &P.ta1, bar_a, c * 64, arow, ahead, ab);
-          if (C::NA == 2) tma_load_4d(s_base + C::OFF_A + kTileA + c * kChunkA, &P.ta2, bar_a, c * 64, arow, ahead, ab);
-        }
         Walk wk{blk_lo, hq_fixed, blk_lo, blk_hi};
+        wk.next();
         bool ok = true;
-        for (int it = 0; it < iters && ok; ++it) {
+        for (int it = 1; it < iters && ok; ++it) {  // block 0 is on its way
           const int s1 = it % NS1, s2 = it % NS2;
           int brow, bhead, bb;
           if (kRowsAreQueries) {
@@ -459,7 +480,8 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_wide_tc_kernel(const __grid_c
           for (int kk = 0; kk < kN / 16; ++kk)
             mma_ts_w(tmem + C::COL_OUT, tmem + C::COL_W + (j & 1) * 32 + kk * 8, dsc(b_lo + moff(kk)), idesc_o, (j > 0) || kk > 0);
         };
-        bool ok = mbar_wait_w(bar_a, 0, W_W_A, abort_flag);
+        bool ok = true;
+        if (warp == kWarpMmaX1 || PASS != PASS_DV) ok = mbar_wait_w(warp == kWarpMmaX1 ? bar_a1 : bar_a2, 0, W_W_A, abort_flag);
         if (warp == kWarpMmaX1) {
           // ---- X1 products
           for (int j = 0; j < iters && ok; ++j) {
