@@ -48,11 +48,28 @@ def _check_last_contig(*ts):
 
 
 def _check_shape(t, *shape):
-    _require(tuple(t.shape) == tuple(shape), "tensor must have shape (%s), got %s" % (", ".join(map(str, shape)), tuple(t.shape)))
+    if t.shape != shape:  # the message is only put together where it is needed
+        raise RuntimeError("tensor must have shape (%s), got %s" % (", ".join(map(str, shape)), tuple(t.shape)))
 
 
 def _stream(t):
-    return ctypes.c_void_p(torch.cuda.current_stream(t.device).cuda_stream)
+    return torch._C._cuda_getCurrentRawStream(t.device.index)
+
+
+class _SameDevice:
+    def __enter__(self):
+        pass
+
+    def __exit__(self, *exc):
+        pass
+
+
+_SAME_DEVICE = _SameDevice()
+
+
+def _on_device(device):
+    """torch.cuda.device(device), or nothing where that is the current device already."""
+    return _SAME_DEVICE if torch.cuda.current_device() == device.index else torch.cuda.device(device)
 
 
 def _pad8(t):
@@ -64,12 +81,22 @@ def _aligned(t):
     """The kernels read 16-byte vectors: a view whose base or strides break that is copied."""
     if t is None:
         return t
-    ok = t.data_ptr() % 16 == 0 and all(s % 8 == 0 for s in t.stride()[:-1])
-    return t if ok else t.contiguous()
+    if t.data_ptr() % 16 == 0:
+        for s in t.stride()[:-1]:
+            if s % 8:
+                return t.contiguous()
+        return t
+    return t.contiguous()
+
+
+_SM_COUNTS = {}  # device index -> number of SMs
 
 
 def _sm_count(dev):
-    return torch.cuda.get_device_properties(dev).multi_processor_count
+    n = _SM_COUNTS.get(dev.index)
+    if n is None:
+        n = _SM_COUNTS[dev.index] = torch.cuda.get_device_properties(dev).multi_processor_count
+    return n
 
 
 def _windows(is_causal, wl, wr, seqlen_k):
@@ -143,7 +170,7 @@ def fwd(q, k, v, out_, p_dropout, softmax_scale, is_causal, window_size_left, wi
     else:
         out = torch.empty((batch, seqlen_q, heads, d), dtype=q.dtype, device=q.device)
 
-    with torch.cuda.device(q.device):
+    with _on_device(q.device):
         lse = torch.empty((batch, heads, seqlen_q), dtype=torch.float32, device=q.device)
         p = None
         if return_softmax:
@@ -237,7 +264,7 @@ def varlen_fwd(q, k, v, out_, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seql
     else:
         out = torch.empty((total_q, heads, d), dtype=q.dtype, device=q.device)
 
-    with torch.cuda.device(q.device):
+    with _on_device(q.device):
         lse = torch.empty((batch, heads, max_seqlen_q), dtype=torch.float32, device=q.device)
         p = None
         if return_softmax:
@@ -334,7 +361,7 @@ def _bwd_common(varlen, dout, q, k, v, out, softmax_lse, dq_, dk_, dv_, cu_q, cu
     dk, dk_user = _grad_out(dk_, k_shape, q, "dk")
     dv, dv_user = _grad_out(dv_, k_shape, q, "dv")
 
-    with torch.cuda.device(q.device):
+    with _on_device(q.device):
         d_seqlen = _round_up(seqlen_q, 128)
         softmax_d = torch.empty((batch, heads, d_seqlen), dtype=torch.float32, device=q.device)
         seed = offset = 0
@@ -506,7 +533,7 @@ def fwd_kvcache(q, kcache, vcache, k_, v_, seqlens_k_, rotary_cos_, rotary_sin_,
         _require(batch_c >= batch, "the KV cache must hold at least `batch` sequences when cache_batch_idx is not given")
     _require(num_splits <= 128, "num_splits > 128 not supported")
 
-    with torch.cuda.device(q.device):
+    with _on_device(q.device):
         lse = torch.empty((batch, heads, seqlen_q), dtype=torch.float32, device=q.device)
         a.q, a.kcache, a.vcache, a.out = tensor3(q_p), tensor3(kc), tensor3(vc), tensor3(out)
         a.softmax_lse = ptr(lse)
