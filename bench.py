@@ -736,7 +736,7 @@ def run_train(args, wl):
     also = {"fwd": {"value": world * tf_fwd, "unit": "TFLOPS/s", "ms": ms_fwd, "kernel": "fwd_tc_kernel",
                     "frac_of_peak": tf_fwd / pk["tflops_burst"], "peak": pk["tflops_burst"], "peak_source": pk["source"]},
             "bwd": {"value": world * tf_bwd, "unit": "TFLOPS/s", "ms": ms_bwd, "frac_of_peak": tf_bwd / pk["tflops_burst"]}}
-    launches = args.steps * (5 if wide else 4)
+    launches = args.steps * (5 if wide else 3)
     if wl == DEFAULT and not args.no_also:
         for name, fn in (("decode", lambda: measure_decode(R, max(3, min(args.steps, 20)), 3)),
                          ("shapes", lambda: measure_other_shapes(R, max(2, min(args.steps, 10)))),

@@ -291,14 +291,15 @@ int fa_bwd(const FaBwdArgs* a, fa_stream_t stream) {
   const int parts = a->parts == 0 ? 3 : a->parts;  // bit 0: dot(dO, O) and dQ, bit 1: dK and dV
   FA_REQUIRE(parts >= 1 && parts <= 3, "parts must be 0 (everything), 1 (preprocess and dQ) or 2 (dK and dV)");
   FA_REQUIRE(parts == 3 || tc, "a backward pass can only be split in parts on the tensor-core path");
-  // the tensor-core path writes dq directly (two kernels: dK / dV per key block, dQ per query block)
-  int rc = (parts & 1) ? fa::bwd_pre(*a, tc ? 0 : 1, st) : 0;
+  // the tensor-core path writes dq directly (two kernels: dQ per query block, which also leaves D = rowsum(dO o O) for
+  // the second, dK / dV per key block; head dims above 128: a pass per output after a launch of its own for D)
+  int rc = (parts & 1) && !(tc && a->head_dim <= 128) ? fa::bwd_pre(*a, tc ? 0 : 1, st) : 0;
   if (rc) return rc;
   g_last_path = !tc ? "bwd_generic" : (a->head_dim > 128 ? "bwd_wide_tc" : "bwd_tc+bwd_dq_tc");
   if (tc) {
     if (a->head_dim > 128) return fa::bwd_wide_tc_main(*a, parts, st);  // one pass per output
-    if (parts & 2) rc = fa::bwd_tc_main(*a, st);
-    if (!rc && (parts & 1)) rc = fa::bwd_dq_tc_main(*a, st);
+    if (parts & 1) rc = fa::bwd_dq_tc_main(*a, st);
+    if (!rc && (parts & 2)) rc = fa::bwd_tc_main(*a, st);
     return rc;
   }
   if (a->seqlen_k > 0) {
