@@ -31,7 +31,8 @@ int bwd_tc_main(const FaBwdArgs& a, cudaStream_t st);
 // fused single-token decode
 bool decode_eligible(const FaKvcacheArgs& a);
 int decode_plan(const FaKvcacheArgs& a, int num_sms);
-int decode_run(const FaKvcacheArgs& a, int num_splits, cudaStream_t st, bool may_allocate = true);
+bool decode_rows_eligible(const FaKvcacheArgs& a);
+int decode_run(const FaKvcacheArgs& a, int num_splits, cudaStream_t st, bool may_allocate = true, int appended = 0, int causal = 0);
 int decode_noalloc_fit(const FaKvcacheArgs& a, int num_splits);
 int decode_run_noalloc(const FaKvcacheArgs& a, int num_splits, cudaStream_t st);
 size_t decode_noalloc_capacity();
@@ -401,7 +402,7 @@ int fa_kvcache_plan(const FaKvcacheArgs* a, int32_t num_sms, int64_t* lse_accum_
   if (kvcache_checks(a)) return -1;
   if (num_sms <= 0) num_sms = fa_host::sm_count();
   int splits;
-  if (!fa_host::env_flag("FA_B200_FORCE_GENERIC") && fa::decode_eligible(*a)) {
+  if (!fa_host::env_flag("FA_B200_FORCE_GENERIC") && (fa::decode_eligible(*a) || fa::decode_rows_eligible(*a))) {
     splits = fa::decode_plan(*a, num_sms);
   } else {
     splits = a->num_splits;
@@ -431,13 +432,22 @@ int fa_fwd_kvcache(const FaKvcacheArgs* a, fa_stream_t stream) {
     return fa::decode_run(*a, splits, st);
   }
   // General path: append/rotate in a first launch, then the forward on the cache.
-  const bool tc = cache_on_tensor_cores(*a);
-  g_last_path = tc ? (splits > 1 ? "kvcache_prep+fwd_tc+combine" : "kvcache_prep+fwd_tc")
+  const bool rows = !fa_host::env_flag("FA_B200_FORCE_GENERIC") && fa::decode_rows_eligible(*a);
+  const bool tc = !rows && cache_on_tensor_cores(*a);
+  g_last_path = rows ? (splits > 1 ? "kvcache_prep+decode+combine" : "kvcache_prep+decode")
+                : tc ? (splits > 1 ? "kvcache_prep+fwd_tc+combine" : "kvcache_prep+fwd_tc")
                    : (splits > 1 ? "kvcache_prep+fwd_generic+combine" : "kvcache_prep+fwd_generic");
   const bool causal_or_local = a->window_left >= 0 || a->window_right >= 0;
   FA_REQUIRE(!a->rotary_cos || a->q_rotated, "rotary needs the q_rotated scratch buffer");
   int rc = fa::kvcache_prep(*a, (causal_or_local && !a->q_rows_share_position) ? 1 : 0, st);
   if (rc) return rc;
+  if (rows) {
+    FaKvcacheArgs c = *a;
+    if (a->rotary_cos) c.q = cache_fwd_args(*a, 1).q;
+    c.rotary_cos = c.rotary_sin = nullptr;
+    c.knew.ptr = c.vnew.ptr = nullptr;
+    return fa::decode_run(c, splits, st, true, a->knew.ptr ? a->seqlen_new : 0, a->window_right == 0);
+  }
   const FaFwdArgs f = cache_fwd_args(*a, splits);
   rc = tc ? fa::fwd_tc_cache(f, a->batch_cache, st) : fa::fwd_generic(f, st);
   if (rc) return rc;

@@ -42,6 +42,8 @@ struct DecodeParams {
   FaKvcacheArgs a;
   int num_splits;
   int keys_per_split;  // multiple of kTileKeys
+  int appended;        // tokens per sequence that an earlier launch has put behind cache_seqlens (a.knew is null then)
+  int causal;          // query row s sees the keys up to the (seqlen_q - 1 - s)-th from the end
   StatusRef status;
 };
 
@@ -125,7 +127,9 @@ __device__ __forceinline__ uint4 rotated_chunk(const T* row, int d0, const T* co
   return pack8<T>(x);
 }
 
-template <typename T, int D>
+// ROWS: tokens appended by an earlier launch and / or a causal mask (an instance of its own: the two registers of the row
+// limits made the single-token one spill)
+template <typename T, int D, bool ROWS>
 __global__ void __launch_bounds__(160, 2) decode_kernel(const __grid_constant__ DecodeParams P) {
   using C = DCfg<D>;
   const FaKvcacheArgs& a = P.a;
@@ -144,8 +148,8 @@ __global__ void __launch_bounds__(160, 2) decode_kernel(const __grid_constant__ 
   const int group = a.heads / a.heads_k;
   const int M = a.seqlen_q * group;  // query rows that share this KV head (<= 16)
   const int L = a.cache_seqlens ? a.cache_seqlens[b] : a.seqlen_cache;
-  const bool has_new = a.knew.ptr != nullptr;
-  const int Ltot = min(L + (has_new ? 1 : 0), a.seqlen_cache);
+  const bool has_new = !ROWS && a.knew.ptr != nullptr;
+  const int Ltot = min(L + (ROWS ? P.appended : has_new ? 1 : 0), a.seqlen_cache);
   const int cb = a.cache_batch_idx ? a.cache_batch_idx[b] : b;
   // paged cache: the tensor maps describe (page, row in page); a 64-key tile never straddles a page
   const int32_t* pages = a.block_table ? a.block_table + (int64_t)b * a.block_table_stride : nullptr;
@@ -235,6 +239,9 @@ __global__ void __launch_bounds__(160, 2) decode_kernel(const __grid_constant__ 
   for (int i = 0; i < D / 8; ++i) o_acc[i][0] = o_acc[i][1] = o_acc[i][2] = o_acc[i][3] = 0.f;
   float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
   const float scale_log2 = a.softmax_scale * kLog2e;
+  int lim[2];  // first key that rows g and g + 8 of this thread do not see
+#pragma unroll
+  for (int r = 0; r < 2; ++r) lim[r] = ROWS && P.causal ? Ltot - (a.seqlen_q - 1) + min((g + 8 * r) / group, a.seqlen_q - 1) : Ltot;
   bool ok = true;
   int rdv_phase = 0;
   // bounded rendezvous of the consumer warps (instead of bar.sync, which could strand a warp if
@@ -307,7 +314,7 @@ __global__ void __launch_bounds__(160, 2) decode_kernel(const __grid_constant__ 
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int key = key0 + warp * 16 + nt * 8 + 2 * t + (e & 1);
-        const float x = key < Ltot ? s[nt][e] * scale_log2 : -INFINITY;
+        const float x = key < lim[e >> 1] ? s[nt][e] * scale_log2 : -INFINITY;
         s[nt][e] = x;
         mx[e >> 1] = fmaxf(mx[e >> 1], x);
       }
@@ -418,19 +425,23 @@ __global__ void __launch_bounds__(160, 2) decode_kernel(const __grid_constant__ 
 }
 
 template <typename T, int D>
-int launch_decode(const FaKvcacheArgs& a, int num_splits, int keys_per_split, cudaStream_t st, bool may_allocate) {
+int launch_decode(const FaKvcacheArgs& a, int num_splits, int keys_per_split, cudaStream_t st, bool may_allocate, int appended,
+                  int causal) {
   using C = DCfg<D>;
   DecodeParams P;
   P.a = a;
   P.num_splits = num_splits;
   P.keys_per_split = keys_per_split;
+  P.appended = appended;
+  P.causal = causal;
   const int slab_rows = a.block_table ? a.page_block_size : a.seqlen_cache;  // rows of one page / of one sequence's cache
   if (make_tmap_4d(&P.tk, a.kcache, a.dtype, slab_rows, a.heads_k, a.batch_cache, a.head_dim, kTileKeys)) return 1;
   if (make_tmap_4d(&P.tv, a.vcache, a.dtype, slab_rows, a.heads_k, a.batch_cache, a.head_dim, kTileKeys)) return 1;
-  auto kern = decode_kernel<T, D>;
+  const bool rows = appended > 0 || causal;
+  auto kern = rows ? decode_kernel<T, D, true> : decode_kernel<T, D, false>;
   P.status = status_ref(may_allocate);
-  static fa_host::DeviceOnce once;
-  if (int rc = fa_host::raise_smem_limit(once, reinterpret_cast<const void*>(kern), C::SMEM_BYTES, "decode_kernel")) return rc;
+  static fa_host::DeviceOnce once[2];
+  if (int rc = fa_host::raise_smem_limit(once[rows], reinterpret_cast<const void*>(kern), C::SMEM_BYTES, "decode_kernel")) return rc;
   dim3 grid(num_splits, a.heads_k, a.batch);
   kern<<<grid, 160, C::SMEM_BYTES, st>>>(P);
   return fa_host::check_launch("decode_kernel");
@@ -446,16 +457,31 @@ int keys_per_split_of(const FaKvcacheArgs& a, int num_splits) {
 int combine(const float* out_parts, const float* lse_parts, const FaTensor& out, float* lse, int lse_pitch, int n_parts,
             int B, int H, int S, int D, int dtype, cudaStream_t st);
 
-bool decode_eligible(const FaKvcacheArgs& a) {
+// What both uses of the kernel need: few rows per KV head, a tile the tensor maps can describe
+static bool decode_shape(const FaKvcacheArgs& a) {
   if (a.head_dim != 64 && a.head_dim != 128) return false;
-  if (a.window_left >= 0 || a.window_right >= 0) return false;
   const int group = a.heads / a.heads_k;
   if (a.seqlen_q * group > kMaxRows || a.seqlen_q < 1) return false;
-  if (a.knew.ptr && a.seqlen_new != 1) return false;
-  if (a.rotary_cos && (a.rotary_dim % 16 != 0 || a.rotary_dim > a.head_dim)) return false;
   if (!tma_compatible(a.kcache) || !tma_compatible(a.vcache)) return false;
   if (a.seqlen_cache <= 0) return false;
   return encode_tiled_fn() != nullptr;
+}
+
+bool decode_eligible(const FaKvcacheArgs& a) {
+  if (!decode_shape(a)) return false;
+  if (a.window_left >= 0 || a.window_right >= 0) return false;
+  if (a.knew.ptr && a.seqlen_new != 1) return false;
+  if (a.rotary_cos && (a.rotary_dim % 16 != 0 || a.rotary_dim > a.head_dim)) return false;
+  return true;
+}
+
+// Several tokens per sequence, appended (and q rotated) by kvcache_prep before this kernel reads the cache: any number of
+// new tokens, and the causal mask (a window whose left side reaches every key).  Speculative decoding's drafts are such
+// calls; the any-shape kernel walks the cache once per query head and fills 5 of its 64 rows with 5 tokens.
+bool decode_rows_eligible(const FaKvcacheArgs& a) {
+  if (!decode_shape(a)) return false;
+  if (a.window_left < 0 && a.window_right < 0) return true;
+  return a.window_right == 0 && (a.window_left < 0 || a.window_left >= a.seqlen_cache);
 }
 
 int decode_plan(const FaKvcacheArgs& a, int num_sms) {
@@ -480,14 +506,14 @@ int decode_plan(const FaKvcacheArgs& a, int num_sms) {
   return splits;
 }
 
-int decode_run(const FaKvcacheArgs& a, int num_splits, cudaStream_t st, bool may_allocate) {
+int decode_run(const FaKvcacheArgs& a, int num_splits, cudaStream_t st, bool may_allocate, int appended, int causal) {
   const int kps = keys_per_split_of(a, num_splits);
   const bool bf = a.dtype == FA_DTYPE_BF16;
   int rc;
   if (a.head_dim == 64)
-    rc = bf ? launch_decode<__nv_bfloat16, 64>(a, num_splits, kps, st, may_allocate) : launch_decode<__half, 64>(a, num_splits, kps, st, may_allocate);
+    rc = bf ? launch_decode<__nv_bfloat16, 64>(a, num_splits, kps, st, may_allocate, appended, causal) : launch_decode<__half, 64>(a, num_splits, kps, st, may_allocate, appended, causal);
   else
-    rc = bf ? launch_decode<__nv_bfloat16, 128>(a, num_splits, kps, st, may_allocate) : launch_decode<__half, 128>(a, num_splits, kps, st, may_allocate);
+    rc = bf ? launch_decode<__nv_bfloat16, 128>(a, num_splits, kps, st, may_allocate, appended, causal) : launch_decode<__half, 128>(a, num_splits, kps, st, may_allocate, appended, causal);
   if (rc) return rc;
   if (num_splits > 1)
     return combine(a.out_accum, a.lse_accum, a.out, a.softmax_lse, a.seqlen_q, num_splits, a.batch, a.heads, a.seqlen_q,
@@ -565,7 +591,7 @@ int decode_run_noalloc(const FaKvcacheArgs& a, int num_splits, cudaStream_t st) 
     b.lse_accum = reinterpret_cast<float*>(base);
     b.out_accum = reinterpret_cast<float*>(base + lse_bytes);
   }
-  return decode_run(b, num_splits, st, /*may_allocate=*/false);
+  return decode_run(b, num_splits, st, /*may_allocate=*/false, 0, 0);
 }
 
 }  // namespace fa

@@ -82,3 +82,41 @@ def test_tiles_shared_by_the_heads_of_a_group(sq, sk, heads, heads_k, d, causal,
         hidden = hidden | (j < i - window[0])
     want = torch.logsumexp(s.masked_fill(hidden, float("-inf")), -1)
     assert torch.allclose(lse, want.masked_fill(want == float("-inf"), float("inf")), atol=1e-3)
+
+
+@pytest.mark.parametrize("num_splits", [0, 1, 5])
+@pytest.mark.parametrize("page", [0, 64])
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("sq,new,heads,heads_k,d,dtype", [
+    (2, 2, 8, 1, 128, torch.bfloat16),   # all 16 rows of the tile
+    (5, 5, 6, 2, 64, torch.float16),     # 15 rows
+    (16, 16, 2, 2, 128, torch.bfloat16),
+    (1, 3, 4, 2, 64, torch.bfloat16),    # more new tokens than queries
+    (4, 0, 4, 2, 128, torch.float16),    # queries against what the cache holds
+])
+def test_a_few_tokens_per_sequence(sq, new, heads, heads_k, d, dtype, causal, page, num_splits):
+    g = torch.Generator().manual_seed(sq + d)
+    cap, B = 512, 5
+    lens = [max(0, sq - new), 64 - new if new else 64, 65, 200, cap - new]
+    q = torch.randn(B, sq, heads, d, generator=g).to(dtype).cuda()
+    kn, vn = (torch.randn(B, new, heads_k, d, generator=g).to(dtype).cuda() if new else None for _ in range(2))
+    kc = torch.randn(B, cap, heads_k, d, generator=g).to(dtype).cuda()
+    vc = torch.randn(B, cap, heads_k, d, generator=g).to(dtype).cuda()
+    lens_t = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    kw = dict(cache_seqlens=lens_t, causal=causal)
+    out_t, kc_t, vc_t = O.kvcache_oracle(q, kc, vc, kn, vn, None, None, **kw)
+    out_l, _, _ = O.kvcache_oracle(q, kc, vc, kn, vn, None, None, upcast=False, reorder_ops=True, **kw)
+    used = torch.arange(cap, device="cuda")[None] < lens_t[:, None] + new
+    kc[~used], vc[~used] = float("nan"), float("nan")
+    kp, vp = kc.clone(), vc.clone()
+    if page:
+        perm = torch.randperm(B * cap // page, generator=g).cuda()
+        kp, vp = torch.empty_like(kc).view(-1, page, heads_k, d), torch.empty_like(vc).view(-1, page, heads_k, d)
+        kp[perm], vp[perm] = kc.view(-1, page, heads_k, d), vc.view(-1, page, heads_k, d)
+        kw["block_table"] = perm.view(B, cap // page).int()
+    out = fa.flash_attn_with_kvcache(q, kp, vp, kn, vn, num_splits=num_splits, **kw)
+    assert "decode" in _lib.last_path(), _lib.last_path()
+    assert_within(out, out_t, out_l, mult=3, what="out")
+    if page:
+        kp, vp = (t[perm].view(B, cap, heads_k, d) for t in (kp, vp))
+    assert torch.equal(kp[used], kc_t[used]) and torch.equal(vp[used], vc_t[used])
