@@ -248,6 +248,8 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
     // ------------------------------------------------------------------ softmax warpgroups
     setmaxnreg_inc<216>();
     const int t = warp >> 2;
+    const int lo_t = t ? lo[1] : lo[0], hi_t = t ? hi[1] : hi[0];  // (indexing by t would put the arrays into local memory)
+    const bool active_t = t ? active[1] : active[0];
     const int row_in_tile = (warp & 3) * 32 + lane;
     const int m0 = m_base + t * tile_pos;
     const int pos_in_tile = (row_in_tile * pack_inv) >> 16;             // row_in_tile / pack
@@ -266,8 +268,8 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
 
     const uint64_t scale2 = pack2(scale_log2, scale_log2);
     uint64_t l_sum2 = pack2(0.f, 0.f);  // two running partial row sums (even / odd columns)
-    for (int j = lo[t]; j < hi[t] && ok; ++j) {
-      const int it = j - lo[t];
+    for (int j = lo_t; j < hi_t && ok; ++j) {
+      const int it = j - lo_t;
       const bool first_block = it == 0;
       ok = mbar_wait(bar_sfull(t), it & 1, W_SFULL, abort_flag);
       if (!ok) break;
@@ -391,17 +393,18 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
     }
 
     // ---- epilogue: O / l -> shared (swizzled) -> coalesced global stores; LSE
-    if (active[t]) {
-      const int n_it = hi[t] - lo[t];
+    if (active_t) {
+      const int n_it = hi_t - lo_t;
       bool have_o = n_it > 0 && ok;
       if (have_o) {
         ok = mbar_wait(bar_ofull(t), (n_it - 1) & 1, W_OFULL, abort_flag);
         have_o = ok;
         tc_fence_after();
       }
+      float inv = 0.f;
       if (ok) {
         const bool empty = !(l_sum > 0.f) || m_used == -INFINITY;
-        const float inv = empty ? 0.f : 1.f / l_sum;
+        inv = empty ? 0.f : 1.f / l_sum;
         const float lse = empty ? INFINITY : (m_used + log2f(l_sum)) * kLn2;
         if (row_valid) {
           if (P.num_splits > 1)  // the split workspaces are (split, batch, head, row): not packed, -inf marks an empty part
@@ -409,69 +412,89 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
           else
             a.softmax_lse[((int64_t)b * a.heads + head) * a.lse_seqlen + row] = lse;
         }
-        unsigned char* stage = smem + t * C::TILE_BYTES;  // the Q tile of this warpgroup is no longer read
-        constexpr int ROWB = DH * 2;
-        // O leaves tensor memory 128 columns per round trip (a trip costs ~250 cycles whatever its size)
-        constexpr int OB = DH < 128 ? DH : 128;
-        uint32_t ob[OB / 32][32];
+      }
+      unsigned char* stage = smem + t * C::TILE_BYTES;  // the Q tile of this warpgroup is no longer read
+      const int tid = threadIdx.x & 127;
+      if (P.num_splits > 1) {
+        // normalised fp32 partial, as many columns at a time as fit the Q tile, through shared memory (a row per thread,
+        // straight from the registers, put every store of a warp in 32 lines); an empty part is not written: its weight is 0
+        constexpr int SC = DH > 64 ? 64 : 32, PPR = SC / 4;  // columns at a time, 16-byte pieces of them per row
+        static_assert(kBM * SC * 4 <= C::TILE_BYTES, "the staged part of O");
+#pragma unroll 1
+        for (int c0 = 0; c0 < DH; c0 += SC) {
+          if (have_o) {
 #pragma unroll
-        for (int c0 = 0; c0 < DH; c0 += 32) {
-          if (c0 % OB == 0) {
-            if (have_o) {
-#pragma unroll
-              for (int c = 0; c < OB; c += 32) tmem_ld32(tO + c0 + c, ob[c / 32]);
+            for (int half = 0; half < SC; half += 32) {
+              uint32_t o[32];
+              tmem_ld32(tO + c0 + half, o);
               tmem_wait_ld();
-            } else {
-#pragma unroll
-              for (int c = 0; c < OB / 32; ++c)
-#pragma unroll
-                for (int i = 0; i < 32; ++i) ob[c][i] = 0u;
-            }
-          }
-          const uint32_t(&o)[32] = ob[(c0 % OB) / 32];
-          if (P.num_splits > 1) {  // normalised fp32 partial, straight from the registers (rows are contiguous)
-            if (row_valid && have_o) {  // an empty part is not read: its weight is zero
-              float* oa = a.out_accum +
-                          (((int64_t)split * a.batch * a.heads + (int64_t)b * a.heads + head) * a.seqlen_q + row) * a.head_dim;
 #pragma unroll
               for (int i = 0; i < 32; i += 4)
-                if (c0 + i < a.head_dim)
-                  *reinterpret_cast<float4*>(oa + c0 + i) =
-                      make_float4(__uint_as_float(o[i]) * inv, __uint_as_float(o[i + 1]) * inv,
-                                  __uint_as_float(o[i + 2]) * inv, __uint_as_float(o[i + 3]) * inv);
+                *reinterpret_cast<float4*>(stage + row_in_tile * (SC * 4) + (((half + i) / 4 ^ (row_in_tile & 7)) << 4)) =
+                    make_float4(__uint_as_float(o[i]) * inv, __uint_as_float(o[i + 1]) * inv, __uint_as_float(o[i + 2]) * inv,
+                                __uint_as_float(o[i + 3]) * inv);
             }
-            continue;
           }
+          named_bar_sync(1 + t, 128);
+          const int piece = tid % PPR, col = c0 + piece * 4;
+          if (have_o && col < a.head_dim) {
+#pragma unroll 4
+            for (int r = tid / PPR; r < kBM; r += 128 / PPR) {
+              const int rp = (r * pack_inv) >> 16;  // r / pack
+              if (rp < tile_pos && m0 + rp < si.sq)
+                *reinterpret_cast<float4*>(a.out_accum + (((int64_t)split * a.batch * a.heads + (int64_t)b * a.heads + h + r - rp * pack) *
+                                                              a.seqlen_q + m0 + rp) * a.head_dim + col) =
+                    *reinterpret_cast<const float4*>(stage + r * (SC * 4) + ((piece ^ (r & 7)) << 4));
+            }
+          }
+          named_bar_sync(1 + t, 128);
+        }
+      } else {
+        if (ok) {
+          constexpr int ROWB = DH * 2;
+          // O leaves tensor memory 128 columns per round trip (a trip costs ~250 cycles whatever its size)
+          constexpr int OB = DH < 128 ? DH : 128;
+          uint32_t ob[OB / 32][32];
 #pragma unroll
-          for (int q4 = 0; q4 < 4; ++q4) {  // four 16-byte chunks of 8 elements
-            uint4 pk;
-            pk.x = Pack<T>::two(__uint_as_float(o[q4 * 8 + 0]) * inv, __uint_as_float(o[q4 * 8 + 1]) * inv);
-            pk.y = Pack<T>::two(__uint_as_float(o[q4 * 8 + 2]) * inv, __uint_as_float(o[q4 * 8 + 3]) * inv);
-            pk.z = Pack<T>::two(__uint_as_float(o[q4 * 8 + 4]) * inv, __uint_as_float(o[q4 * 8 + 5]) * inv);
-            pk.w = Pack<T>::two(__uint_as_float(o[q4 * 8 + 6]) * inv, __uint_as_float(o[q4 * 8 + 7]) * inv);
-            const int chunk = c0 / 8 + q4;
-            const int phys = (chunk & ~7) | ((chunk ^ row_in_tile) & 7);
-            *reinterpret_cast<uint4*>(stage + row_in_tile * ROWB + phys * 16) = pk;
+          for (int c0 = 0; c0 < DH; c0 += 32) {
+            if (c0 % OB == 0) {
+              if (have_o) {
+#pragma unroll
+                for (int c = 0; c < OB; c += 32) tmem_ld32(tO + c0 + c, ob[c / 32]);
+                tmem_wait_ld();
+              } else {
+#pragma unroll
+                for (int c = 0; c < OB / 32; ++c)
+#pragma unroll
+                  for (int i = 0; i < 32; ++i) ob[c][i] = 0u;
+              }
+            }
+            const uint32_t(&o)[32] = ob[(c0 % OB) / 32];
+#pragma unroll
+            for (int q4 = 0; q4 < 4; ++q4) {  // four 16-byte chunks of 8 elements
+              uint4 pk;
+              pk.x = Pack<T>::two(__uint_as_float(o[q4 * 8 + 0]) * inv, __uint_as_float(o[q4 * 8 + 1]) * inv);
+              pk.y = Pack<T>::two(__uint_as_float(o[q4 * 8 + 2]) * inv, __uint_as_float(o[q4 * 8 + 3]) * inv);
+              pk.z = Pack<T>::two(__uint_as_float(o[q4 * 8 + 4]) * inv, __uint_as_float(o[q4 * 8 + 5]) * inv);
+              pk.w = Pack<T>::two(__uint_as_float(o[q4 * 8 + 6]) * inv, __uint_as_float(o[q4 * 8 + 7]) * inv);
+              const int chunk = c0 / 8 + q4;
+              const int phys = (chunk & ~7) | ((chunk ^ row_in_tile) & 7);
+              *reinterpret_cast<uint4*>(stage + row_in_tile * ROWB + phys * 16) = pk;
+            }
           }
         }
-      }
-      named_bar_sync(1 + t, 128);
-      if (ok && P.num_splits <= 1) {
+        named_bar_sync(1 + t, 128);
         constexpr int CPR = DH / 8;  // 16-byte chunks per row
-        const int tid = threadIdx.x & 127;
-        unsigned char* stage = smem + t * C::TILE_BYTES;
-        T* og = reinterpret_cast<T*>(a.out.ptr) + si.q_batch * a.out.stride_b + si.q_row0 * a.out.stride_s +
-                (int64_t)h * a.out.stride_h;
+        const int chunk = tid % CPR;
+        if (ok && chunk * 8 < a.head_dim) {
+          T* og = reinterpret_cast<T*>(a.out.ptr) + si.q_batch * a.out.stride_b + (si.q_row0 + m0) * a.out.stride_s +
+                  (int64_t)h * a.out.stride_h + chunk * 8;
 #pragma unroll 4
-        for (int i = tid; i < kBM * CPR; i += 128) {
-          const int r = i / CPR, chunk = i % CPR;
-          const int rp = (r * pack_inv) >> 16;  // r / pack
-          const int grow_ = m0 + rp;
-          if (rp < tile_pos && grow_ < si.sq) {
-            const int phys = (chunk & ~7) | ((chunk ^ r) & 7);
-            uint4 v = *reinterpret_cast<const uint4*>(stage + r * (DH * 2) + phys * 16);
-            if (chunk * 8 < a.head_dim) 
-              *reinterpret_cast<uint4*>(og + (int64_t)grow_ * a.out.stride_s + (r - rp * pack) * a.out.stride_h + chunk * 8) = v;
+          for (int r = tid / CPR; r < kBM; r += 128 / CPR) {
+            const int rp = (r * pack_inv) >> 16;  // r / pack
+            if (rp < tile_pos && m0 + rp < si.sq)
+              *reinterpret_cast<uint4*>(og + rp * a.out.stride_s + (r - rp * pack) * a.out.stride_h) =
+                  *reinterpret_cast<const uint4*>(stage + r * (DH * 2) + (((chunk & ~7) | ((chunk ^ r) & 7)) << 4));
           }
         }
       }
