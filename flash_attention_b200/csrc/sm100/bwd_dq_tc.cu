@@ -16,7 +16,7 @@
 // and at most 113 KiB: two CTAs share an SM, and one's waits, start and end run under the other's blocks.  An N = 64 SS MMA
 // takes 48 cycles against 32 of math (it reads its A slice for half the columns); on long sequences that eats what
 // the second CTA gives.  16 x 2048 tokens, with D: 16 heads of 128 causal 455 + 47 -> 440 us, 32 heads of 64 full
-// 1186 + 47 -> 950 us; 32768 tokens causal 10354 + 98 -> 10390 us.
+// 1186 + 47 -> 906 us (two buffers of dS of its own, so that dP(j+1) need not wait for dQ(j): 948); 32768 tokens causal 10354 + 98 -> 10390 us.
 //
 // Warps: 0-7 compute (warpgroup w handles key columns [32w, 32w+32) of the block; in the epilogue,
 // head-dim columns [D/2*w, ...)), 8 = TMA producer, 9 = MMA issuer, 10 = TMEM owner, 11 = issuer of dQ.
@@ -60,9 +60,7 @@ struct QCfg {
   static constexpr int NBAR = 2 * NSK + 2 * NSV + 8;
   static constexpr int OFF_D = OFF_BAR + NBAR * 8 + 32;  // D of the 128 rows, fp32
   static constexpr int SMEM_BYTES = OFF_D + kM * 4;
-  // dS (16-bit): two buffers of its own where the 256 columns have room for them (head dim 64), else over dP
-  static constexpr bool OWN_DS = DH <= 64;
-  static constexpr int COL_S = 0, COL_DP = kN, COL_DQ = 2 * kN, COL_DS = 2 * kN + DH;
+  static constexpr int COL_S = 0, COL_DP = kN, COL_DQ = 2 * kN;  // dS (16-bit) goes over dP
   static constexpr int TMEM_COLS = 256;
 };
 
@@ -102,7 +100,7 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_dq_tc_kernel(const __grid_con
   auto bar_v_empty = [&](int st) { return bar0 + 8 * (2 * NSK + NSV + st); };
   constexpr int kB0 = 2 * NSK + 2 * NSV;
   const uint32_t bar_s = bar0 + 8 * kB0, bar_sread = bar0 + 8 * (kB0 + 1), bar_q = bar0 + 8 * (kB0 + 2), bar_do = bar0 + 8 * (kB0 + 6),
-                 bar_dp = bar0 + 8 * (kB0 + 3), bar_ds = bar0 + 8 * (kB0 + 4), bar_dpread = bar0 + 8 * (kB0 + 7), bar_done = bar0 + 8 * (kB0 + 5);
+                 bar_dp = bar0 + 8 * (kB0 + 3), bar_ds = bar0 + 8 * (kB0 + 4), bar_done = bar0 + 8 * (kB0 + 5);
   volatile uint32_t* tmem_ptr_smem = reinterpret_cast<volatile uint32_t*>(smem + C::OFF_BAR + C::NBAR * 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + C::OFF_BAR + C::NBAR * 8 + 4);
 
@@ -148,7 +146,6 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_dq_tc_kernel(const __grid_con
     mbar_init(bar_do, 1);
     mbar_init(bar_dp, 1);
     mbar_init(bar_ds, kCompute);
-    mbar_init(bar_dpread, kCompute);
     mbar_init(bar_done, 1);
     fence_barrier_init();
     fence_proxy_async();
@@ -264,7 +261,7 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_dq_tc_kernel(const __grid_con
 #pragma unroll
         for (int c = 0; c < 32; ++c) p[c] = (c >= c_lo && c <= c_hi) ? p[c] : 0.f;
       }
-      // ---- dS = P o (dP - D), 16-bit, over this warp's own, now read, columns of dP (or in its buffer)
+      // ---- dS = P o (dP - D), 16-bit, over this warp's own, now read, columns of dP
       ok = mbar_wait(bar_dp, j & 1, W_Q_DP, abort_flag);
       if (!ok) break;
       tc_fence_after();
@@ -272,25 +269,13 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_dq_tc_kernel(const __grid_con
         uint32_t d[32], pk[16];
         tmem_ld32(tdP, d);
         tmem_wait_ld();
-        if constexpr (C::OWN_DS) {
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bar_dpread);  // dP(j) is in registers: dP(j+1) may overwrite it
-        }
 #pragma unroll
         for (int c = 0; c < 32; c += 2) {
           float x0, x1;
           unpack2(mul2(pack2(p[c], p[c + 1]), add2(pack2u(d[c], d[c + 1]), neg_d2)), x0, x1);
           pk[c >> 1] = Pack<T>::two(x0, x1);
         }
-        if constexpr (C::OWN_DS) {
-          // the buffer held dS(j-2): dQ(j-2), whose commit releases that block's K tile, must have read it
-          if (j >= 2) ok = mbar_wait(bar_k_empty((j - 2) % NSK), ((j - 2) / NSK) & 1, W_Q_KV_EMPTY, abort_flag);
-          if (!ok) break;
-          tmem_st16(tmem + lane_off + C::COL_DS + (j & 1) * 32 + w * 16, pk);
-        } else {
-          tmem_st16(tdP, pk);
-        }
+        tmem_st16(tdP, pk);
       }
       tmem_wait_st();
       tc_fence_before();
@@ -357,9 +342,8 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_dq_tc_kernel(const __grid_con
       }
     } else if (warp == kWarpMma || warp == kWarpMmaDq) {
       // -------------------------------------------------------------- MMA issuer
-      // Warp 9 issues S(j+1) as soon as the compute warps hold S(j) in registers.  Head dim 128: warp 11 issues the chain
-      // dQ(j) | dP(j+1): dS(j) sits over dP(j), and the MMAs of one thread execute in order.  Head dim 64: dS has buffers
-      // of its own, so warp 9 issues dP(j+1) too, once dP(j) is in registers, and dQ(j) is not in front of it.  MMAs of the two threads are
+      // Warp 9 issues S(j+1) as soon as the compute warps hold S(j) in registers; warp 11 issues the chain
+      // dQ(j) | dP(j+1): dS(j) sits over dP(j), and the MMAs of one thread execute in order.  MMAs of the two threads are
       // not ordered among themselves and need not be.
       if (run) {  // the whole warp runs the loops (see mma_ss_w); one elected lane issues
         constexpr int F = QFmt<T>::kIdesc;
@@ -381,16 +365,6 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_dq_tc_kernel(const __grid_con
           for (int kk = 0; kk < DH / 16; ++kk) mma_ss_w(tmem + d_col, dsc(a_lo + koff_m(kk)), dsc(b_lo + koff_n(kk)), idesc_s, kk > 0);
           tc_commit_w(bar);
         };
-        auto issue_dp = [&](int i) {
-          const int vs = i % NSV;
-          const bool k = mbar_wait_w(bar_v_full(vs), (i / NSV) & 1, W_Q_KV_FULL, abort_flag);
-          if (k) {
-            tc_fence_after();
-            issue_s(C::COL_DP, oDO, oV + vs * kTile16, bar_dp);
-            tc_commit_w(bar_v_empty(vs));
-          }
-          return k;
-        };
         if (warp == kWarpMma) {
           bool ok = mbar_wait_w(bar_q, 0, W_Q_QDO, abort_flag);
           for (int j = 0; j < iters && ok; ++j) {
@@ -400,17 +374,20 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_dq_tc_kernel(const __grid_con
             if (!ok) break;
             tc_fence_after();
             issue_s(C::COL_S, oQ, oK + ks * kTile16, bar_s);
-            if constexpr (C::OWN_DS) {
-              ok = j > 0 ? mbar_wait_w(bar_dpread, (j - 1) & 1, W_Q_DP, abort_flag) : mbar_wait_w(bar_do, 0, W_Q_QDO, abort_flag);
-              if (ok) ok = issue_dp(j);
-            }
           }
         } else {
-          bool ok = true;
-          if constexpr (!C::OWN_DS) {
-            ok = mbar_wait_w(bar_do, 0, W_Q_QDO, abort_flag);
-            if (ok) ok = issue_dp(0);
-          }
+          auto issue_dp = [&](int i) {
+            const int vs = i % NSV;
+            const bool k = mbar_wait_w(bar_v_full(vs), (i / NSV) & 1, W_Q_KV_FULL, abort_flag);
+            if (k) {
+              tc_fence_after();
+              issue_s(C::COL_DP, oDO, oV + vs * kTile16, bar_dp);
+              tc_commit_w(bar_v_empty(vs));
+            }
+            return k;
+          };
+          bool ok = mbar_wait_w(bar_do, 0, W_Q_QDO, abort_flag);
+          if (ok) ok = issue_dp(0);
           for (int j = 0; j < iters && ok; ++j) {
             const int ks = j % NSK;
             // dS(j) is in TMEM: dQ += dS K.  Its commit releases the K tile, which S(j) of the other issuer read as well:
@@ -420,11 +397,10 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_dq_tc_kernel(const __grid_con
             tc_fence_after();
 #pragma unroll
             for (int kk = 0; kk < kN / 16; ++kk)
-              mma_ts_w(tmem + C::COL_DQ,
-                       tmem + (C::OWN_DS ? C::COL_DS + (j & 1) * 32 + kk * 8 : C::COL_DP + (kk >> 1) * 32 + (kk & 1) * 8),
-                       dsc(oK + ks * kTile16 + moff(kk)), idesc_dq, (j > 0) || kk > 0);
+              mma_ts_w(tmem + C::COL_DQ, tmem + C::COL_DP + (kk >> 1) * 32 + (kk & 1) * 8, dsc(oK + ks * kTile16 + moff(kk)),
+                       idesc_dq, (j > 0) || kk > 0);
             tc_commit_w(bar_k_empty(ks));
-            if (!C::OWN_DS && j + 1 < iters) ok = issue_dp(j + 1);
+            if (j + 1 < iters) ok = issue_dp(j + 1);
           }
           if (ok) tc_commit_w(bar_done);
         }
@@ -462,7 +438,8 @@ int launch_bwd_dq_tc(const FaBwdArgs& a, cudaStream_t st) {
   P.status = status_ref(true);
   static fa_host::DeviceOnce once;
   if (int rc = fa_host::raise_smem_limit(once, reinterpret_cast<const void*>(kern), C::SMEM_BYTES, "bwd_dq_tc_kernel")) return rc;
-  dim3 grid((a.seqlen_q + kM - 1) / kM, a.heads, a.batch);
+  const int rows = a.d_seqlen > a.seqlen_q ? a.d_seqlen : a.seqlen_q;  // the padding rows of D are written too
+  dim3 grid((rows + kM - 1) / kM, a.heads, a.batch);
   kern<<<grid, kThreads, C::SMEM_BYTES, st>>>(P);
   return fa_host::check_launch("bwd_dq_tc_kernel");
 }

@@ -16,7 +16,7 @@
 //   S^T  = K Q^T          (lanes = keys, columns = queries)            SS MMA  -> TMEM tS
 //   dP^T = V dO^T                                                       SS MMA  -> TMEM tdP
 //   P^T  = exp2(S^T*scale*log2e - LSE*log2e)        one thread per key  -> TMEM (16-bit, over tdP)
-//   dS^T = P^T o (dP^T - D)                                             -> TMEM (over tdP) or shared memory
+//   dS^T = P^T o (dP^T - D)                                             -> TMEM (16-bit, over tdP)
 //   dV  += P^T  dO        A = P^T from TMEM, B = dO tile (MN-major)     -> TMEM tdV
 //   dK  += dS^T Q         A = dS^T, B = Q tile (MN-major)                -> TMEM tdK
 //
@@ -26,9 +26,10 @@
 //   power cap on long sequences), and so was dS in shared memory (the Q ring shrinks to two slots, S(i+1) waits for Q).
 //   Head dim 64: half the tile rows, 256 columns and 113 KiB, so that two CTAs share an SM and one's waits, start and end
 //   run under the other's blocks; the exponentials (16 per clock and SM: 1024 cycles per 128 x 128) come next.
+//   (dS in shared memory, so that dP(i+1) need not wait for dK(i), was slower: 1084 -> 1210 us below.)
 //   Start and end: the first loads leave before the CTA has set itself up, and the result leaves in whole rows through
 //   shared memory (a row per thread cost 7700 cycles per CTA at head dim 128, it is 4300 now).
-// 16 x 2048 tokens: 16 heads of 128 causal 602 -> 535 us, 32 heads of 64 full 1509 -> 1096 us.
+// 16 x 2048 tokens: 16 heads of 128 causal 602 -> 535 us, 32 heads of 64 full 1509 -> 1090 us.
 //
 // Warps: 0-7 compute (warpgroup w handles the half w of a block's query columns; in the epilogue, of the head dim),
 // 8 = TMA producer, 9 = MMA issuer, 10 = loader of the per-row LSE / D vectors and TMEM owner, 11 = issuer of S.
@@ -67,15 +68,12 @@ struct BCfg {
   static constexpr int REGS = DH > 64 ? 200 : 88, REGS_OTHER = DH > 64 ? 104 : 64;
   static_assert(256 * REGS + 128 * REGS_OTHER <= THREADS * (DH > 64 ? 168 : 80), "the registers of one CTA");
   // Q(i) is needed from S^T(i) (issued a block early) to dK(i), dO(i) from dP^T(i) to dV(i): Q gets the deeper ring
-  static constexpr int NSQ = 3, NSO = DH > 64 ? 2 : 4;
-  // Head dim 64: dS^T goes to shared memory, where there is room for it, so that dP^T(i+1) waits for dV(i) only
-  static constexpr bool DS_SMEM = DH <= 64;
+  static constexpr int NSQ = DH > 64 ? 3 : 4, NSO = DH > 64 ? 2 : 4;
   static constexpr int OFF_K = 0;
   static constexpr int OFF_V = TILE_K;
   static constexpr int OFF_Q = 2 * TILE_K;
   static constexpr int OFF_DO = OFF_Q + NSQ * TILE_Q;
-  static constexpr int OFF_DS = OFF_DO + NSO * TILE_Q;                     // dS^T: 128 keys x 64 queries, K-major
-  static constexpr int OFF_STATS = OFF_DS + (DS_SMEM ? kChunkBytes : 0);  // 2 slots x (BQ -lse2, BQ -dsum) fp32
+  static constexpr int OFF_STATS = OFF_DO + NSO * TILE_Q;  // 2 slots x (BQ -lse2, BQ -dsum) fp32
   static constexpr int OFF_BAR = OFF_STATS + 2 * 2 * BQ * 4;
   static constexpr int NBAR = 2 * NSQ + 2 * NSO + 11;
   static constexpr int SMEM_BYTES = OFF_BAR + NBAR * 8 + 32;
@@ -299,22 +297,13 @@ __global__ void __launch_bounds__(BCfg<DH>::THREADS, BCfg<DH>::CTAS) bwd_tc_kern
           dk[c >> 1] = Pack<T>::two(x0, x1);
           dk[(c >> 1) + 1] = Pack<T>::two(x2, x3);
         }
-        if constexpr (C::DS_SMEM) {
-          // dK(it-1) has read dS^T(it-1)
-          if (it > 0) ok = mbar_wait(bar_q_empty((it - 1) % NSQ), ((it - 1) / NSQ) & 1, W_B_QDO_EMPTY, abort_flag);
-          if (!ok) break;
-          // row kr, 16-byte pieces 4w ... 4w+3, 128-byte swizzle
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-            *reinterpret_cast<uint4*>(smem + C::OFF_DS + kr * 128 + (((w * 4 + i) ^ (kr & 7)) << 4)) =
-                make_uint4(dk[4 * i], dk[4 * i + 1], dk[4 * i + 2], dk[4 * i + 3]);
-          fence_proxy_async();
-        } else {
+        if constexpr (CW == 64)
           tmem_st32(tdP + w * CW + CW / 2, dk);
-          tmem_wait_st();
-          tc_fence_before();
-        }
+        else
+          tmem_st16(tdP + w * CW + CW / 2, dk);
       }
+      tmem_wait_st();
+      tc_fence_before();
       __syncwarp();
       if (lane == 0) {
         mbar_arrive(bar_st_empty(slot));
@@ -450,8 +439,8 @@ __global__ void __launch_bounds__(BCfg<DH>::THREADS, BCfg<DH>::CTAS) bwd_tc_kern
     } else if (warp == C::WARP_MMA || warp == C::WARP_MMA_S) {
       // -------------------------------------------------------------- MMA issuer
       // Two issuing warps.  One issues S^T(i+1) as soon as the compute warps hold S^T(i) in registers.  The other issues
-      // the chain dV(i) | dK(i) | dP^T(i+1) (head dim 64: dV(i) | dP^T(i+1) | dK(i)): dV(i) waits for P^T(i), dK(i) for
-      // dS^T(i); what sits over dP^T(i) is read before dP^T(i+1) overwrites it, because the MMAs of one thread execute in order.
+      // the chain dV(i) | dK(i) | dP^T(i+1): dV(i) waits for P^T(i), dK(i) for dS^T(i); both sit over dP^T(i),
+      // and the MMAs of one thread execute in order, so dP^T(i+1) overwrites them only after they were read.
       // MMAs of the two threads are not ordered among themselves and need not be.
       if (run) {  // the whole warp runs the loops (see mma_ss_w); one elected lane issues
         constexpr int F = BFmt<T>::kIdesc;
@@ -464,7 +453,7 @@ __global__ void __launch_bounds__(BCfg<DH>::THREADS, BCfg<DH>::CTAS) bwd_tc_kern
         auto dsc = [&](uint32_t lo_add) { return ((uint64_t)d_hi << 32) | (uint64_t)(d_lo + lo_add); };
         constexpr uint32_t kMn = (uint32_t)((C::QCHUNK - 16) >> 4) << 16;  // K-major -> MN-major (LBO = chunk stride)
         constexpr uint32_t oK = 0, oV = (C::OFF_V - C::OFF_K) >> 4, oQ = (C::OFF_Q - C::OFF_K) >> 4,
-                           oDO = (C::OFF_DO - C::OFF_K) >> 4, oDS = (C::OFF_DS - C::OFF_K) >> 4, kTile16 = C::TILE_Q >> 4;
+                           oDO = (C::OFF_DO - C::OFF_K) >> 4, kTile16 = C::TILE_Q >> 4;
         auto koff = [](int kk) { return (uint32_t)(((kk >> 2) * kChunkBytes + (kk & 3) * 32) >> 4); };  // K-major k-step
         auto koff_q = [](int kk) { return (uint32_t)(((kk >> 2) * C::QCHUNK + (kk & 3) * 32) >> 4); };
         auto moff = [](int kk) { return (uint32_t)((kk * 2048) >> 4) + kMn; };                          // MN-major k-step
@@ -507,8 +496,6 @@ __global__ void __launch_bounds__(BCfg<DH>::THREADS, BCfg<DH>::CTAS) bwd_tc_kern
               mma_ts_w(tmem + C::COL_DV, tmem + C::COL_DP + pcol(kk), dsc(oDO + os * kTile16 + moff(kk)),
                        idesc_dv, (it > 0) || kk > 0);
             tc_commit_w(bar_do_empty(os));
-            if (C::DS_SMEM && it + 1 < iters) ok = issue_dp(it + 1);
-            if (!ok) break;
             // dS^T(it) is written: dK += dS^T Q, the last use of this Q tile (S^T(it) of the other issuer read it
             // too: P^T(it) was computed from it)
             ok = mbar_wait_w(bar_ds, it & 1, W_B_PDS, abort_flag);
@@ -516,13 +503,10 @@ __global__ void __launch_bounds__(BCfg<DH>::THREADS, BCfg<DH>::CTAS) bwd_tc_kern
             tc_fence_after();
 #pragma unroll
             for (int kk = 0; kk < BQ / 16; ++kk)
-              if constexpr (C::DS_SMEM)
-                mma_ss_w(tmem + C::COL_DK, dsc(oDS + koff(kk)), dsc(oQ + qs * kTile16 + moff(kk)), idesc_dv, (it > 0) || kk > 0);
-              else
-                mma_ts_w(tmem + C::COL_DK, tmem + C::COL_DP + CW / 2 + pcol(kk), dsc(oQ + qs * kTile16 + moff(kk)),
-                         idesc_dv, (it > 0) || kk > 0);
+              mma_ts_w(tmem + C::COL_DK, tmem + C::COL_DP + CW / 2 + pcol(kk), dsc(oQ + qs * kTile16 + moff(kk)),
+                       idesc_dv, (it > 0) || kk > 0);
             tc_commit_w(bar_q_empty(qs));
-            if (!C::DS_SMEM && it + 1 < iters) ok = issue_dp(it + 1);
+            if (it + 1 < iters) ok = issue_dp(it + 1);
           }
         }
       }
