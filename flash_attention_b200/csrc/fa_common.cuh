@@ -61,6 +61,27 @@ __device__ __forceinline__ bool visible(int i, int j, int sk, int shift, int wl,
   return true;
 }
 
+// Work item of a CTA of the tensor-core kernels, whose grid is (row blocks, heads, batch).  CTAs start in linear order, and
+// under a causal mask the row blocks (0 first) get lighter: they are taken block-major over groups of `head_group`
+// (batch, head) pairs, so that what starts last is light on every SM.  Per-head order left SMs idle for the last heavy CTA
+// of the last head, 4 - 6 % of 16 x 2048 tokens.  The group is what the L2 holds of the streamed operand (cta_head_group).
+struct CtaItem {
+  int block, head, batch;
+};
+__device__ __forceinline__ CtaItem cta_item(int head_group) {
+  const uint32_t nb = gridDim.x, pairs = gridDim.y * gridDim.z;
+  const uint32_t lin = blockIdx.x + nb * (blockIdx.y + gridDim.y * blockIdx.z);
+  const uint32_t first = lin / (nb * (uint32_t)head_group) * (uint32_t)head_group, rem = lin - first * nb;
+  const uint32_t size = min((uint32_t)head_group, pairs - first);
+  CtaItem it;
+  // (the divisions run in vector registers; the shuffles tell the compiler that the results are the same in every lane)
+  it.block = __shfl_sync(0xffffffffu, (int)(rem / size), 0);
+  const uint32_t pair = first + rem - (uint32_t)it.block * size;
+  it.batch = __shfl_sync(0xffffffffu, (int)(pair / gridDim.y), 0);
+  it.head = __shfl_sync(0xffffffffu, (int)(pair - (uint32_t)it.batch * gridDim.y), 0);
+  return it;
+}
+
 // Range of key blocks [lo, hi) of width BN that rows [m0, m0+BM) can see.
 __device__ __forceinline__ void key_block_range(int m0, int BM, int BN, int sk, int shift, int wl, int wr, int& lo,
                                                 int& hi) {
@@ -221,6 +242,15 @@ inline bool device_once_needed(DeviceOnce& once, int dev) {
   if (once.done[dev]) return false;
   once.done[dev] = true;
   return true;
+}
+// (batch, head) pairs whose streamed operand (`bytes` per pair) stays in the L2 while their row blocks run: 16 MB, a fraction
+// of it, because the first pass over a group comes from HBM.  1 (per-head order) where all row blocks cost the same: there
+// is nothing to balance, and neighbouring CTAs then share the streamed operand at the same time (32 heads of 64,
+// 16 x 2048 full: dK / dV 1084 us, 1215 us block-major).
+inline int cta_head_group(bool uneven, int64_t bytes, int64_t pairs) {
+  if (!uneven) return 1;
+  const int64_t g = (16ll << 20) / (bytes > 0 ? bytes : 1);
+  return (int)(g < 1 ? 1 : g > pairs ? pairs : g);
 }
 int raise_smem_limit(DeviceOnce& once, const void* kernel, int bytes, const char* name);
 }  // namespace fa_host

@@ -68,6 +68,7 @@ struct DqTcParams {
   CUtensorMap tq, tk, tv, tdo;
   FaBwdArgs a;
   StatusRef status;
+  int32_t head_group;
 };
 
 template <typename T>
@@ -111,12 +112,13 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_dq_tc_kernel(const __grid_con
     prefetch_tensormap(&P.tdo);
     prefetch_tensormap(&P.tv);
   }
-  const int hq = blockIdx.y, b = blockIdx.z;
+  const CtaItem item = cta_item(P.head_group);
+  const int hq = item.head, b = item.batch;
   const int hk = hq / (a.heads / a.heads_k);
   const SeqInfo si = seq_info(a.cu_seqlens_q, a.cu_seqlens_k, nullptr, nullptr, a.seqlen_q, a.seqlen_k,
                               a.use_mask_shift, a.mask_shift, b);
   // heavy query blocks (bottom rows of a causal mask see the most keys) are scheduled first
-  const int mblk = (int)gridDim.x - 1 - (int)blockIdx.x;
+  const int mblk = (int)gridDim.x - 1 - item.block;
   const int m0 = mblk * kM;
   float* d_out = a.softmax_d + ((int64_t)b * a.heads + hq) * a.d_seqlen + m0;
   if (m0 >= si.sq) {  // a shorter sequence of a packed batch: only its padding rows of D
@@ -440,6 +442,8 @@ int launch_bwd_dq_tc(const FaBwdArgs& a, cudaStream_t st) {
   if (int rc = fa_host::raise_smem_limit(once, reinterpret_cast<const void*>(kern), C::SMEM_BYTES, "bwd_dq_tc_kernel")) return rc;
   const int rows = a.d_seqlen > a.seqlen_q ? a.d_seqlen : a.seqlen_q;  // the padding rows of D are written too
   dim3 grid((rows + kM - 1) / kM, a.heads, a.batch);
+  P.head_group = fa_host::cta_head_group(a.window_left >= 0 || a.window_right >= 0 || a.cu_seqlens_q, (int64_t)a.seqlen_k * a.head_dim * 4 / (a.heads / a.heads_k),
+                                         (int64_t)a.heads * a.batch);
   kern<<<grid, kThreads, C::SMEM_BYTES, st>>>(P);
   return fa_host::check_launch("bwd_dq_tc_kernel");
 }

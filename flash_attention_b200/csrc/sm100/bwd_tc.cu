@@ -86,6 +86,7 @@ struct BwdTcParams {
   CUtensorMap tq, tk, tv, tdo;
   FaBwdArgs a;
   StatusRef status;
+  int32_t head_group;
 };
 
 template <typename T>
@@ -132,7 +133,8 @@ __global__ void __launch_bounds__(BCfg<DH>::THREADS, BCfg<DH>::CTAS) bwd_tc_kern
     prefetch_tensormap(&P.tdo);
     prefetch_tensormap(&P.tv);
   }
-  const int nblk = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
+  const CtaItem item = cta_item(P.head_group);
+  const int nblk = item.block, hk = item.head, b = item.batch;
   const int group = a.heads / a.heads_k;
   const SeqInfo si = seq_info(a.cu_seqlens_q, a.cu_seqlens_k, nullptr, nullptr, a.seqlen_q, a.seqlen_k,
                               a.use_mask_shift, a.mask_shift, b);
@@ -544,6 +546,8 @@ int launch_bwd_tc(const FaBwdArgs& a, cudaStream_t st) {
   static fa_host::DeviceOnce once;
   if (int rc = fa_host::raise_smem_limit(once, reinterpret_cast<const void*>(kern), C::SMEM_BYTES, "bwd_tc_kernel")) return rc;
   dim3 grid((a.seqlen_k + kB - 1) / kB, a.heads_k, a.batch);
+  P.head_group = fa_host::cta_head_group(a.window_left >= 0 || a.window_right >= 0 || a.cu_seqlens_q, (int64_t)a.seqlen_q * (a.heads / a.heads_k) * a.head_dim * 4,
+                                         (int64_t)a.heads_k * a.batch);
   kern<<<grid, C::THREADS, C::SMEM_BYTES, st>>>(P);
   return fa_host::check_launch("bwd_tc_kernel");
 }

@@ -79,6 +79,7 @@ struct FwdTcParams {
   CUtensorMap tq, tk, tv;
   FaFwdArgs a;
   StatusRef status;
+  int32_t head_group;
   int32_t num_splits;  // split-KV: a sequence's key blocks are divided evenly
   // A 128-row query tile holds `tile_pos` positions of `pack` neighbouring heads of one KV head's group, rows ordered
   // (position, head): pack * tile_pos <= 128.  pack = 1: 128 positions of one head.
@@ -129,13 +130,14 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
   }
   const int pack = GROUPED ? P.pack : 1, tile_pos = GROUPED ? P.tile_pos : kBM, pack_inv = GROUPED ? P.pack_inv : 65536;
   const bool cache = GROUPED && P.cache;
-  const int b = blockIdx.z, h = blockIdx.y * pack, hk = h / (a.heads / a.heads_k);  // h: first head of the tile rows
+  const CtaItem item = cta_item(P.head_group);
+  const int b = item.batch, h = item.head * pack, hk = h / (a.heads / a.heads_k);  // h: first head of the tile rows
   SeqInfo si = seq_info(a.cu_seqlens_q, a.cu_seqlens_k, GROUPED ? a.seqused_k : nullptr, GROUPED ? a.kv_batch_idx : nullptr, a.seqlen_q,
                         a.seqlen_k, a.use_mask_shift, a.mask_shift, b, GROUPED ? a.seqused_k_extra : 0);
   if (cache) si.sk = min(si.sk, a.seqlen_k);
   // heaviest blocks (largest row index under a causal mask) first; with split-KV the splits of a row block are neighbours
-  const int split = P.num_splits > 1 ? (int)blockIdx.x % P.num_splits : 0;
-  const int mrank = P.num_splits > 1 ? (int)blockIdx.x / P.num_splits : (int)blockIdx.x;
+  const int split = P.num_splits > 1 ? item.block % P.num_splits : 0;
+  const int mrank = P.num_splits > 1 ? item.block / P.num_splits : item.block;
   const int mblk = (int)gridDim.x / P.num_splits - 1 - mrank;
   const int m_base = mblk * C::NT * tile_pos;
   if (m_base >= si.sq) return;  // uniform for the CTA
@@ -666,6 +668,8 @@ int launch_fwd_tc(const FaFwdArgs& a, int64_t kv_batches, cudaStream_t st) {
   if (int rc = fa_host::raise_smem_limit(once[grouped], reinterpret_cast<const void*>(kern), C::SMEM_BYTES, "fwd_tc_kernel")) return rc;
   const int n_m = (a.seqlen_q + C::NT * P.tile_pos - 1) / (C::NT * P.tile_pos);
   dim3 grid(n_m * P.num_splits, a.heads / P.pack, a.batch);
+  P.head_group = fa_host::cta_head_group(a.window_left >= 0 || a.window_right >= 0 || a.cu_seqlens_q, (int64_t)a.seqlen_k * a.head_dim * 4 / (a.heads / P.pack / a.heads_k),
+                                         (int64_t)a.heads / P.pack * a.batch);
   kern<<<grid, 384, C::SMEM_BYTES, st>>>(P);
   return fa_host::check_launch("fwd_tc_kernel");
 }
