@@ -42,7 +42,7 @@ METRIC = "attention fwd+bwd TFLOPS/s"
 
 # dram__bytes_read.sum + dram__bytes_write.sum of the backward kernels of one step, from ncu captures of these
 # kernels on these workloads (d128: dK/dV kernel + dQ kernel; d256: the three passes of the wide kernel)
-NCU_DRAM_BYTES_PER_BACKWARD = {"train_b16_s2048_h16_d128_causal": 1.4427e9, "train_b16_s2048_h8_d256": 1.8399e9}
+NCU_DRAM_BYTES_PER_BACKWARD = {"train_b16_s2048_h16_d128_causal": 1.5821e9, "train_b16_s2048_h8_d256": 1.8399e9}
 
 WORKLOADS = {
     # name: (batch, seqlen, heads, heads_k, head_dim, causal, dtype)
@@ -666,7 +666,7 @@ def run_train(args, wl):
     # (dV, dK, dQ) that execute 8 (S three times, dP twice); a small bandwidth kernel (dot(dO, O)) precedes them.
     wide = D > 128
     bwd_kernels = ("backward (bwd_dot_do_o + bwd_wide_tc_kernel x3 [dV, dK, dQ passes])" if wide else
-                   "backward (bwd_dot_do_o + bwd_tc_kernel [dK,dV] + bwd_dq_tc_kernel [dQ])")
+                   "backward (bwd_dq_tc_kernel [dQ, D] + bwd_tc_kernel [dK,dV])")
     roofline = {"bound": "tensor", "kernel": bwd_kernels,
                 "achieved": tf_bwd, "peak": pk["tflops_burst"], "unit": "TFLOP/s",
                 "frac": tf_bwd / pk["tflops_burst"], "traffic": NCU_DRAM_BYTES_PER_BACKWARD.get(wl), "peak_source": pk["source"],

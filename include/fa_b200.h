@@ -96,7 +96,7 @@ typedef struct FaFwdArgs {
 /* Backward.  Replaces mha_bwd (flash_api.cpp:609-811) and mha_varlen_bwd (flash_api.cpp:813-1036),
    i.e. the three launches dot_do_o -> dq_dk_dv -> convert_dq of
    csrc/flash_attn/src/flash_bwd_launch_template.h:47-90.  Without dropout the launches are
-   dot_do_o -> dK/dV kernel -> dQ kernel (head dims up to 128) or dot_do_o -> dV pass -> dK pass ->
+   dQ kernel (which also computes softmax_d) -> dK/dV kernel (head dims up to 128) or dot_do_o -> dV pass -> dK pass ->
    dQ pass (129..256) instead: dq is written directly, without atomics, and dq_accum is not touched. */
 typedef struct FaBwdArgs {
   FaTensor q, k, v, out, dout, dq, dk, dv;
@@ -200,7 +200,9 @@ int fa_fwd_kvcache(const FaKvcacheArgs* args, fa_stream_t stream);
 int fa_fwd_kvcache_noalloc(const FaKvcacheArgs* args, fa_stream_t stream);
 int64_t fa_noalloc_scratch_bytes(void);
 
-/* Number of KV splits fa_fwd would like for these sizes (num_splits_heuristic, flash_api.cpp:206-246).
+/* Number of KV splits fa_fwd would like for these sizes: the least estimated time (in the place of
+   num_splits_heuristic, flash_api.cpp:206-246).  Grouped-query heads share the 128-row tiles: pass
+   heads = heads_k and seqlen_q * (heads / heads_k) rows.
    The caller sizes lse_accum/out_accum from it and passes it back in FaFwdArgs.num_splits. */
 int fa_fwd_num_splits(int32_t batch, int32_t heads, int32_t seqlen_q, int32_t seqlen_k, int32_t head_dim,
                       int32_t num_sms);
