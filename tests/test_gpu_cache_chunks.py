@@ -23,6 +23,8 @@ if torch.cuda.is_available():
     (17, 14, 2, 96, torch.bfloat16, False),
     (40, 48, 1, 64, torch.float16, False),   # 48 heads on one KV head: tiles of 8 positions x 16 heads
     (70, 2, 1, 256, torch.bfloat16, True),
+    (5, 8, 2, 128, torch.bfloat16, False),   # 20 rows
+    (17, 3, 3, 80, torch.float16, False),    # 17 rows: one more than the decode kernel takes
 ])
 def test_chunk_against_a_cache_with_nan_behind_the_keys(sq, heads, heads_k, d, dtype, interleaved, page, num_splits):
     g = torch.Generator().manual_seed(sq + d)
