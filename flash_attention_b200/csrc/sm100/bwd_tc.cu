@@ -560,10 +560,14 @@ int launch_bwd_tc(const FaBwdArgs& a, cudaStream_t st) {
 bool bwd_tc_eligible(const FaBwdArgs& a) {
   if (a.head_dim > 256 || a.p_dropout > 0.f) return false;  // head dims 129..256 run in bwd_wide_tc.cu
   if (a.seqlen_k <= 0 || a.seqlen_q <= 0) return false;
-  if (!tma_compatible(a.q) || !tma_compatible(a.k) || !tma_compatible(a.v) || !tma_compatible(a.dout)) return false;
+  const bool varlen = a.cu_seqlens_q != nullptr;
+  const int64_t nb = varlen ? 1 : a.batch, q_rows = varlen ? a.total_q : a.seqlen_q, k_rows = varlen ? a.total_k : a.seqlen_k;
+  if (!tma_compatible(a.q, q_rows, a.heads, nb) || !tma_compatible(a.dout, q_rows, a.heads, nb) ||
+      !tma_compatible(a.k, k_rows, a.heads_k, nb) || !tma_compatible(a.v, k_rows, a.heads_k, nb))
+    return false;
   // the epilogues store 16 bytes at a time
-  if (!tma_compatible(a.dq)) return false;
-  if (!a.accumulate_dkv && (!tma_compatible(a.dk) || !tma_compatible(a.dv))) return false;
+  if (!rows_compatible(a.dq)) return false;
+  if (!a.accumulate_dkv && (!rows_compatible(a.dk) || !rows_compatible(a.dv))) return false;
   if (a.head_dim % 8) return false;
   if (a.cu_seqlens_q && (a.total_q <= 0 || a.total_k <= 0)) return false;
   return encode_tiled_fn() != nullptr;

@@ -462,7 +462,9 @@ static bool decode_shape(const FaKvcacheArgs& a) {
   if (a.head_dim != 64 && a.head_dim != 128) return false;
   const int group = a.heads / a.heads_k;
   if (a.seqlen_q * group > kMaxRows || a.seqlen_q < 1) return false;
-  if (!tma_compatible(a.kcache) || !tma_compatible(a.vcache)) return false;
+  const int64_t slab_rows = a.block_table ? a.page_block_size : a.seqlen_cache;
+  if (!tma_compatible(a.kcache, slab_rows, a.heads_k, a.batch_cache) || !tma_compatible(a.vcache, slab_rows, a.heads_k, a.batch_cache))
+    return false;
   if (a.seqlen_cache <= 0) return false;
   return encode_tiled_fn() != nullptr;
 }

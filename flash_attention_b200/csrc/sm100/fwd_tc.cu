@@ -689,7 +689,12 @@ static bool fwd_tc_takes(const FaFwdArgs& a, int64_t kv_batches) {
   if (a.num_splits > 1 && a.cu_seqlens_q) return false;
   if ((a.seqused_k || a.kv_batch_idx || a.block_table) && kv_batches <= 0) return false;
   if (a.seqlen_k <= 0) return false;
-  if (!tma_compatible(a.q) || !tma_compatible(a.k) || !tma_compatible(a.v)) return false;
+  const bool varlen = a.cu_seqlens_q != nullptr;
+  const int64_t nb = varlen ? 1 : a.batch, q_rows = varlen ? a.total_q : a.seqlen_q;
+  const int64_t kv_rows = a.block_table ? a.page_block_size : varlen ? a.total_k : a.seqlen_k, kv_nb = kv_batches > 0 ? kv_batches : nb;
+  if (!tma_compatible(a.q, q_rows, a.heads, nb) || !tma_compatible(a.k, kv_rows, a.heads_k, kv_nb) ||
+      !tma_compatible(a.v, kv_rows, a.heads_k, kv_nb))
+    return false;
   if ((reinterpret_cast<uintptr_t>(a.out.ptr) & 15) || a.out.stride_s % 8 || a.out.stride_h % 8 || a.out.stride_b % 8)
     return false;
   if (a.cu_seqlens_q && (a.total_q <= 0 || a.total_k <= 0)) return false;

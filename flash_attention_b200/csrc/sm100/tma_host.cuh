@@ -38,7 +38,8 @@ static inline int make_tmap(CUtensorMap* map, const FaTensor& t, int dtype, int 
     return 1;
   }
   cuuint64_t dims[4] = {(cuuint64_t)head_dim, (cuuint64_t)extent[0], (cuuint64_t)extent[1], (cuuint64_t)extent[2]};
-  // strides of dims 1..3 in bytes; a degenerate dim still needs a legal (non-zero, 16 B multiple) stride
+  // strides of dims 1..3 in bytes; a dim of one element still needs a legal (non-zero, 16 B multiple) stride, whatever it
+  // is.  (A stride of 0 on more elements does not come here: tma_compatible refuses it.)
   auto legal = [](int64_t elems) { return (cuuint64_t)(elems > 0 ? elems : 8) * 2; };
   cuuint64_t strides[3] = {legal(stride[0]), legal(stride[1]), legal(stride[2])};
   cuuint32_t box[4] = {64, (cuuint32_t)box_of[0], (cuuint32_t)box_of[1], (cuuint32_t)box_of[2]};
@@ -74,9 +75,17 @@ static inline int make_tmap_4d_heads(CUtensorMap* map, const FaTensor& t, int dt
                    {box_heads, box_rows, 1});
 }
 
-static inline bool tma_compatible(const FaTensor& t) {
+// Base and strides in 16-byte pieces
+static inline bool rows_compatible(const FaTensor& t) {
   auto ok = [](int64_t s) { return s >= 0 && s % 8 == 0 && s < (1ll << 38); };
   return (reinterpret_cast<uintptr_t>(t.ptr) & 15) == 0 && ok(t.stride_s) && ok(t.stride_h) && ok(t.stride_b);
+}
+
+// ... and no dim that repeats its elements: a map has no stride of 0, the kernels that take addresses do.  (A null pointer
+// is a plan made before the tensors exist: its strides say nothing yet.)
+static inline bool tma_compatible(const FaTensor& t, int64_t rows, int64_t heads, int64_t batches) {
+  const bool repeats = (t.stride_s == 0 && rows > 1) || (t.stride_h == 0 && heads > 1) || (t.stride_b == 0 && batches > 1);
+  return rows_compatible(t) && !(t.ptr && repeats);
 }
 
 }  // namespace fa

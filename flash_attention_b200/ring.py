@@ -337,8 +337,10 @@ def ring_backward(dout, q, k, v, out, lse, scale, causal, window_size, group=Non
     # slot src: this rank's share of (dK, dV) of the block that started on rank src
     g = torch.zeros((P,) + tuple(kv[0].shape), dtype=torch.float32, device=k.device)
     dq = torch.zeros(q.shape, dtype=torch.float32, device=q.device)
-    if dout.stride(-1) != 1:
+    if dout.stride(-1) != 1 or 0 in dout.stride():
         dout = dout.contiguous()
+    if 0 in q.stride():  # the backward's tensor maps have no stride of 0 (k and v were stacked)
+        q = q.contiguous()
     for s in range(n_steps):
         src = (r - s) % P
         kv_cur, kv_nxt = kv[s & 1], kv[(s + 1) & 1]

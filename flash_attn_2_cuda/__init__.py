@@ -89,6 +89,16 @@ def _aligned(t):
     return t.contiguous()
 
 
+def _operand(t):
+    """_aligned, and a view that repeats its elements (the gradient of a sum, an expanded k) is copied as well: a tensor map has
+    no stride of 0.  For inputs only: an output is written where it is, a cache is not copied."""
+    if 0 in t.stride():
+        for s, n in zip(t.stride(), t.shape):
+            if s == 0 and n > 1:
+                return t.contiguous()
+    return _aligned(t)
+
+
 _SM_COUNTS = {}  # device index -> number of SMs
 
 
@@ -157,7 +167,7 @@ def fwd(q, k, v, out_, p_dropout, softmax_scale, is_causal, window_size_left, wi
     _check_shape(k, batch, seqlen_k, heads_k, d_og)
     _check_shape(v, batch, seqlen_k, heads_k, d_og)
 
-    q_p, k_p, v_p = _aligned(_pad8(q)), _aligned(_pad8(k)), _aligned(_pad8(v))
+    q_p, k_p, v_p = _operand(_pad8(q)), _operand(_pad8(k)), _operand(_pad8(v))
     d = q_p.shape[-1]
     if out_ is not None:
         out = out_
@@ -251,7 +261,7 @@ def varlen_fwd(q, k, v, out_, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seql
     _check_shape(cu_seqlens_k, batch + 1)
     wl, wr = _windows(is_causal, window_size_left, window_size_right, max_seqlen_k)
 
-    q_p, k_p, v_p = _aligned(_pad8(q)), _aligned(_pad8(k)), _aligned(_pad8(v))
+    q_p, k_p, v_p = _operand(_pad8(q)), _operand(_pad8(k)), _operand(_pad8(v))
     d = q_p.shape[-1]
     if out_ is not None:
         out = out_
@@ -355,8 +365,8 @@ def _bwd_common(varlen, dout, q, k, v, out, softmax_lse, dq_, dk_, dv_, cu_q, cu
     _check_shape(out, *q_shape)
     wl, wr = _windows(is_causal, wl_in, wr_in, seqlen_k)
 
-    dout_p = _aligned(_pad8(dout))
-    q, k, v, out = _aligned(q), _aligned(k), _aligned(v), _aligned(out)
+    dout_p = _operand(_pad8(dout))
+    q, k, v, out = _operand(q), _operand(k), _operand(v), _aligned(out)
     dq, dq_user = _grad_out(dq_, q_shape, q, "dq")
     dk, dk_user = _grad_out(dk_, k_shape, q, "dk")
     dv, dv_user = _grad_out(dv_, k_shape, q, "dv")
@@ -472,7 +482,7 @@ def fwd_kvcache(q, kcache, vcache, k_, v_, seqlens_k_, rotary_cos_, rotary_sin_,
     _check_shape(vcache, batch_c, page_block_size or seqlen_k, heads_k, d_og)
 
     padded = d_og % 8 != 0
-    q_p = _aligned(_pad8(q))
+    q_p = _operand(_pad8(q))
     kc, vc = (_pad8(kcache), _pad8(vcache)) if padded else (kcache, vcache)
     _require(_aligned(kc) is kc and _aligned(vc) is vc, "k_cache / v_cache must be 16-byte aligned with strides that are multiples of 8")
     d = q_p.shape[-1]

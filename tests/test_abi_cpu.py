@@ -218,3 +218,17 @@ def test_paged_cache_arguments_are_validated_before_launch(lib):
     f.block_table_stride = 8
     f.kv_batch_idx = ctypes.cast(idx, ctypes.c_void_p)
     assert lib.fa_fwd(ctypes.byref(f), None) == 1 and b"paged" in lib.fa_last_error()
+
+
+def test_operands_that_repeat_their_elements_are_copied():
+    import flash_attn_2_cuda as m
+
+    x = torch.randn(2, 1, 4, 64)
+    whole = x.expand(2, 5, 4, 64)
+    assert m._operand(whole).stride() == (5 * 4 * 64, 4 * 64, 64, 1) and torch.equal(m._operand(whole), whole)
+    # an extent of 1 may have any stride, and what can be read as it is stays as it is
+    one = torch.randn(64, 4, 64).as_strided((1, 64, 4, 64), (0, 256, 64, 1))
+    packed = torch.randn(2, 5, 3, 4, 64).select(2, 1)
+    assert m._operand(one) is one and m._operand(packed) is packed
+    # outputs and caches are used where they are
+    assert m._aligned(whole) is whole
