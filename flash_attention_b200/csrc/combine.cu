@@ -1,6 +1,7 @@
 // Merge of partial attention results by log-sum-exp.  Same math as combine_attn_seqk_parallel
 // (csrc/flash_attn/src/flash_fwd_kernel.h:1169-1327): LSE = logsumexp_s(LSE_s),
-// O = sum_s exp(LSE_s - LSE) * O_s; a row whose parts are all empty (-inf) gets O = 0, LSE = +inf.
+// O = sum_s exp(LSE_s - LSE) * O_s; a row whose parts are all empty (-inf) gets O = 0, LSE = +inf, a row with a part whose
+// LSE is NaN (a NaN score) gets what one pass gives: O = NaN, LSE = +inf.
 #include "fa_common.cuh"
 
 namespace fa {
@@ -37,8 +38,10 @@ __global__ void __launch_bounds__(128) combine_kernel(const CombineParams p) {
   for (int i = 0; i < 4; ++i) sum += __expf(l[i] - msafe);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-  const bool empty = !(sum > 0.f) || mx == -INFINITY;
-  const float lse = empty ? INFINITY : logf(sum) + mx;
+  // (fmaxf drops a NaN, so the LSEs are asked)
+  const bool nan = __any_sync(0xffffffffu, l[0] != l[0] || l[1] != l[1] || l[2] != l[2] || l[3] != l[3]);
+  const bool empty = !nan && (!(sum > 0.f) || mx == -INFINITY);
+  const float lse = empty || nan ? INFINITY : logf(sum) + mx;
   const int s_idx = (int)(row % p.S);
   const int64_t bh = row / p.S;
   const int h = (int)(bh % p.H), b = (int)(bh / p.H);
@@ -47,22 +50,27 @@ __global__ void __launch_bounds__(128) combine_kernel(const CombineParams p) {
   // head_dim <= 256: at most two 4-column groups per lane
   float4 acc[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
   float wgt[4];
+  uint32_t live[4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) wgt[i] = empty ? 0.f : __expf(l[i] - lse);
+  for (int i = 0; i < 4; ++i) {
+    wgt[i] = nan ? sum : empty ? 0.f : __expf(l[i] - lse);
+    live[i] = __ballot_sync(0xffffffffu, !empty && l[i] != -INFINITY);
+  }
   // Bound by the latency of the loads: four parts are in flight at a time (16 parts of 2048 x 128: 9.4 us, 11.5 us with one
-  // at a time).  A part of weight zero is not read: nobody may have written it.
+  // at a time).  Empty parts, those past the last one among them, are not read: nobody may have written them.
   for (int s0 = 0; s0 < p.n_parts; s0 += 4) {  // uniform trip count: every lane takes part in the shuffles
     const float wsel = (s0 >> 5) == 0 ? wgt[0] : (s0 >> 5) == 1 ? wgt[1] : (s0 >> 5) == 2 ? wgt[2] : wgt[3];
+    const uint32_t lsel = ((s0 >> 5) == 0 ? live[0] : (s0 >> 5) == 1 ? live[1] : (s0 >> 5) == 2 ? live[2] : live[3]) >> (s0 & 31);
     float w[4];
     float4 x[4][2];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      w[k] = __shfl_sync(0xffffffffu, wsel, (s0 + k) & 31);  // parts past the last one have weight zero
+      w[k] = __shfl_sync(0xffffffffu, wsel, (s0 + k) & 31);
       const float* src = p.out_parts + ((int64_t)(s0 + k) * rows + row) * p.D;
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         const int c = lane * 4 + i * 128;
-        x[k][i] = w[k] != 0.f && c < p.D ? *reinterpret_cast<const float4*>(src + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        x[k][i] = (lsel >> k & 1) && c < p.D ? *reinterpret_cast<const float4*>(src + c) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
     }
 #pragma unroll

@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(128) fwd_generic_kernel(const __grid_constant_
     float l = l_run[r];
     l += __shfl_xor_sync(0xffffffffu, l, 1);
     l += __shfl_xor_sync(0xffffffffu, l, 2);
-    bool empty = !(l > 0.f) || m_run[r] == -INFINITY;
+    bool empty = l == 0.f;  // no key; NaN where a score is NaN: O and the LSE of a part are NaN then
     inv[r] = empty ? 0.f : 1.f / l;
     lse[r] = empty ? INFINITY : (m_run[r] + log2f(l)) * kLn2;
   }
@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(128) fwd_generic_kernel(const __grid_constant_
     for (int r = 0; r < 2; ++r) {
       int row = row_a + r * 8;
       if (row >= si.sq) continue;
-      if (t == 0) p.softmax_lse[(int64_t)bh * p.lse_seqlen + row] = lse[r];
+      if (t == 0) p.softmax_lse[(int64_t)bh * p.lse_seqlen + row] = lse[r] == lse[r] ? lse[r] : INFINITY;
       float sc = inv[r] * rp_keep;
 #pragma unroll
       for (int i = 0; i < DP / 8; ++i) {

@@ -403,9 +403,9 @@ __global__ void __launch_bounds__(160, 2) decode_kernel(const __grid_constant__ 
         acc.z += f * x.z;
         acc.w += f * x.w;
       }
-      const bool empty = !(lsum > 0.f);
+      const bool empty = lsum == 0.f;  // no key; NaN where a score is NaN: O and the LSE of a part are NaN then
       const float inv = empty ? 0.f : 1.f / lsum;
-      const float lse = empty ? INFINITY : (mmax + log2f(lsum)) * kLn2;
+      const float lse = (mmax + log2f(lsum)) * kLn2;
       const int64_t ri = row_index(r);
       if (nsplit > 1) {
         *reinterpret_cast<float4*>(a.out_accum + ((int64_t)split * rows_total + ri) * D + d0) =
@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(160, 2) decode_kernel(const __grid_constant__ 
         pk.x = Pack<T>::two(acc.x * inv, acc.y * inv);
         pk.y = Pack<T>::two(acc.z * inv, acc.w * inv);
         *reinterpret_cast<uint2*>(o + d0) = pk;
-        if (d0 == 0) a.softmax_lse[ri] = lse;
+        if (d0 == 0) a.softmax_lse[ri] = lsum > 0.f ? lse : INFINITY;
       }
     }
   }
@@ -590,7 +590,7 @@ int decode_run_noalloc(const FaKvcacheArgs& a, int num_splits, cudaStream_t st) 
     unsigned char* base = nullptr;
     if (noalloc_scratch_ptr(&base)) return 2;
     // Nothing has to be cleared: every (split, row) LSE is written by each launch (-inf for an empty
-    // split) and the combine step never reads the partial output of a part whose weight is zero.
+    // split) and the combine step never reads the partial output of an empty part.
     b.lse_accum = reinterpret_cast<float*>(base);
     b.out_accum = reinterpret_cast<float*>(base + lse_bytes);
   }

@@ -412,14 +412,16 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
       }
       float inv = 0.f;
       if (ok) {
-        const bool empty = !(l_sum > 0.f) || m_used == -INFINITY;
+        // The sum is 0 without a visible key and NaN where a score is NaN: O and the LSE of a part are NaN then, so that the
+        // merge cannot take the part for an empty one.  (In one pass the LSE of both is +inf, as in the reference.)
+        const bool empty = l_sum == 0.f;
         inv = empty ? 0.f : 1.f / l_sum;
-        const float lse = empty ? INFINITY : (m_used + log2f(l_sum)) * kLn2;
+        const float lse = (m_used + log2f(l_sum)) * kLn2;
         if (row_valid) {
           if (P.num_splits > 1)  // the split workspaces are (split, batch, head, row): not packed, -inf marks an empty part
             a.lse_accum[((int64_t)split * a.batch * a.heads + (int64_t)b * a.heads + head) * a.seqlen_q + row] = empty ? -INFINITY : lse;
           else
-            a.softmax_lse[((int64_t)b * a.heads + head) * a.lse_seqlen + row] = lse;
+            a.softmax_lse[((int64_t)b * a.heads + head) * a.lse_seqlen + row] = l_sum > 0.f ? lse : INFINITY;
         }
       }
       unsigned char* stage = smem + t * C::TILE_BYTES;  // the Q tile of this warpgroup is no longer read
