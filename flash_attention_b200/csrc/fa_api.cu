@@ -439,6 +439,8 @@ int fa_fwd_kvcache(const FaKvcacheArgs* a, fa_stream_t stream) {
                    : (splits > 1 ? "kvcache_prep+fwd_generic+combine" : "kvcache_prep+fwd_generic");
   const bool causal_or_local = a->window_left >= 0 || a->window_right >= 0;
   FA_REQUIRE(!a->rotary_cos || a->q_rotated, "rotary needs the q_rotated scratch buffer");
+  // (every kernel reads it in 16-byte pieces; a plan is made without it and must not depend on where it is)
+  FA_REQUIRE((reinterpret_cast<uintptr_t>(a->q_rotated) & 15) == 0, "q_rotated: pointer must be 16-byte aligned");
   int rc = fa::kvcache_prep(*a, (causal_or_local && !a->q_rows_share_position) ? 1 : 0, st);
   if (rc) return rc;
   if (rows) {

@@ -560,6 +560,7 @@ def fwd_kvcache(q, kcache, vcache, k_, v_, seqlens_k_, rotary_cos_, rotary_sin_,
         ns = lib().fa_kvcache_plan(ctypes.byref(a), _sm_count(q.device), ctypes.byref(lse_b), ctypes.byref(out_b))
         if ns < 0:
             raise RuntimeError("flash_attn_2_cuda.fwd_kvcache: " + _lib.last_error())
+        a.num_splits = ns  # what the workspaces are sized for
         keep = []
         if ns > 1:
             lse_acc = torch.empty(lse_b.value // 4, dtype=torch.float32, device=q.device)

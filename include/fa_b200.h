@@ -151,10 +151,10 @@ typedef struct FaKvcacheArgs {
      (flash_api.cpp:1096-1104); rotary then uses one position for all rows. */
   int32_t q_rows_share_position;
   int32_t num_splits;             /* 0 = choose, 1 = none, <= 128 */
-  /* workspaces, fa_kvcache_workspace_bytes() */
+  /* workspaces, fa_kvcache_plan() */
   float* lse_accum;
   float* out_accum;
-  void* q_rotated;                /* scratch for rotated q when the generic path is taken, or NULL */
+  void* q_rotated;                /* scratch for rotated q (16-byte aligned), or NULL without rotary / with one fused token */
   /* Paged cache: block_table != NULL makes kcache / vcache pools of pages (batch_cache = number of pages,
      page_block_size rows each, stride_b = page pitch); key j of sequence b is row j % page_block_size of
      page block_table[b * block_table_stride + j / page_block_size]; seqlen_cache is then the capacity
@@ -207,7 +207,9 @@ int64_t fa_noalloc_scratch_bytes(void);
 int fa_fwd_num_splits(int32_t batch, int32_t heads, int32_t seqlen_q, int32_t seqlen_k, int32_t head_dim,
                       int32_t num_sms);
 /* Splits and workspace sizes of fa_fwd_kvcache for these arguments (pointers may be NULL);
-   returns the number of splits that the call will use and stores the byte sizes. */
+   returns the number of splits that the call will use and stores the byte sizes.  Pass the count back in
+   FaKvcacheArgs.num_splits: the call then uses it whatever it would have chosen itself, so that it cannot
+   outgrow the workspaces (with 0 it plans again, from the arguments and the device of that moment). */
 int fa_kvcache_plan(const FaKvcacheArgs* args, int32_t num_sms, int64_t* lse_accum_bytes, int64_t* out_accum_bytes);
 /* Bytes of FaBwdArgs.dq_accum (dq_accum of flash_api.cpp:735-739, 950-961). */
 int64_t fa_bwd_workspace_bytes(int32_t batch, int32_t seqlen_q, int32_t heads, int32_t head_dim, int32_t total_q,

@@ -232,3 +232,68 @@ def test_operands_that_repeat_their_elements_are_copied():
     assert m._operand(one) is one and m._operand(packed) is packed
     # outputs and caches are used where they are
     assert m._aligned(whole) is whole
+
+
+def _rotary_cache_args(d=96, sq=40):
+    from flash_attention_b200 import _lib
+
+    a = _lib.FaKvcacheArgs()
+    a.batch, a.batch_cache, a.seqlen_q, a.seqlen_cache, a.seqlen_new, a.heads, a.heads_k, a.head_dim, a.dtype = 2, 2, sq, 8192, sq, 8, 2, d, 1
+    a.window_left, a.window_right = 8192, 0
+    for t, rows, heads in ((a.q, sq, 8), (a.out, sq, 8), (a.kcache, 8192, 2), (a.vcache, 8192, 2), (a.knew, sq, 2), (a.vnew, sq, 2)):
+        t.ptr, t.stride_b, t.stride_s, t.stride_h = 1 << 20, rows * heads * d, heads * d, d  # never followed: nothing is launched
+    a.cache_seqlens = a.rotary_cos = a.rotary_sin = a.softmax_lse = a.lse_accum = a.out_accum = 1 << 20
+    a.rotary_dim, a.seqlen_ro = d // 16 * 16, 8192
+    return a
+
+
+@pytest.mark.parametrize("d,sq", [(96, 40), (128, 40), (128, 4), (64, 1)])
+def test_cache_plan_does_not_depend_on_buffers_that_come_later(lib, d, sq):
+    def plan(a):
+        lb, ob = ctypes.c_int64(), ctypes.c_int64()
+        ns = lib.fa_kvcache_plan(ctypes.byref(a), 148, ctypes.byref(lb), ctypes.byref(ob))
+        return ns, lb.value, ob.value
+
+    a = _rotary_cache_args(d, sq)
+    want = plan(a)
+    assert want[0] > 1
+    a.q_rotated = 1 << 20
+    assert plan(a) == want
+    a.num_splits = want[0]  # passed back: used as it is
+    assert plan(a) == want
+    a.num_splits = 0
+    a.q = a.out = a.kcache = a.vcache = type(a.q)()  # planned before the tensors exist
+    assert plan(a) == want
+
+
+def test_misaligned_scratch_is_refused_before_launch(lib):
+    a = _rotary_cache_args()
+    a.q_rotated = (1 << 20) + 2
+    assert lib.fa_fwd_kvcache(ctypes.byref(a), None) == 1
+    assert b"q_rotated" in lib.fa_last_error()
+
+
+def test_cache_call_uses_the_split_count_that_sized_its_workspaces(monkeypatch):
+    import flash_attn_2_cuda as m
+
+    seen = {}
+
+    class Lib:
+        @staticmethod
+        def fa_kvcache_plan(args, sms, lse_bytes, out_bytes):
+            lse_bytes._obj.value, out_bytes._obj.value = 3 * 2 * 4 * 5 * 4, 3 * 2 * 4 * 5 * 64 * 4
+            return 3
+
+        @staticmethod
+        def fa_fwd_kvcache(args, stream):
+            seen["splits"] = args._obj.num_splits
+            return 0
+
+    monkeypatch.setattr(m, "lib", lambda: Lib)
+    monkeypatch.setattr(m, "_check_device", lambda *ts: None)
+    monkeypatch.setattr(m, "_on_device", lambda device: m._SAME_DEVICE)
+    monkeypatch.setattr(m, "_stream", lambda t: None)
+    monkeypatch.setattr(m, "_sm_count", lambda device: 148)
+    q, cache = torch.zeros(2, 5, 4, 64, dtype=torch.float16), torch.zeros(2, 512, 4, 64, dtype=torch.float16)
+    m.fwd_kvcache(q, cache, cache, None, None, None, None, None, None, None, 0.125, True, -1, -1, False, 0)
+    assert seen == {"splits": 3}
