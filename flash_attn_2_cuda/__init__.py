@@ -52,8 +52,12 @@ def _check_shape(t, *shape):
         raise RuntimeError("tensor must have shape (%s), got %s" % (", ".join(map(str, shape)), tuple(t.shape)))
 
 
+# (torch's own shortcut for the stream's handle, 2.2 us cheaper per call than a Stream object; not part of its public API)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream(t):
-    return torch._C._cuda_getCurrentRawStream(t.device.index)
+    return _raw_stream(t.device.index) if _raw_stream else torch.cuda.current_stream(t.device).cuda_stream
 
 
 class _SameDevice:

@@ -297,3 +297,17 @@ def test_cache_call_uses_the_split_count_that_sized_its_workspaces(monkeypatch):
     q, cache = torch.zeros(2, 5, 4, 64, dtype=torch.float16), torch.zeros(2, 512, 4, 64, dtype=torch.float16)
     m.fwd_kvcache(q, cache, cache, None, None, None, None, None, None, None, 0.125, True, -1, -1, False, 0)
     assert seen == {"splits": 3}
+
+
+def test_stream_without_the_private_shortcut(monkeypatch):
+    import flash_attn_2_cuda as m
+
+    class Stream:
+        cuda_stream = 77
+
+    t = torch.empty(1)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device: Stream)
+    monkeypatch.setattr(m, "_raw_stream", None)
+    assert m._stream(t) == 77
+    monkeypatch.setattr(m, "_raw_stream", lambda index: (index, 78))
+    assert m._stream(t) == (t.device.index, 78)
