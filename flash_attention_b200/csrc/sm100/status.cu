@@ -34,6 +34,14 @@ int current_device() {
   return dev;
 }
 
+// The first call of a process may already be inside a stream capture.  The status word's address and the mirror are not part
+// of what is captured, but a thread that captures may only ask for them in the relaxed mode.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // A kernel that does nothing but wait, with a short limit, for a barrier phase that no one
 // completes: exercises the give-up path (status word, mirror, wind-down) without any fault.
 __global__ void wait_timeout_selftest_kernel(StatusRef status, long long limit_cycles, int code) {
@@ -60,6 +68,7 @@ StatusRef status_ref(bool may_allocate) {
   const int dev = current_device();
   if (dev < 0) return r;
   if (!g_dev_ptr[dev]) {
+    RelaxedCapture relaxed;
     void* p = nullptr;
     if (cudaGetSymbolAddress(&p, g_status_word) != cudaSuccess) {
       cudaGetLastError();
@@ -70,6 +79,7 @@ StatusRef status_ref(bool may_allocate) {
   r.dev = g_dev_ptr[dev];
   int* mirror = g_host_mirror.load(std::memory_order_acquire);
   if (!mirror && may_allocate) {
+    RelaxedCapture relaxed;
     void* p = nullptr;
     if (cudaHostAlloc(&p, kMaxDevices * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) == cudaSuccess) {
       for (int i = 0; i < kMaxDevices; ++i) static_cast<int*>(p)[i] = 0;
