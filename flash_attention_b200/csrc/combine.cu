@@ -61,6 +61,7 @@ __global__ void __launch_bounds__(128) combine_kernel(const CombineParams p) {
   for (int s0 = 0; s0 < p.n_parts; s0 += 4) {  // uniform trip count: every lane takes part in the shuffles
     const float wsel = (s0 >> 5) == 0 ? wgt[0] : (s0 >> 5) == 1 ? wgt[1] : (s0 >> 5) == 2 ? wgt[2] : wgt[3];
     const uint32_t lsel = ((s0 >> 5) == 0 ? live[0] : (s0 >> 5) == 1 ? live[1] : (s0 >> 5) == 2 ? live[2] : live[3]) >> (s0 & 31);
+    if (!(lsel & 15)) continue;  // the same in every lane
     float w[4];
     float4 x[4][2];
 #pragma unroll
