@@ -1,7 +1,7 @@
 // Backward attention on tcgen05 tensor cores (head dim <= 128), part 2 of 2: dQ.
 //
 // One CTA owns 128 query rows of one (batch, query head), keeps Q and dO in shared memory and dQ in
-// tensor memory, and walks every 64-key block those rows can see (bwd_tc.cu holds part 1, dK / dV,
+// tensor memory, and walks every block of 64 (or 128) keys those rows can see (bwd_tc.cu holds part 1, dK / dV,
 // and says why the pass is split).  Same math as the dQ half of compute_dq_dk_dv_1colblock
 // (csrc/flash_attn/src/flash_bwd_kernel.h:425-1112):
 //   S   = Q K^T           (lanes = queries, columns = keys)             SS MMA  -> TMEM tS
@@ -16,9 +16,11 @@
 // and at most 113 KiB: two CTAs share an SM, and one's waits, start and end run under the other's blocks.  An N = 64 SS MMA
 // takes 48 cycles against 32 of math (it reads its A slice for half the columns); on long sequences that eats what
 // the second CTA gives.  16 x 2048 tokens, with D: 16 heads of 128 causal 455 + 47 -> 440 us, 32 heads of 64 full
-// 1186 + 47 -> 906 us (two buffers of dS of its own, so that dP(j+1) need not wait for dQ(j): 948); 32768 tokens causal 10354 + 98 -> 10390 us.
+// 1186 + 47 -> 906 us (two buffers of dS of its own, so that dP(j+1) need not wait for dQ(j): 948); 32768 tokens causal unchanged.
+// Where the grid leaves every CTA an SM of its own, nothing runs under its waits: blocks of 128 keys halve them (bwd_dq_tc_main).
+// Registers: 80 a thread in the 64-key form, with 4 to 28 bytes spilled, none in the 128-key one.
 //
-// Warps: 0-7 compute (warpgroup w handles key columns [32w, 32w+32) of the block; in the epilogue,
+// Warps: 0-7 compute (warpgroup w handles the half w of a block's key columns; in the epilogue,
 // head-dim columns [D/2*w, ...)), 8 = TMA producer, 9 = MMA issuer, 10 = TMEM owner, 11 = issuer of dQ.
 #include <cstdlib>
 
@@ -35,9 +37,7 @@ StatusRef status_ref(bool may_allocate);
 namespace {
 
 constexpr int kM = 128;                  // query rows per CTA
-constexpr int kN = 64;                   // keys per block
 constexpr int kChunkM = kM * 128;        // [128 rows][64 x 16-bit]
-constexpr int kChunkN = kN * 128;        // [64 rows][64 x 16-bit]
 constexpr int kCompute = 8;              // compute warps
 constexpr int kThreads = 32 * kCompute + 128;
 constexpr int kWarpProducer = kCompute, kWarpMma = kCompute + 1, kWarpTmem = kCompute + 2, kWarpMmaDq = kCompute + 3;
@@ -45,13 +45,16 @@ constexpr int kWarpProducer = kCompute, kWarpMma = kCompute + 1, kWarpTmem = kCo
 enum DqWait { W_Q_ALIGN = 40, W_Q_QDO = 41, W_Q_KV_FULL = 42, W_Q_KV_EMPTY = 43, W_Q_S = 44, W_Q_DP = 45, W_Q_DS = 46,
               W_Q_DONE = 47 };
 
-template <int DH>
+// KN: keys per block
+template <int DH, int KN>
 struct QCfg {
+  static constexpr int CTAS = KN > 64 ? 1 : 2;  // per SM
   static constexpr int NCHUNK = DH / 64;
-  static constexpr int TILE_M = NCHUNK * kChunkM, TILE_N = NCHUNK * kChunkN;  // Q / dO tile, K / V tile
+  static constexpr int CHUNK_N = KN * 128;  // [KN rows][64 x 16-bit]
+  static constexpr int TILE_M = NCHUNK * kChunkM, TILE_N = NCHUNK * CHUNK_N;  // Q / dO tile, K / V tile
   // K(j) is needed from S(j) (issued a block early) to dQ(j), V(j) only by dP(j): K gets the deeper ring
   static constexpr int NSK = DH > 64 ? 2 : 4;
-  static constexpr int NSV = DH > 64 ? 1 : 3;
+  static constexpr int NSV = DH > 64 ? (KN > 64 ? 2 : 1) : 3;
   static constexpr int OFF_Q = 0;
   static constexpr int OFF_DO = TILE_M;
   static constexpr int OFF_K = 2 * TILE_M;
@@ -60,8 +63,9 @@ struct QCfg {
   static constexpr int NBAR = 2 * NSK + 2 * NSV + 8;
   static constexpr int OFF_D = OFF_BAR + NBAR * 8 + 32;  // D of the 128 rows, fp32
   static constexpr int SMEM_BYTES = OFF_D + kM * 4;
-  static constexpr int COL_S = 0, COL_DP = kN, COL_DQ = 2 * kN;  // dS (16-bit) goes over dP
-  static constexpr int TMEM_COLS = 256;
+  static constexpr int COL_S = 0, COL_DP = KN, COL_DQ = 2 * KN;  // dS (16-bit) goes over dP
+  static constexpr int TMEM_COLS = KN > 64 ? 512 : 256;
+  static_assert(CTAS * (SMEM_BYTES + 1024) <= 228 * 1024 && COL_DQ + DH <= TMEM_COLS, "what the CTAs of an SM share");
 };
 
 struct DqTcParams {
@@ -85,14 +89,13 @@ struct QFmt<__nv_bfloat16> {
 
 // UNEVEN: CTAs in the order of cta_item.  (An instance of its own: with the block and head worked out instead of read from
 // blockIdx the even case took 4 % longer at head dim 64.)
-template <typename T, int DH, bool UNEVEN>
-__global__ void __launch_bounds__(kThreads, 2) bwd_dq_tc_kernel(const __grid_constant__ DqTcParams P) {
-  using C = QCfg<DH>;
+template <typename T, int DH, int KN, bool UNEVEN>
+__global__ void __launch_bounds__(kThreads, QCfg<DH, KN>::CTAS) bwd_dq_tc_kernel(const __grid_constant__ DqTcParams P) {
+  using C = QCfg<DH, KN>;
   constexpr int NSK = C::NSK, NSV = C::NSV;
   const FaBwdArgs& a = P.a;
   extern __shared__ __align__(1024) unsigned char smem[];
   const uint32_t s_base = smem_addr(smem);
-  static_assert(2 * (C::SMEM_BYTES + 1024) <= 228 * 1024, "two CTAs per SM");
   const uint32_t sQ = s_base + C::OFF_Q, sDO = s_base + C::OFF_DO;
   auto sK = [&](int st) { return s_base + C::OFF_K + st * C::TILE_N; };
   auto sV = [&](int st) { return s_base + C::OFF_V + st * C::TILE_N; };
@@ -128,7 +131,7 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_dq_tc_kernel(const __grid_con
     return;
   }
   int n_lo, n_hi;
-  key_block_range(m0, kM, kN, si.sk, si.shift, a.window_left, a.window_right, n_lo, n_hi);
+  key_block_range(m0, kM, KN, si.sk, si.shift, a.window_left, a.window_right, n_lo, n_hi);
   const int iters = n_hi - n_lo;
 
   if (threadIdx.x == 64) {  // reads global memory: not in front of the first loads
@@ -161,9 +164,9 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_dq_tc_kernel(const __grid_con
         for (int c = 0; c < C::NCHUNK; ++c) tma_load_4d(dst + c * chunk, tm, bar, c * 64, (int)row, head, (int)batch);
       };
       load(sQ, &P.tq, bar_q, kChunkM, si.q_row0 + m0, hq, si.q_batch);
-      load(sK(0), &P.tk, bar_k_full(0), kChunkN, si.k_row0 + n_lo * kN, hk, si.k_batch);
+      load(sK(0), &P.tk, bar_k_full(0), C::CHUNK_N, si.k_row0 + n_lo * KN, hk, si.k_batch);
       load(sDO, &P.tdo, bar_do, kChunkM, si.q_row0 + m0, hq, si.q_batch);
-      load(sV(0), &P.tv, bar_v_full(0), kChunkN, si.k_row0 + n_lo * kN, hk, si.k_batch);
+      load(sV(0), &P.tv, bar_v_full(0), C::CHUNK_N, si.k_row0 + n_lo * KN, hk, si.k_batch);
     }
   }
   if (warp == kWarpTmem) {
@@ -179,11 +182,12 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_dq_tc_kernel(const __grid_con
 
   if (warp < kCompute) {
     // ---------------------------------------------------------------- compute warpgroups
+    constexpr int KW = KN / 2;                  // key columns of a warpgroup
     const int w = warp >> 2;                    // key-column half / head-dim half
     const int r = (warp & 3) * 32 + lane;       // query row of this thread within the CTA tile
     const int qrow = m0 + r;
     const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
-    const uint32_t tdP = tmem + lane_off + C::COL_DP + w * 32;
+    const uint32_t tdP = tmem + lane_off + C::COL_DP + w * KW;
     bool ok = (*abort_flag == 0);  // with iters == 0 the loop is skipped and the epilogue writes zeros
     // D = rowsum(dO o O) of the CTA's rows, while the first tiles and S(0) are on their way: DH / 8 threads share a row.
     // bwd_tc.cu, launched after this kernel, reads D.  (A launch of its own took 47 us next to 1050 us of both kernels on
@@ -235,51 +239,56 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_dq_tc_kernel(const __grid_con
     if (a.window_left >= 0) k_lo = max(k_lo, qrow + si.shift - a.window_left);
     const uint64_t scale2 = pack2(scale_log2, scale_log2), neg_lse2 = pack2(-lse2, -lse2), neg_d2 = pack2(-dsum, -dsum);
     for (int j = 0; j < iters && ok; ++j) {
-      const int n0 = (n_lo + j) * kN;
-      const uint32_t tS = tmem + lane_off + C::COL_S + w * 32;
-      const bool need_mask = (n0 + kN > si.sk) ||
-                             (a.window_right >= 0 && n0 + kN - 1 > m0 + si.shift + a.window_right) ||
+      const int n0 = (n_lo + j) * KN;
+      const uint32_t tS = tmem + lane_off + C::COL_S + w * KW;
+      const bool need_mask = (n0 + KN > si.sk) ||
+                             (a.window_right >= 0 && n0 + KN - 1 > m0 + si.shift + a.window_right) ||
                              (a.window_left >= 0 && n0 < m0 + kM - 1 + si.shift - a.window_left);
-      // ---- P = exp2(S * scale - LSE), 32 key columns per thread, kept in registers
+      // ---- P = exp2(S * scale - LSE), KW key columns per thread, kept in registers
       ok = mbar_wait(bar_s, j & 1, W_Q_S, abort_flag);
       if (!ok) break;
       tc_fence_after();
-      float p[32];
+      float p[KW];
       {
-        uint32_t s[32];
-        tmem_ld32(tS, s);
+        uint32_t s[KW / 32][32];
+#pragma unroll
+        for (int h = 0; h < KW / 32; ++h) tmem_ld32(tS + h * 32, s[h]);
         tmem_wait_ld();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_sread);  // S(j) is in registers: S(j+1) may overwrite it
 #pragma unroll
-        for (int c = 0; c < 32; c += 2) {
+        for (int c = 0; c < KW; c += 2) {
           float x0, x1;
-          unpack2(fma2(pack2u(s[c], s[c + 1]), scale2, neg_lse2), x0, x1);
+          unpack2(fma2(pack2u(s[c / 32][c % 32], s[c / 32][c % 32 + 1]), scale2, neg_lse2), x0, x1);
           p[c] = ex2(x0);
           p[c + 1] = ex2(x1);
         }
       }
       if (need_mask) {
-        const int c_lo = k_lo - n0 - w * 32, c_hi = k_hi - n0 - w * 32;
+        const int c_lo = k_lo - n0 - w * KW, c_hi = k_hi - n0 - w * KW;
 #pragma unroll
-        for (int c = 0; c < 32; ++c) p[c] = (c >= c_lo && c <= c_hi) ? p[c] : 0.f;
+        for (int c = 0; c < KW; ++c) p[c] = (c >= c_lo && c <= c_hi) ? p[c] : 0.f;
       }
       // ---- dS = P o (dP - D), 16-bit, over this warp's own, now read, columns of dP
       ok = mbar_wait(bar_dp, j & 1, W_Q_DP, abort_flag);
       if (!ok) break;
       tc_fence_after();
       {
-        uint32_t d[32], pk[16];
-        tmem_ld32(tdP, d);
+        uint32_t d[KW / 32][32], pk[KW / 2];
+#pragma unroll
+        for (int h = 0; h < KW / 32; ++h) tmem_ld32(tdP + h * 32, d[h]);
         tmem_wait_ld();
 #pragma unroll
-        for (int c = 0; c < 32; c += 2) {
+        for (int c = 0; c < KW; c += 2) {
           float x0, x1;
-          unpack2(mul2(pack2(p[c], p[c + 1]), add2(pack2u(d[c], d[c + 1]), neg_d2)), x0, x1);
+          unpack2(mul2(pack2(p[c], p[c + 1]), add2(pack2u(d[c / 32][c % 32], d[c / 32][c % 32 + 1]), neg_d2)), x0, x1);
           pk[c >> 1] = Pack<T>::two(x0, x1);
         }
-        tmem_st16(tdP, pk);
+        if constexpr (KW == 64)
+          tmem_st32(tdP, pk);
+        else
+          tmem_st16(tdP, pk);
       }
       tmem_wait_st();
       tc_fence_before();
@@ -333,15 +342,15 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_dq_tc_kernel(const __grid_con
         bool ok = true;
         for (int j = 1; j < iters && ok; ++j) {  // block 0 is on its way
           const int ks = j % NSK, vs = j % NSV;
-          const int row = (int)si.k_row0 + (n_lo + j) * kN;
+          const int row = (int)si.k_row0 + (n_lo + j) * KN;
           ok = mbar_wait(bar_k_empty(ks), ((j / NSK) & 1) ^ 1, W_Q_KV_EMPTY, abort_flag);
           if (!ok) break;
           mbar_expect_tx(bar_k_full(ks), C::TILE_N);
-          for (int c = 0; c < C::NCHUNK; ++c) tma_load_4d(sK(ks) + c * kChunkN, &P.tk, bar_k_full(ks), c * 64, row, hk, kb);
+          for (int c = 0; c < C::NCHUNK; ++c) tma_load_4d(sK(ks) + c * C::CHUNK_N, &P.tk, bar_k_full(ks), c * 64, row, hk, kb);
           ok = mbar_wait(bar_v_empty(vs), ((j / NSV) & 1) ^ 1, W_Q_KV_EMPTY, abort_flag);
           if (!ok) break;
           mbar_expect_tx(bar_v_full(vs), C::TILE_N);
-          for (int c = 0; c < C::NCHUNK; ++c) tma_load_4d(sV(vs) + c * kChunkN, &P.tv, bar_v_full(vs), c * 64, row, hk, kb);
+          for (int c = 0; c < C::NCHUNK; ++c) tma_load_4d(sV(vs) + c * C::CHUNK_N, &P.tv, bar_v_full(vs), c * 64, row, hk, kb);
         }
       }
     } else if (warp == kWarpMma || warp == kWarpMmaDq) {
@@ -351,18 +360,18 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_dq_tc_kernel(const __grid_con
       // not ordered among themselves and need not be.
       if (run) {  // the whole warp runs the loops (see mma_ss_w); one elected lane issues
         constexpr int F = QFmt<T>::kIdesc;
-        constexpr uint32_t idesc_s = make_idesc(kM, kN, F, 0, 0);   // S, dP: K-major x K-major, N = 64 keys
+        constexpr uint32_t idesc_s = make_idesc(kM, KN, F, 0, 0);   // S, dP: K-major x K-major, N = KN keys
         constexpr uint32_t idesc_dq = make_idesc(kM, DH, F, 0, 1);  // dQ: A in TMEM, B MN-major, N = DH
         // One descriptor is built (Q tile, K-major); every other operand differs from it only in the
         // low word: the address field (+ byte offset >> 4) and, for MN-major reads, the LBO field.
         const uint64_t d_base = smem_desc_sw128(sQ, 16, 1024);
         const uint32_t d_lo = (uint32_t)d_base, d_hi = (uint32_t)(d_base >> 32);
         auto dsc = [&](uint32_t lo_add) { return ((uint64_t)d_hi << 32) | (uint64_t)(d_lo + lo_add); };
-        constexpr uint32_t kMn = (uint32_t)((kChunkN - 16) >> 4) << 16;  // K-major -> MN-major (LBO = chunk stride)
+        constexpr uint32_t kMn = (uint32_t)((C::CHUNK_N - 16) >> 4) << 16;  // K-major -> MN-major (LBO = chunk stride)
         constexpr uint32_t oQ = 0, oDO = C::TILE_M >> 4, oK = (C::OFF_K - C::OFF_Q) >> 4, oV = (C::OFF_V - C::OFF_Q) >> 4,
                            kTile16 = C::TILE_N >> 4;
         auto koff_m = [](int kk) { return (uint32_t)(((kk >> 2) * kChunkM + (kk & 3) * 32) >> 4); };  // K-major k-step
-        auto koff_n = [](int kk) { return (uint32_t)(((kk >> 2) * kChunkN + (kk & 3) * 32) >> 4); };
+        auto koff_n = [](int kk) { return (uint32_t)(((kk >> 2) * C::CHUNK_N + (kk & 3) * 32) >> 4); };
         auto moff = [](int kk) { return (uint32_t)((kk * 2048) >> 4) + kMn; };                        // MN-major k-step
         auto issue_s = [&](uint32_t d_col, uint32_t a_lo, uint32_t b_lo, uint32_t bar) {
 #pragma unroll
@@ -400,8 +409,8 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_dq_tc_kernel(const __grid_con
             if (!ok) break;
             tc_fence_after();
 #pragma unroll
-            for (int kk = 0; kk < kN / 16; ++kk)
-              mma_ts_w(tmem + C::COL_DQ, tmem + C::COL_DP + (kk >> 1) * 32 + (kk & 1) * 8, dsc(oK + ks * kTile16 + moff(kk)),
+            for (int kk = 0; kk < KN / 16; ++kk)  // (a warpgroup's dS sits over the first half of its columns of dP)
+              mma_ts_w(tmem + C::COL_DQ, tmem + C::COL_DP + kk / (KN / 32) * (KN / 2) + kk % (KN / 32) * 8, dsc(oK + ks * kTile16 + moff(kk)),
                        idesc_dq, (j > 0) || kk > 0);
             tc_commit_w(bar_k_empty(ks));
             if (j + 1 < iters) ok = issue_dp(j + 1);
@@ -426,9 +435,9 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_dq_tc_kernel(const __grid_con
 }
 
 
-template <typename T, int DH>
+template <typename T, int DH, int KN>
 int launch_bwd_dq_tc(const FaBwdArgs& a, cudaStream_t st) {
-  using C = QCfg<DH>;
+  using C = QCfg<DH, KN>;
   DqTcParams P;
   P.a = a;
   const bool varlen = a.cu_seqlens_q != nullptr;
@@ -436,10 +445,11 @@ int launch_bwd_dq_tc(const FaBwdArgs& a, cudaStream_t st) {
   const int64_t nb = varlen ? 1 : a.batch;
   if (make_tmap_4d(&P.tq, a.q, a.dtype, q_rows, a.heads, nb, a.head_dim, kM)) return 1;
   if (make_tmap_4d(&P.tdo, a.dout, a.dtype, q_rows, a.heads, nb, a.head_dim, kM)) return 1;
-  if (make_tmap_4d(&P.tk, a.k, a.dtype, k_rows, a.heads_k, nb, a.head_dim, kN)) return 1;
-  if (make_tmap_4d(&P.tv, a.v, a.dtype, k_rows, a.heads_k, nb, a.head_dim, kN)) return 1;
-  const bool uneven = a.window_left >= 0 || a.window_right >= 0 || a.cu_seqlens_q;
-  auto kern = uneven ? bwd_dq_tc_kernel<T, DH, true> : bwd_dq_tc_kernel<T, DH, false>;
+  if (make_tmap_4d(&P.tk, a.k, a.dtype, k_rows, a.heads_k, nb, a.head_dim, KN)) return 1;
+  if (make_tmap_4d(&P.tv, a.v, a.dtype, k_rows, a.heads_k, nb, a.head_dim, KN)) return 1;
+  // (CTAs that all start at once need no order)
+  const bool uneven = KN <= 64 && (a.window_left >= 0 || a.window_right >= 0 || a.cu_seqlens_q);
+  auto kern = uneven ? bwd_dq_tc_kernel<T, DH, KN, (KN <= 64)> : bwd_dq_tc_kernel<T, DH, KN, false>;
   P.status = status_ref(true);
   static fa_host::DeviceOnce once[2];
   if (int rc = fa_host::raise_smem_limit(once[uneven], reinterpret_cast<const void*>(kern), C::SMEM_BYTES, "bwd_dq_tc_kernel")) return rc;
@@ -453,10 +463,19 @@ int launch_bwd_dq_tc(const FaBwdArgs& a, cudaStream_t st) {
 
 }  // namespace
 
-int bwd_dq_tc_main(const FaBwdArgs& a, cudaStream_t st) {
+template <int KN>
+static int dq_dispatch(const FaBwdArgs& a, cudaStream_t st) {
   const bool bf = a.dtype == FA_DTYPE_BF16;
-  if (a.head_dim <= 64) return bf ? launch_bwd_dq_tc<__nv_bfloat16, 64>(a, st) : launch_bwd_dq_tc<__half, 64>(a, st);
-  return bf ? launch_bwd_dq_tc<__nv_bfloat16, 128>(a, st) : launch_bwd_dq_tc<__half, 128>(a, st);
+  if (a.head_dim <= 64) return bf ? launch_bwd_dq_tc<__nv_bfloat16, 64, KN>(a, st) : launch_bwd_dq_tc<__half, 64, KN>(a, st);
+  return bf ? launch_bwd_dq_tc<__nv_bfloat16, 128, KN>(a, st) : launch_bwd_dq_tc<__half, 128, KN>(a, st);
+}
+
+int bwd_dq_tc_main(const FaBwdArgs& a, cudaStream_t st) {
+  // 128-key blocks where no two CTAs share an SM: 1 x 1024 tokens, 16 heads of 128 (128 CTAs) 21.5 us with 64 keys, 17.3 with
+  // 128; 1 x 2048, 8/2 heads of 128 35.4 and 27.7; 1 x 16384, 1 head of 64 (128 CTAs) 164 and 137.  From 149 CTAs on two share:
+  // 8 x 256, 10 heads of 128 (160 CTAs) 13.6 and 16.1; 1 x 2048, 16 heads of 64 (256 CTAs) 39.9 and 42.1.
+  const int64_t ctas = (int64_t)((a.seqlen_q + kM - 1) / kM) * a.heads * a.batch;
+  return ctas <= fa_host::sm_count() ? dq_dispatch<128>(a, st) : dq_dispatch<64>(a, st);
 }
 
 }  // namespace fa

@@ -9,7 +9,7 @@
 // the latency of the Q / dO tile loads.  Two more MMAs per block cost less than that, need no
 // workspace, and make the gradient deterministic.
 //
-// One CTA owns 128 keys of one (batch, KV head) and walks every query block (128 rows; 64 at head dim 64) that can see
+// One CTA owns 128 keys of one (batch, KV head) and walks every query block (128 rows; 64 mostly at head dim 64) that can see
 // them, for every query head of the KV head's group (so grouped-query dK/dV need no expanded
 // temporaries or group reduction, cf. flash_api.cpp:744-751, 799-803).  Everything is computed
 // TRANSPOSED so that the operands the tensor cores need next are already where tcgen05 wants them:
@@ -25,7 +25,8 @@
 //   Head dim 128: tensor memory and shared memory are full with one CTA.  16 compute warps instead of 8 were slower (the
 //   power cap on long sequences), and so was dS in shared memory (the Q ring shrinks to two slots, S(i+1) waits for Q).
 //   Head dim 64: half the tile rows, 256 columns and 113 KiB, so that two CTAs share an SM and one's waits, start and end
-//   run under the other's blocks; the exponentials (16 per clock and SM: 1024 cycles per 128 x 128) come next.
+//   run under the other's blocks; the exponentials (16 per clock and SM: 1024 cycles per 128 x 128) come next.  Where the
+//   grid leaves every CTA an SM of its own, the tiles of head dim 128 (bwd_tc_main).
 //   (dS in shared memory, so that dP(i+1) need not wait for dK(i), was slower: 1084 -> 1210 us below.)
 //   Start and end: the first loads leave before the CTA has set itself up, and the result leaves in whole rows through
 //   shared memory (a row per thread cost 7700 cycles per CTA at head dim 128, it is 4300 now).
@@ -53,20 +54,20 @@ constexpr int kChunkBytes = kB * 128;   // [128 rows][64 x 16-bit]
 enum BwdWait { W_B_KV = 21, W_B_QDO_FULL = 22, W_B_QDO_EMPTY = 23, W_B_STATS_FULL = 24, W_B_STATS_EMPTY = 25,
                W_B_S = 26, W_B_DP = 27, W_B_PDS = 28, W_B_ALIGN = 20 };
 
-template <int DH>
+// BQ: query rows per block
+template <int DH, int BQ>
 struct BCfg {
   static constexpr int NCHUNK = DH / 64;
-  static constexpr int BQ = DH > 64 ? 128 : 64;  // query rows per block
   static constexpr int QCHUNK = BQ * 128;
   static constexpr int TILE_K = NCHUNK * kChunkBytes, TILE_Q = NCHUNK * QCHUNK;  // K / V tile, Q / dO tile
   // 8 compute warps: each takes 32 key rows and half the query columns of a block
   static constexpr int WARPS = 8, CW = BQ / 2;
   static constexpr int THREADS = 32 * WARPS + 128;
   static constexpr int WARP_PRODUCER = WARPS, WARP_MMA = WARPS + 1, WARP_STATS = WARPS + 2, WARP_MMA_S = WARPS + 3;
-  static constexpr int CTAS = DH > 64 ? 1 : 2;  // per SM
+  static constexpr int CTAS = BQ > 64 ? 1 : 2;  // per SM
   // a thread is launched with 168 (one CTA) or 80 registers (two): setmaxnreg only redistributes those
-  static constexpr int REGS = DH > 64 ? 200 : 88, REGS_OTHER = DH > 64 ? 104 : 64;
-  static_assert(256 * REGS + 128 * REGS_OTHER <= THREADS * (DH > 64 ? 168 : 80), "the registers of one CTA");
+  static constexpr int REGS = BQ > 64 ? 200 : 88, REGS_OTHER = BQ > 64 ? 104 : 64;
+  static_assert(256 * REGS + 128 * REGS_OTHER <= THREADS * (BQ > 64 ? 168 : 80), "the registers of one CTA");
   // Q(i) is needed from S^T(i) (issued a block early) to dK(i), dO(i) from dP^T(i) to dV(i): Q gets the deeper ring
   static constexpr int NSQ = DH > 64 ? 3 : 4, NSO = DH > 64 ? 2 : 4;
   static constexpr int OFF_K = 0;
@@ -78,8 +79,8 @@ struct BCfg {
   static constexpr int NBAR = 2 * NSQ + 2 * NSO + 11;
   static constexpr int SMEM_BYTES = OFF_BAR + NBAR * 8 + 32;
   static constexpr int COL_S = 0, COL_DP = BQ, COL_DV = 2 * BQ, COL_DK = 2 * BQ + DH;
-  static constexpr int TMEM_COLS = 2 * BQ + 2 * DH;
-  static_assert(CTAS * (SMEM_BYTES + 1024) <= 228 * 1024 && CTAS * TMEM_COLS <= 512, "what the CTAs of an SM share");
+  static constexpr int TMEM_COLS = BQ > 64 ? 512 : 256;
+  static_assert(CTAS * (SMEM_BYTES + 1024) <= 228 * 1024 && COL_DK + DH <= TMEM_COLS, "what the CTAs of an SM share");
 };
 
 struct BwdTcParams {
@@ -103,13 +104,13 @@ struct BFmt<__nv_bfloat16> {
 
 // UNEVEN: CTAs in the order of cta_item.  (An instance of its own: with the block and head worked out instead of read from
 // blockIdx the even case took 4 % longer at head dim 64.)
-template <typename T, int DH, bool UNEVEN>
-__global__ void __launch_bounds__(BCfg<DH>::THREADS, BCfg<DH>::CTAS) bwd_tc_kernel(const __grid_constant__ BwdTcParams P) {
-  using C = BCfg<DH>;
+template <typename T, int DH, int BQ, bool UNEVEN>
+__global__ void __launch_bounds__(BCfg<DH, BQ>::THREADS, BCfg<DH, BQ>::CTAS) bwd_tc_kernel(const __grid_constant__ BwdTcParams P) {
+  using C = BCfg<DH, BQ>;
   const FaBwdArgs& a = P.a;
   extern __shared__ __align__(1024) unsigned char smem[];
   const uint32_t s_base = smem_addr(smem);
-  constexpr int NSQ = C::NSQ, NSO = C::NSO, BQ = C::BQ, CW = C::CW;
+  constexpr int NSQ = C::NSQ, NSO = C::NSO, CW = C::CW;
   const uint32_t sK = s_base + C::OFF_K, sV = s_base + C::OFF_V;
   auto sQ = [&](int slot) { return s_base + C::OFF_Q + slot * C::TILE_Q; };
   auto sDO = [&](int slot) { return s_base + C::OFF_DO + slot * C::TILE_Q; };
@@ -531,20 +532,21 @@ __global__ void __launch_bounds__(BCfg<DH>::THREADS, BCfg<DH>::CTAS) bwd_tc_kern
 }
 
 
-template <typename T, int DH>
+template <typename T, int DH, int BQ>
 int launch_bwd_tc(const FaBwdArgs& a, cudaStream_t st) {
-  using C = BCfg<DH>;
+  using C = BCfg<DH, BQ>;
   BwdTcParams P;
   P.a = a;
   const bool varlen = a.cu_seqlens_q != nullptr;
   const int64_t q_rows = varlen ? a.total_q : a.seqlen_q, k_rows = varlen ? a.total_k : a.seqlen_k;
   const int64_t nb = varlen ? 1 : a.batch;
-  if (make_tmap_4d(&P.tq, a.q, a.dtype, q_rows, a.heads, nb, a.head_dim, C::BQ)) return 1;
-  if (make_tmap_4d(&P.tdo, a.dout, a.dtype, q_rows, a.heads, nb, a.head_dim, C::BQ)) return 1;
+  if (make_tmap_4d(&P.tq, a.q, a.dtype, q_rows, a.heads, nb, a.head_dim, BQ)) return 1;
+  if (make_tmap_4d(&P.tdo, a.dout, a.dtype, q_rows, a.heads, nb, a.head_dim, BQ)) return 1;
   if (make_tmap_4d(&P.tk, a.k, a.dtype, k_rows, a.heads_k, nb, a.head_dim, kB)) return 1;
   if (make_tmap_4d(&P.tv, a.v, a.dtype, k_rows, a.heads_k, nb, a.head_dim, kB)) return 1;
-  const bool uneven = a.window_left >= 0 || a.window_right >= 0 || a.cu_seqlens_q;
-  auto kern = uneven ? bwd_tc_kernel<T, DH, true> : bwd_tc_kernel<T, DH, false>;
+  constexpr bool kAlone = DH <= 64 && BQ > 64;  // (CTAs that all start at once need no order)
+  const bool uneven = !kAlone && (a.window_left >= 0 || a.window_right >= 0 || a.cu_seqlens_q);
+  auto kern = uneven ? bwd_tc_kernel<T, DH, BQ, !kAlone> : bwd_tc_kernel<T, DH, BQ, false>;
   P.status = status_ref(true);
   static fa_host::DeviceOnce once[2];
   if (int rc = fa_host::raise_smem_limit(once[uneven], reinterpret_cast<const void*>(kern), C::SMEM_BYTES, "bwd_tc_kernel")) return rc;
@@ -575,8 +577,16 @@ bool bwd_tc_eligible(const FaBwdArgs& a) {
 
 int bwd_tc_main(const FaBwdArgs& a, cudaStream_t st) {
   const bool bf = a.dtype == FA_DTYPE_BF16;
-  if (a.head_dim <= 64) return bf ? launch_bwd_tc<__nv_bfloat16, 64>(a, st) : launch_bwd_tc<__half, 64>(a, st);
-  return bf ? launch_bwd_tc<__nv_bfloat16, 128>(a, st) : launch_bwd_tc<__half, 128>(a, st);
+  if (a.head_dim <= 64) {
+    // 128-row blocks where no two CTAs share an SM: 1 x 2048 tokens, 8/2 heads (32 CTAs) 107.6 us with 64 rows, 81.5 with 128;
+    // 1 x 1024, 16 heads (128 CTAs) 19.3 and 16.0.  From 149 CTAs on two share: 8 x 256, 10 heads (160 CTAs) 10.5 and 13.9;
+    // 1 x 2048, 16 heads (256 CTAs) 46.1 and 50.2.
+    const int64_t ctas = (int64_t)((a.seqlen_k + kB - 1) / kB) * a.heads_k * a.batch;
+    if (ctas <= fa_host::sm_count())
+      return bf ? launch_bwd_tc<__nv_bfloat16, 64, 128>(a, st) : launch_bwd_tc<__half, 64, 128>(a, st);
+    return bf ? launch_bwd_tc<__nv_bfloat16, 64, 64>(a, st) : launch_bwd_tc<__half, 64, 64>(a, st);
+  }
+  return bf ? launch_bwd_tc<__nv_bfloat16, 128, 128>(a, st) : launch_bwd_tc<__half, 128, 128>(a, st);
 }
 
 }  // namespace fa
