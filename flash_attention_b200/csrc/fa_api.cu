@@ -199,19 +199,23 @@ int fa_abi_struct_size(int32_t which) {
 int fa_fwd_num_splits(int32_t batch, int32_t heads, int32_t seqlen_q, int32_t seqlen_k, int32_t head_dim,
                       int32_t num_sms) {
   // For the tensor-core kernel (a work item is 256 query rows, 128 above head dim 128, and walks 128-key blocks): the
-  // split count with the least estimated time.  A block takes about 2 us, a round of CTAs 5 us before and after its
-  // blocks, merging the parts 5 us and what writing and reading their fp32 rows takes at 5 TB/s.  On 2 x 512 x 8 x 64,
-  // where a split into single blocks fills the SMs, that split took 9.2 + 6.2 us.
+  // split count with the least estimated time, in us.  The terms are fitted to 362 shapes of head dim 64 to 256, 8 to 2048
+  // query rows and 128 to 32768 keys, each timed with up to 17 counts (one B200, 1965 MHz): a round of CTAs takes 6 and 1.75
+  // (d <= 64), 2 (d <= 128) or 2.25 per key block, the merge 4, 0.15 per part and what writing and reading the parts' fp32
+  // rows takes at 5 TB/s.  The count it finds is 0.5 % off the best one on average and 7 % at most.  With 2 per block for all
+  // head dims, 5 for the merge and nothing per part: 0.8 % and 20 %; with splits_by_wave_efficiency: 7 % and a factor
+  // of 2.3.  (82 x 7511, 2 heads of 256: 1 part 125 us, 59 parts 33.5, 20 parts 24.7.)  A mask is not looked at.
   if (num_sms <= 0) num_sms = fa_host::sm_count();
   const int rows = head_dim > 128 ? 128 : 256;
   const int64_t ctas = (int64_t)batch * heads * ((seqlen_q + rows - 1) / rows);
   const int n_blocks = (seqlen_k + 127) / 128;
   if (ctas >= 0.8f * num_sms) return 1;
-  const float part_us = (float)batch * heads * seqlen_q * head_dim * 8.f / 5e6f;
+  const float block_us = head_dim <= 64 ? 1.75f : head_dim <= 128 ? 2.f : 2.25f;
+  const float part_us = 0.15f + (float)batch * heads * seqlen_q * head_dim * 8.f / 5e6f;
   int best = 1;
-  float best_time = 5.f + 2.f * n_blocks;
+  float best_time = 6.f + block_us * n_blocks;
   for (int s = 2; s <= n_blocks && s <= 128; ++s) {
-    const float t = (float)((ctas * s + num_sms - 1) / num_sms) * (5.f + 2.f * ((n_blocks + s - 1) / s)) + 5.f + s * part_us;
+    const float t = (float)((ctas * s + num_sms - 1) / num_sms) * (6.f + block_us * ((n_blocks + s - 1) / s)) + 4.f + s * part_us;
     if (t < best_time) {
       best_time = t;
       best = s;

@@ -311,3 +311,15 @@ def test_stream_without_the_private_shortcut(monkeypatch):
     assert m._stream(t) == 77
     monkeypatch.setattr(m, "_raw_stream", lambda index: (index, 78))
     assert m._stream(t) == (t.device.index, 78)
+
+
+@pytest.mark.parametrize("batch,heads,rows,keys,d,lo,hi", [
+    (1, 2, 82, 7511, 256, 12, 32),   # measured: 1 part 125 us, 12 to 32 parts 24.7 to 26.6, 59 parts of one block 33.5
+    (1, 2, 13 * 4, 4380, 128, 8, 24),  # 1 part 58 us, 8 to 24 parts 16.5 to 18.7, 35 parts 19.8
+    (1, 5, 777, 777, 256, 3, 6),     # 1 part 21.3 us, 4 parts 20.2
+    (2, 8, 512, 512, 64, 1, 1),      # 1 part 12.6 us, 4 parts 9.2 + 6.2
+    (1, 8, 128, 128, 128, 1, 1),     # one block
+    (16, 16, 2048, 2048, 128, 1, 1),  # the items fill the SMs
+])
+def test_split_count_of_a_dense_forward(lib, batch, heads, rows, keys, d, lo, hi):
+    assert lo <= lib.fa_fwd_num_splits(batch, heads, rows, keys, d, 148) <= hi
