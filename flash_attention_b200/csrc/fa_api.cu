@@ -294,7 +294,7 @@ int fa_bwd(const FaBwdArgs* a, fa_stream_t stream) {
   if (refuse_if_device_failed()) return 3;
   const bool tc = a->seqlen_k > 0 && !fa_host::env_flag("FA_B200_FORCE_GENERIC") && fa::bwd_tc_eligible(*a);
   const int parts = a->parts == 0 ? 3 : a->parts;  // bit 0: dot(dO, O) and dQ, bit 1: dK and dV
-  FA_REQUIRE(parts >= 1 && parts <= 3, "parts must be 0 (everything), 1 (preprocess and dQ) or 2 (dK and dV)");
+  FA_REQUIRE(parts >= 1 && parts <= 3, "parts must be 0 (everything), 1 (D = rowsum(dO o O) and dQ) or 2 (dK and dV)");
   FA_REQUIRE(parts == 3 || tc, "a backward pass can only be split in parts on the tensor-core path");
   // the tensor-core path writes dq directly (two kernels: dQ per query block, which also leaves D = rowsum(dO o O) for
   // the second, dK / dV per key block; head dims above 128: a pass per output after a launch of its own for D)
