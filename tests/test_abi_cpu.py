@@ -2,6 +2,7 @@
 include/fa_b200.h declares, agrees with the ctypes layout, validates arguments before any launch,
 and the drop-in module has the five entry points of the reference's extension."""
 import ctypes
+import importlib
 import inspect
 import os
 import re
@@ -306,11 +307,16 @@ def test_stream_without_the_private_shortcut(monkeypatch):
         cuda_stream = 77
 
     t = torch.empty(1)
-    monkeypatch.setattr(torch.cuda, "current_stream", lambda device: Stream)
-    monkeypatch.setattr(m, "_raw_stream", None)
-    assert m._stream(t) == 77
-    monkeypatch.setattr(m, "_raw_stream", lambda index: (index, 78))
-    assert m._stream(t) == (t.device.index, 78)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda index: Stream)
+    try:
+        with monkeypatch.context() as mp:
+            mp.delattr(torch._C, "_cuda_getCurrentRawStream", raising=False)
+            assert importlib.reload(m)._stream(t) == 77
+        with monkeypatch.context() as mp:
+            mp.setattr(torch._C, "_cuda_getCurrentRawStream", lambda index: (index, 78), raising=False)
+            assert importlib.reload(m)._stream(t) == (t.device.index, 78)
+    finally:
+        importlib.reload(m)
 
 
 @pytest.mark.parametrize("batch,heads,rows,keys,d,lo,hi", [
