@@ -11,11 +11,13 @@
 //   warp  9     MMA issuer: the warp stays converged, one elected lane issues every tcgen05.mma
 //   warp  10    owns the TMEM allocation
 //   warp  11    KV cache: clears the rows of the last V tile that hold no key
+// Registers: 168 a thread at launch, 4 to 8 bytes spilled.
 // With grouped-query heads a tile's 128 rows are (positions x heads of the group), so that both tiles of a CTA end at the same
 // key block of a causal mask and a few tokens per sequence fill a tile (prefill of 4096 tokens, 32/8 heads: 179 -> 157 us, and
 // 137 with the CTA order of cta_item).  K and V may be a KV cache: lengths on the device, batch index, pages of 64 rows and up.
 // What bounds it: the chain S -> softmax -> PV of each tile (about 3100 cycles per pair of 128 x 128 blocks, 2048 of MMA and 2048
-// of exponentials at 16 per clock and SM), and per CTA about 5000 cycles before the first and 5000 after the last block.
+// of exponentials at 16 per clock and SM), and per CTA about 5000 cycles before the first and 5000 after the last block (the latter
+// worked out from launch times).
 // 16 x 2048 x 16 x 128 causal 400 -> 337 us.
 // TMEM columns (fp32): S0 [0,128) S1 [128,256) O0 [256,256+D) O1 [256+D,256+2D).  P (16-bit) is
 // written over the first 64 columns of its S and fed to the PV MMA as the TMEM A operand.
@@ -725,8 +727,11 @@ int fwd_tc(const FaFwdArgs& a, cudaStream_t st) { return fwd_tc_run(a, 0, st); }
 
 // Several tokens per sequence against a KV cache (4 x 128 tokens, 32/8 heads, pages of 256: 469 us on the any-shape kernel,
 // 62 + 13 us merge here).  From 17 rows (tokens x heads of a group) on, where the decode kernel's 16 end: 20 rows, batch 8,
-// 8192 keys, 32/8 heads of 128 575 -> 131 us; 17 rows, batch 2, 16384 keys, 8 heads of 64 109 -> 58 us.  With a window
+// 8192 keys, 32/8 heads of 128 575 -> 126 us; 17 rows, batch 2, 16384 keys, 8 heads of 64 109 -> 59 us.  With a window
 // that cuts keys off, the any-shape kernel's 64-row tiles keep what has 32 rows or fewer, and other head dims' few rows.
+// The lengths are on the device and the capacity stands for them.  Short sequences in large caches pay for that (16 x 33 rows,
+// 4 heads of 128, capacity 8192, attention and merge here / any-shape: no keys before the call 15 / 10 us, 400 21 / 17,
+// 1500 28 / 41, 3900 53 / 137; 64 sequences, 32 heads of 64: 90 / 26 without keys, 151 / 193 with 400, 667 / 1537 with 3900).
 bool fwd_tc_cache_eligible(const FaFwdArgs& a, int64_t kv_batches) {
   const int64_t rows = (int64_t)a.seqlen_q * (a.heads / a.heads_k);
   const bool all_keys = a.window_right <= 0 && (a.window_left < 0 || (a.window_right == 0 && a.window_left >= a.seqlen_k));
