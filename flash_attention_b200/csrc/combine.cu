@@ -15,19 +15,23 @@ struct CombineParams {
   int32_t n_parts, B, H, S, D, lse_pitch;
 };
 
-template <typename T>
+// G: groups of 32 parts, one part per lane.  One group is an instance of its own, without the choice among groups and with two
+// steps of the walk in flight, four with more groups (16384 rows of 128 in 5 parts: 10.9 us, 11.6 with four groups for all;
+// 2048 rows in 64 parts: 12.6 us, 16.6 with two steps in flight).
+template <typename T, int G>
 __global__ void __launch_bounds__(128) combine_kernel(const CombineParams p) {
   const int lane = threadIdx.x & 31;
   const int64_t rows = (int64_t)p.B * p.H * p.S;
   const int64_t row = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
   if (row >= rows) return;
-  // up to 128 parts: 4 per lane
-  float l[4];
+  float l[G];
+  uint32_t live[G];  // parts with keys (+inf is not an LSE of theirs)
   float mx = -INFINITY;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < G; ++i) {
     int s = lane + 32 * i;
     l[i] = s < p.n_parts ? p.lse_parts[(int64_t)s * rows + row] : -INFINITY;
+    live[i] = __ballot_sync(0xffffffffu, l[i] != -INFINITY && l[i] != INFINITY);
     mx = fmaxf(mx, l[i]);
   }
 #pragma unroll
@@ -35,11 +39,11 @@ __global__ void __launch_bounds__(128) combine_kernel(const CombineParams p) {
   float sum = 0.f;
   const float msafe = mx == -INFINITY ? 0.f : mx;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) sum += __expf(l[i] - msafe);
+  for (int i = 0; i < G; ++i) sum += __expf(l[i] - msafe);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-  // (fmaxf drops a NaN, so the LSEs are asked)
-  const bool nan = __any_sync(0xffffffffu, l[0] != l[0] || l[1] != l[1] || l[2] != l[2] || l[3] != l[3]);
+  // (fmaxf drops a NaN, the sum does not; an LSE of +inf makes it NaN as well)
+  const bool nan = sum != sum && mx != INFINITY;
   const bool empty = !nan && (!(sum > 0.f) || mx == -INFINITY);
   const float lse = empty || nan ? INFINITY : logf(sum) + mx;
   const int s_idx = (int)(row % p.S);
@@ -49,24 +53,27 @@ __global__ void __launch_bounds__(128) combine_kernel(const CombineParams p) {
   T* o = reinterpret_cast<T*>(p.out) + b * p.out_sb + s_idx * p.out_ss + h * p.out_sh;
   // head_dim <= 256: at most two 4-column groups per lane
   float4 acc[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
-  float wgt[4];
-  uint32_t live[4];
+  float wgt[G];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    wgt[i] = nan ? sum : empty ? 0.f : __expf(l[i] - lse);
-    live[i] = __ballot_sync(0xffffffffu, !empty && l[i] != -INFINITY);
-  }
+  for (int i = 0; i < G; ++i) wgt[i] = nan ? sum : empty ? 0.f : __expf(l[i] - lse);
   // Bound by the latency of the loads: four parts are in flight at a time (16 parts of 2048 x 128: 9.4 us, 11.5 us with one
   // at a time).  Empty parts, those past the last one among them, are not read: nobody may have written them.  The walk ends
-  // behind the last part with keys (2048 rows of 128, 64 parts, 4 of them with keys: 8.9 -> 3.5 us; all with keys: 13.2 ->
-  // 12.3; a test of every four parts in the loop instead: 4.6 and 16.2).
+  // behind the last part with keys (2048 rows of 128, 64 parts, 4 of them with keys: 8.9 -> 3.5 us; a test of every four parts
+  // in the loop instead: 4.6, and 16.2 where all have keys).
+  constexpr int kSteps = G == 1 ? 2 : 4;
   int end = 0;
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < G; ++i)
     if (live[i]) end = 32 * (i + 1) - __clz(live[i]);
+#pragma unroll kSteps
   for (int s0 = 0; s0 < end; s0 += 4) {  // uniform trip count: every lane takes part in the shuffles
-    const float wsel = (s0 >> 5) == 0 ? wgt[0] : (s0 >> 5) == 1 ? wgt[1] : (s0 >> 5) == 2 ? wgt[2] : wgt[3];
-    const uint32_t lsel = ((s0 >> 5) == 0 ? live[0] : (s0 >> 5) == 1 ? live[1] : (s0 >> 5) == 2 ? live[2] : live[3]) >> (s0 & 31);
+    float wsel = wgt[0];
+    uint32_t lsel = live[0];
+    if constexpr (G > 1) {
+      wsel = (s0 >> 5) == 0 ? wgt[0] : (s0 >> 5) == 1 ? wgt[1] : (s0 >> 5) == 2 ? wgt[2] : wgt[3];
+      lsel = (s0 >> 5) == 0 ? live[0] : (s0 >> 5) == 1 ? live[1] : (s0 >> 5) == 2 ? live[2] : live[3];
+    }
+    lsel >>= s0 & 31;
     float w[4];
     float4 x[4][2];
 #pragma unroll
@@ -106,10 +113,9 @@ int combine(const float* out_parts, const float* lse_parts, const FaTensor& out,
   CombineParams p{out_parts, lse_parts, out.ptr, lse, out.stride_b, out.stride_s, out.stride_h, n_parts, B, H, S, D, lse_pitch};
   int64_t rows = (int64_t)B * H * S;
   unsigned grid = (unsigned)((rows + 3) / 4);
-  if (dtype == FA_DTYPE_BF16)
-    combine_kernel<__nv_bfloat16><<<grid, 128, 0, st>>>(p);
-  else
-    combine_kernel<__half><<<grid, 128, 0, st>>>(p);
+  auto kern = dtype == FA_DTYPE_BF16 ? (n_parts <= 32 ? combine_kernel<__nv_bfloat16, 1> : combine_kernel<__nv_bfloat16, 4>)
+                                     : (n_parts <= 32 ? combine_kernel<__half, 1> : combine_kernel<__half, 4>);
+  kern<<<grid, 128, 0, st>>>(p);
   return fa_host::check_launch("combine_kernel");
 }
 
