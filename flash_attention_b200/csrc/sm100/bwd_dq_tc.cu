@@ -89,7 +89,7 @@ struct QFmt<__nv_bfloat16> {
 
 // UNEVEN: CTAs in the order of cta_item.  (An instance of its own: with the block and head worked out instead of read from
 // blockIdx the even case took 4 % longer at head dim 64.)
-template <typename T, int DH, int KN, bool UNEVEN>
+template <typename T, int DH, int KN, bool UNEVEN, bool TRIM>
 __global__ void __launch_bounds__(kThreads, QCfg<DH, KN>::CTAS) bwd_dq_tc_kernel(const __grid_constant__ DqTcParams P) {
   using C = QCfg<DH, KN>;
   constexpr int NSK = C::NSK, NSV = C::NSV;
@@ -358,10 +358,11 @@ __global__ void __launch_bounds__(kThreads, QCfg<DH, KN>::CTAS) bwd_dq_tc_kernel
       // Warp 9 issues S(j+1) as soon as the compute warps hold S(j) in registers; warp 11 issues the chain
       // dQ(j) | dP(j+1): dS(j) sits over dP(j), and the MMAs of one thread execute in order.  MMAs of the two threads are
       // not ordered among themselves and need not be.
-      if (run) {  // the whole warp runs the loops (see mma_ss_w); one elected lane issues
+      if (run) with_head_steps<DH, TRIM>(a.head_dim, [&](auto steps) {  // the whole warp runs the loops (see mma_ss_w); one elected lane issues
         constexpr int F = QFmt<T>::kIdesc;
         constexpr uint32_t idesc_s = make_idesc(kM, KN, F, 0, 0);   // S, dP: K-major x K-major, N = KN keys
-        constexpr uint32_t idesc_dq = make_idesc(kM, DH, F, 0, 1);  // dQ: A in TMEM, B MN-major, N = DH
+        constexpr int KS = decltype(steps)::value;
+        constexpr uint32_t idesc_dq = make_idesc(kM, KS * 16, F, 0, 1);  // dQ: A in TMEM, B MN-major, N = head dim
         // One descriptor is built (Q tile, K-major); every other operand differs from it only in the
         // low word: the address field (+ byte offset >> 4) and, for MN-major reads, the LBO field.
         const uint64_t d_base = smem_desc_sw128(sQ, 16, 1024);
@@ -375,7 +376,8 @@ __global__ void __launch_bounds__(kThreads, QCfg<DH, KN>::CTAS) bwd_dq_tc_kernel
         auto moff = [](int kk) { return (uint32_t)((kk * 2048) >> 4) + kMn; };                        // MN-major k-step
         auto issue_s = [&](uint32_t d_col, uint32_t a_lo, uint32_t b_lo, uint32_t bar) {
 #pragma unroll
-          for (int kk = 0; kk < DH / 16; ++kk) mma_ss_w(tmem + d_col, dsc(a_lo + koff_m(kk)), dsc(b_lo + koff_n(kk)), idesc_s, kk > 0);
+          for (int kk = 0; kk < KS; ++kk)
+            mma_ss_w(tmem + d_col, dsc(a_lo + koff_m(kk)), dsc(b_lo + koff_n(kk)), idesc_s, kk > 0);
           tc_commit_w(bar);
         };
         if (warp == kWarpMma) {
@@ -417,7 +419,7 @@ __global__ void __launch_bounds__(kThreads, QCfg<DH, KN>::CTAS) bwd_dq_tc_kernel
           }
           if (ok) tc_commit_w(bar_done);
         }
-      }
+      });
     }
   }
 
@@ -449,10 +451,12 @@ int launch_bwd_dq_tc(const FaBwdArgs& a, cudaStream_t st) {
   if (make_tmap_4d(&P.tv, a.v, a.dtype, k_rows, a.heads_k, nb, a.head_dim, KN)) return 1;
   // (CTAs that all start at once need no order)
   const bool uneven = KN <= 64 && (a.window_left >= 0 || a.window_right >= 0 || a.cu_seqlens_q);
-  auto kern = uneven ? bwd_dq_tc_kernel<T, DH, KN, (KN <= 64)> : bwd_dq_tc_kernel<T, DH, KN, false>;
+  const bool trim = head_trims<DH>(a.head_dim);
+  auto kern = trim ? (uneven ? bwd_dq_tc_kernel<T, DH, KN, (KN <= 64), true> : bwd_dq_tc_kernel<T, DH, KN, false, true>)
+                   : (uneven ? bwd_dq_tc_kernel<T, DH, KN, (KN <= 64), false> : bwd_dq_tc_kernel<T, DH, KN, false, false>);
   P.status = status_ref(true);
-  static fa_host::DeviceOnce once[2];
-  if (int rc = fa_host::raise_smem_limit(once[uneven], reinterpret_cast<const void*>(kern), C::SMEM_BYTES, "bwd_dq_tc_kernel")) return rc;
+  static fa_host::DeviceOnce once[2][2];
+  if (int rc = fa_host::raise_smem_limit(once[trim][uneven], reinterpret_cast<const void*>(kern), C::SMEM_BYTES, "bwd_dq_tc_kernel")) return rc;
   const int rows = a.d_seqlen > a.seqlen_q ? a.d_seqlen : a.seqlen_q;  // the padding rows of D are written too
   dim3 grid((rows + kM - 1) / kM, a.heads, a.batch);
   P.head_group = fa_host::cta_head_group(uneven, (int64_t)a.seqlen_k * a.head_dim * 4 / (a.heads / a.heads_k),

@@ -104,7 +104,7 @@ struct BFmt<__nv_bfloat16> {
 
 // UNEVEN: CTAs in the order of cta_item.  (An instance of its own: with the block and head worked out instead of read from
 // blockIdx the even case took 4 % longer at head dim 64.)
-template <typename T, int DH, int BQ, bool UNEVEN>
+template <typename T, int DH, int BQ, bool UNEVEN, bool TRIM>
 __global__ void __launch_bounds__(BCfg<DH, BQ>::THREADS, BCfg<DH, BQ>::CTAS) bwd_tc_kernel(const __grid_constant__ BwdTcParams P) {
   using C = BCfg<DH, BQ>;
   const FaBwdArgs& a = P.a;
@@ -447,10 +447,11 @@ __global__ void __launch_bounds__(BCfg<DH, BQ>::THREADS, BCfg<DH, BQ>::CTAS) bwd
       // the chain dV(i) | dK(i) | dP^T(i+1): dV(i) waits for P^T(i), dK(i) for dS^T(i); both sit over dP^T(i),
       // and the MMAs of one thread execute in order, so dP^T(i+1) overwrites them only after they were read.
       // MMAs of the two threads are not ordered among themselves and need not be.
-      if (run) {  // the whole warp runs the loops (see mma_ss_w); one elected lane issues
+      if (run) with_head_steps<DH, TRIM>(a.head_dim, [&](auto steps) {  // the whole warp runs the loops (see mma_ss_w); one elected lane issues
         constexpr int F = BFmt<T>::kIdesc;
         constexpr uint32_t idesc_st = make_idesc(kB, BQ, F, 0, 0);   // S^T, dP^T: K-major x K-major, N = BQ queries
-        constexpr uint32_t idesc_dv = make_idesc(kB, DH, F, 0, 1);   // dV, dK: A K-major (or TMEM), B MN-major, N = DH
+        constexpr int KS = decltype(steps)::value;
+        constexpr uint32_t idesc_dv = make_idesc(kB, KS * 16, F, 0, 1);  // dV, dK: A K-major (or TMEM), B MN-major, N = head dim
         // One descriptor is built (K tile, K-major); every other operand differs from it only in the
         // low word: the address field (+ byte offset >> 4) and, for MN-major reads, the LBO field.
         const uint64_t d_base = smem_desc_sw128(sK, 16, 1024);
@@ -465,7 +466,8 @@ __global__ void __launch_bounds__(BCfg<DH, BQ>::THREADS, BCfg<DH, BQ>::CTAS) bwd
         auto pcol = [](int kk) { return kk / (CW / 16) * CW + kk % (CW / 16) * 8; };  // k-step of P in the warps' halves
         auto issue_st = [&](uint32_t d_col, uint32_t a_lo, uint32_t b_lo, uint32_t bar) {
 #pragma unroll
-          for (int kk = 0; kk < DH / 16; ++kk) mma_ss_w(tmem + d_col, dsc(a_lo + koff(kk)), dsc(b_lo + koff_q(kk)), idesc_st, kk > 0);
+          for (int kk = 0; kk < KS; ++kk)
+            mma_ss_w(tmem + d_col, dsc(a_lo + koff(kk)), dsc(b_lo + koff_q(kk)), idesc_st, kk > 0);
           tc_commit_w(bar);
         };
         auto issue_dp = [&](int i) {
@@ -514,7 +516,7 @@ __global__ void __launch_bounds__(BCfg<DH, BQ>::THREADS, BCfg<DH, BQ>::CTAS) bwd
             if (it + 1 < iters) ok = issue_dp(it + 1);
           }
         }
-      }
+      });
     }
   }
 
@@ -546,10 +548,12 @@ int launch_bwd_tc(const FaBwdArgs& a, cudaStream_t st) {
   if (make_tmap_4d(&P.tv, a.v, a.dtype, k_rows, a.heads_k, nb, a.head_dim, kB)) return 1;
   constexpr bool kAlone = DH <= 64 && BQ > 64;  // (CTAs that all start at once need no order)
   const bool uneven = !kAlone && (a.window_left >= 0 || a.window_right >= 0 || a.cu_seqlens_q);
-  auto kern = uneven ? bwd_tc_kernel<T, DH, BQ, !kAlone> : bwd_tc_kernel<T, DH, BQ, false>;
+  const bool trim = head_trims<DH>(a.head_dim);
+  auto kern = trim ? (uneven ? bwd_tc_kernel<T, DH, BQ, !kAlone, true> : bwd_tc_kernel<T, DH, BQ, false, true>)
+                   : (uneven ? bwd_tc_kernel<T, DH, BQ, !kAlone, false> : bwd_tc_kernel<T, DH, BQ, false, false>);
   P.status = status_ref(true);
-  static fa_host::DeviceOnce once[2];
-  if (int rc = fa_host::raise_smem_limit(once[uneven], reinterpret_cast<const void*>(kern), C::SMEM_BYTES, "bwd_tc_kernel")) return rc;
+  static fa_host::DeviceOnce once[2][2];
+  if (int rc = fa_host::raise_smem_limit(once[trim][uneven], reinterpret_cast<const void*>(kern), C::SMEM_BYTES, "bwd_tc_kernel")) return rc;
   dim3 grid((a.seqlen_k + kB - 1) / kB, a.heads_k, a.batch);
   P.head_group = fa_host::cta_head_group(uneven, (int64_t)a.seqlen_q * (a.heads / a.heads_k) * a.head_dim * 4,
                                          (int64_t)a.heads_k * a.batch);

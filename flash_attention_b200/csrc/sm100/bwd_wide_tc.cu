@@ -94,7 +94,7 @@ struct Walk {
   }
 };
 
-template <typename T, int PASS>
+template <typename T, int PASS, bool TRIM>
 __global__ void __launch_bounds__(kThreads, 1) bwd_wide_tc_kernel(const __grid_constant__ WParams P) {
   using C = WCfg<PASS>;
   constexpr int NS1 = C::NS1, NS2 = C::NS2;
@@ -146,6 +146,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_wide_tc_kernel(const __grid_c
     iters = (blk_hi - blk_lo) * group;
   }
 
+  const int nchunk = head_chunks<kDH, TRIM>(a.head_dim);
   if (threadIdx.x == 64) {  // reads global memory: not in front of the first loads
     abort_init(abort_flag, P.status);
     if (s_base & 1023u) abort_raise(abort_flag, W_W_ALIGN);  // the swizzled tiles need a 1024-byte aligned base
@@ -173,8 +174,8 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_wide_tc_kernel(const __grid_c
       // This thread has made the barriers, so it can start the first block's loads while the CTA still sets itself up,
       // in the order in which the first products need them
       auto load = [&](uint32_t dst, const CUtensorMap* tm, uint32_t bar, int chunk, int64_t row, int head, int64_t batch) {
-        mbar_expect_tx(bar, 4 * chunk);
-        for (int c = 0; c < 4; ++c) tma_load_4d(dst + c * chunk, tm, bar, c * 64, (int)row, head, (int)batch);
+        mbar_expect_tx(bar, nchunk * chunk);
+        for (int c = 0; c < nchunk; ++c) tma_load_4d(dst + c * chunk, tm, bar, c * 64, (int)row, head, (int)batch);
       };
       const int64_t arow = (kRowsAreQueries ? si.q_row0 : si.k_row0) + r0, ab = kRowsAreQueries ? si.q_batch : si.k_batch;
       const int64_t brow = (kRowsAreQueries ? si.k_row0 : si.q_row0) + blk_lo * kN, bb = kRowsAreQueries ? si.k_batch : si.q_batch;
@@ -434,13 +435,13 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_wide_tc_kernel(const __grid_c
             if (first) {
               ok = mbar_wait(bar_b1_empty(s1), ((it / NS1) & 1) ^ 1, W_W_B_EMPTY, abort_flag);
               if (!ok) break;
-              mbar_expect_tx(bar_b1_full(s1), kTileB);
-              for (int c = 0; c < 4; ++c) tma_load_4d(sB1(s1) + c * kChunkB, &P.tb1, bar_b1_full(s1), c * 64, brow, bhead, bb);
+              mbar_expect_tx(bar_b1_full(s1), nchunk * kChunkB);
+              for (int c = 0; c < nchunk; ++c) tma_load_4d(sB1(s1) + c * kChunkB, &P.tb1, bar_b1_full(s1), c * 64, brow, bhead, bb);
             } else {
               ok = mbar_wait(bar_b2_empty(s2), ((it / NS2) & 1) ^ 1, W_W_B_EMPTY, abort_flag);
               if (!ok) break;
-              mbar_expect_tx(bar_b2_full(s2), kTileB);
-              for (int c = 0; c < 4; ++c) tma_load_4d(sB2(s2) + c * kChunkB, &P.tb2, bar_b2_full(s2), c * 64, brow, bhead, bb);
+              mbar_expect_tx(bar_b2_full(s2), nchunk * kChunkB);
+              for (int c = 0; c < nchunk; ++c) tma_load_4d(sB2(s2) + c * kChunkB, &P.tb2, bar_b2_full(s2), c * 64, brow, bhead, bb);
             }
           }
         }
@@ -456,10 +457,11 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_wide_tc_kernel(const __grid_c
       //   X2(j+1): once they hold X2(j) and its tile has landed
       //   last product of block j: once W(j) is in its buffer; its commit releases the tile X1(j) read as well
       //   (X1(j) is complete by then: W(j) was computed from it)
-      if (run) {  // the whole warp runs the loops (see mma_ss_w); one elected lane issues
+      if (run) with_head_steps<kDH, TRIM>(a.head_dim, [&](auto steps) {  // the whole warp runs the loops (see mma_ss_w); one elected lane issues
         constexpr int F = WFmt<T>::kIdesc;
         constexpr uint32_t idesc_x = make_idesc(kR, kN, F, 0, 0);    // X1, X2: K-major x K-major, N = 64 streamed rows
-        constexpr uint32_t idesc_o = make_idesc(kR, kDH, F, 0, 1);   // last product: A in TMEM, B MN-major, N = 256
+        constexpr int KS = decltype(steps)::value;
+        constexpr uint32_t idesc_o = make_idesc(kR, KS * 16, F, 0, 1);  // last product: A in TMEM, B MN-major, N = head dim
         // One descriptor is built (first stationary tile, K-major); every other operand differs from it only
         // in the low word: the address field (+ byte offset >> 4) and, for MN-major reads, the LBO field.
         const uint64_t d_base = smem_desc_sw128(s_base + C::OFF_A, 16, 1024);
@@ -473,7 +475,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_wide_tc_kernel(const __grid_c
         auto moff = [](int kk) { return (uint32_t)((kk * 2048) >> 4) + kMn; };  // MN-major k-step: 16 rows of 128 bytes
         auto issue_x = [&](uint32_t d_col, uint32_t a_lo, uint32_t b_lo) {
 #pragma unroll
-          for (int kk = 0; kk < kDH / 16; ++kk)
+          for (int kk = 0; kk < KS; ++kk)
             mma_ss_w(tmem + d_col, dsc(a_lo + koff_a(kk)), dsc(b_lo + koff_b(kk)), idesc_x, kk > 0);
         };
         auto issue_out = [&](int j, uint32_t b_lo) {
@@ -532,7 +534,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_wide_tc_kernel(const __grid_c
           }
           if (ok) tc_commit_w(bar_done);
         }
-      }
+      });
     }
   }
 
@@ -568,10 +570,11 @@ int launch_wide(const FaBwdArgs& a, cudaStream_t st) {
   } else {
     P.ta1 = tk, P.ta2 = tv, P.tb1 = tq, P.tb2 = tdo;
   }
-  auto kern = bwd_wide_tc_kernel<T, PASS>;
+  const bool trim = head_trims<kDH>(a.head_dim);
+  auto kern = trim ? bwd_wide_tc_kernel<T, PASS, true> : bwd_wide_tc_kernel<T, PASS, false>;
   P.status = status_ref(true);
-  static fa_host::DeviceOnce once;
-  if (int rc = fa_host::raise_smem_limit(once, reinterpret_cast<const void*>(kern), C::SMEM_BYTES, "bwd_wide_tc_kernel")) return rc;
+  static fa_host::DeviceOnce once[2];
+  if (int rc = fa_host::raise_smem_limit(once[trim], reinterpret_cast<const void*>(kern), C::SMEM_BYTES, "bwd_wide_tc_kernel")) return rc;
   dim3 grid(((PASS == PASS_DQ ? a.seqlen_q : a.seqlen_k) + kR - 1) / kR, PASS == PASS_DQ ? a.heads : a.heads_k, a.batch);
   const int group = a.heads / a.heads_k;
   const bool uneven = a.window_left >= 0 || a.window_right >= 0 || a.cu_seqlens_q;

@@ -110,7 +110,7 @@ struct Fmt<__nv_bfloat16> {
 
 // GROUPED: tiles shared by heads and / or keys in a KV cache (the plain instance keeps its geometry as constants: read from
 // the parameters it took 436 us instead of 397 on 16 x 2048 x 16 x 128 causal)
-template <typename T, int DH, bool GROUPED>
+template <typename T, int DH, bool GROUPED, bool TRIM>
 __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ FwdTcParams P) {
   using C = Cfg<DH>;
   const FaFwdArgs& a = P.a;
@@ -197,11 +197,12 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
   // Cache: block whose V rows past the last key are zeroed in shared memory (their P is 0, but 0 * NaN is not)
   const int j_tail = cache && (si.sk % kBN) && (si.sk - 1) / kBN < J_hi && (si.sk - 1) / kBN >= J_lo ? (si.sk - 1) / kBN : -1;
 
+  const int nchunk = head_chunks<DH, TRIM>(a.head_dim);
   auto load_q = [&](int t) {
     if (!active[t] || hi[t] <= lo[t]) return;
-    mbar_expect_tx(bar_qfull(t), C::NCHUNK * 128 * pack * tile_pos);
+    mbar_expect_tx(bar_qfull(t), nchunk * 128 * pack * tile_pos);
     const int r0 = (int)si.q_row0 + m_base + t * tile_pos;
-    for (int c = 0; c < C::NCHUNK; ++c)
+    for (int c = 0; c < nchunk; ++c)
       tma_load_4d(sQ + t * C::TILE_BYTES + c * kChunkBytes, &P.tq, bar_qfull(t), c * 64, pack > 1 ? h : r0, pack > 1 ? r0 : h, (int)si.q_batch);
   };
   // Paged cache: the page of the block after the current one is looked up a block ahead, so that the producer does not
@@ -216,16 +217,16 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
     const uint32_t dst = sKV + slot * C::TILE_BYTES;
     if (GROUPED && a.block_table) {  // one lookup per load; rows past the last key are not loaded page by page
       const int n_box = min((min(kBN, si.sk - j * kBN) + P.kv_box - 1) / P.kv_box, kBN / P.kv_box);
-      mbar_expect_tx(bar_full(slot), n_box * P.kv_box * C::NCHUNK * 128);
+      mbar_expect_tx(bar_full(slot), n_box * P.kv_box * nchunk * 128);
       for (int i = 0; i < n_box; ++i) {
         const int key = j * kBN + i * P.kv_box;
         const int page = page_of(key);
-        for (int c = 0; c < C::NCHUNK; ++c)
+        for (int c = 0; c < nchunk; ++c)
           tma_load_4d(dst + c * kChunkBytes + i * P.kv_box * 128, tm, bar_full(slot), c * 64, key % a.page_block_size, hk, page);
       }
     } else {
-      mbar_expect_tx(bar_full(slot), C::TILE_BYTES);
-      for (int c = 0; c < C::NCHUNK; ++c)
+      mbar_expect_tx(bar_full(slot), nchunk * kChunkBytes);
+      for (int c = 0; c < nchunk; ++c)
         tma_load_4d(dst + c * kChunkBytes, tm, bar_full(slot), c * 64, (int)si.k_row0 + j * kBN, hk, (int)si.k_batch);
     }
   };
@@ -542,9 +543,10 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
       }
     } else if (warp == 9) {
       // ---------------------------------------------------------------- MMA issuer
-      {  // the whole warp runs the loop (see mma_ss_w); one elected lane issues
+      with_head_steps<DH, TRIM>(a.head_dim, [&](auto steps) {  // the whole warp runs the loop (see mma_ss_w); one elected lane issues
         constexpr uint32_t idesc_s = make_idesc(kBM, kBN, Fmt<T>::kIdesc, 0, 0);
-        constexpr uint32_t idesc_o = make_idesc(kBM, DH, Fmt<T>::kIdesc, 0, 1);
+        constexpr int KS = decltype(steps)::value;
+        constexpr uint32_t idesc_o = make_idesc(kBM, KS * 16, Fmt<T>::kIdesc, 0, 1);
         bool ok = true;
         int p_iter[2] = {0, 0};  // softmax iterations consumed per tile
         // One descriptor is built (Q tile 0, K-major); every other operand differs from it only in the
@@ -558,7 +560,7 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
           const uint32_t d = tmem + (t ? C::COL_S1 : C::COL_S0);
           const uint32_t a_lo = t ? kTile16 : 0u, b_lo = oKV + slot * kTile16;
 #pragma unroll
-          for (int kk = 0; kk < DH / 16; ++kk) {
+          for (int kk = 0; kk < KS; ++kk) {
             const uint32_t off = (uint32_t)(((kk >> 2) * kChunkBytes + (kk & 3) * 32) >> 4);
             mma_ss_w(d, dsc(a_lo + off), dsc(b_lo + off), idesc_s, kk > 0);
           }
@@ -623,7 +625,7 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
             }
           }
         }
-      }
+      });
     } else if (GROUPED && warp == 11 && j_tail >= 0) {
       // ---------------------------------------------------------------- zeroes the rows of the last V tile that hold no key
       // (The MMA warp says when: a wait of this warp's own on the slot's barrier would have to pass all its earlier phases.)
@@ -686,9 +688,11 @@ int launch_fwd_tc(const FaFwdArgs& a, int64_t kv_batches, cudaStream_t st) {
   P.status = status_ref(true);
   P.num_splits = a.num_splits > 1 ? a.num_splits : 1;
   const bool grouped = P.pack > 1 || P.cache;
-  auto kern = grouped ? fwd_tc_kernel<T, DH, true> : fwd_tc_kernel<T, DH, false>;
-  static fa_host::DeviceOnce once[2];
-  if (int rc = fa_host::raise_smem_limit(once[grouped], reinterpret_cast<const void*>(kern), C::SMEM_BYTES, "fwd_tc_kernel")) return rc;
+  const bool trim = head_trims<DH>(a.head_dim);
+  auto kern = trim ? (grouped ? fwd_tc_kernel<T, DH, true, true> : fwd_tc_kernel<T, DH, false, true>)
+                   : (grouped ? fwd_tc_kernel<T, DH, true, false> : fwd_tc_kernel<T, DH, false, false>);
+  static fa_host::DeviceOnce once[2][2];
+  if (int rc = fa_host::raise_smem_limit(once[trim][grouped], reinterpret_cast<const void*>(kern), C::SMEM_BYTES, "fwd_tc_kernel")) return rc;
   const int n_m = (a.seqlen_q + C::NT * P.tile_pos - 1) / (C::NT * P.tile_pos);
   dim3 grid(n_m * P.num_splits, a.heads / P.pack, a.batch);
   P.head_group = fa_host::cta_head_group(a.window_left >= 0 || a.window_right >= 0 || a.cu_seqlens_q, (int64_t)a.seqlen_k * a.head_dim * 4 / (a.heads / P.pack / a.heads_k),

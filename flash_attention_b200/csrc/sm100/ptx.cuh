@@ -6,6 +6,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 namespace fa {
 namespace ptx {
 
@@ -316,6 +318,44 @@ __host__ __device__ constexpr uint32_t make_idesc(int M, int N, int ab_format, i
          | ((uint32_t)b_mn_major << 16)      // B major
          | ((uint32_t)(N >> 3) << 17)        // N / 8
          | ((uint32_t)(M >> 4) << 24);       // M / 16
+}
+
+// Head dims between the kernels' own (64, 128, 256): the products take the 16-column k-steps and the result columns that hold
+// data, and the loads the 64-column chunks that do; what a tile holds behind them is not read.
+// 8 x 2048 tokens, full, forward / backward in us with the padding and without: 32 heads of 32 420 / 1000 -> 409 / 944, 25 of 80
+// 372 / 1153 -> 356 / 1026, 21 of 96 333 / 1022 -> 324 / 932, 12 of 160 448 / 1425 -> 382 / 1267, 10 of 192 369 / 1199 -> 333 / 1132.
+// f(integral_constant) is called with the number of k-steps, a constant, because the issuing warp is often what a product waits
+// for: with a test per MMA of a count read from the parameters head dims 64 and 128 took 1 to 4 % longer, 256 (backward) 20 %.
+// TRIM is an instance of the kernel of its own for the same reason (all in one: 128 1.4 %, 256 9 % longer).
+template <int DH, bool TRIM, typename F>
+__device__ __forceinline__ void with_head_steps(int head_dim, F&& f) {
+  if (!TRIM)
+    f(std::integral_constant<int, DH / 16>{});
+  else if (DH == 64 && head_dim <= 32)
+    f(std::integral_constant<int, 2>{});
+  else if (DH == 64 && head_dim <= 48)
+    f(std::integral_constant<int, 3>{});
+  else if (DH == 128 && head_dim <= 80)
+    f(std::integral_constant<int, 5>{});
+  else if (DH == 128 && head_dim <= 96)
+    f(std::integral_constant<int, 6>{});
+  else if (DH == 256 && head_dim <= 160)
+    f(std::integral_constant<int, 10>{});
+  else if (DH == 256 && head_dim <= 192)
+    f(std::integral_constant<int, 12>{});
+  else
+    f(std::integral_constant<int, DH / 16>{});
+}
+// chunks of a tile of DH columns (a tile of up to 128 columns is always loaded whole: its last chunk holds data)
+template <int DH, bool TRIM>
+__device__ __forceinline__ int head_chunks(int head_dim) {
+  return TRIM && DH > 128 ? (head_dim + 63) / 64 : DH / 64;
+}
+
+// whether with_head_steps has a smaller count than DH / 16 for this head dim
+template <int DH>
+constexpr bool head_trims(int head_dim) {
+  return head_dim <= DH * 3 / 4;
 }
 
 // ---- packed fp32 pairs (sm_100 has two-wide fp32 FMA/ADD and a three-input max) ------------------
