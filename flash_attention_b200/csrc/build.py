@@ -1,4 +1,5 @@
-"""Builds libfa_b200.so in-tree with nvcc for sm_100a (cross-compiles without a GPU).
+"""Builds libfa_b200.so in-tree with nvcc for sm_100a (cross-compiles without a GPU), and _torch_glue.so, which hands torch
+tensors to it, with g++.
 
 Usage: python -m flash_attention_b200.csrc.build [--force] [--verbose]
 The shared library lands next to this file; object files go to csrc/build/.
@@ -12,6 +13,8 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(os.path.dirname(HERE))
 OUT = os.path.join(HERE, "libfa_b200.so")
+GLUE_SRC = os.path.join(HERE, "torch_glue.cpp")
+GLUE_OUT = os.path.join(HERE, "_torch_glue.so")
 OBJ_DIR = os.path.join(HERE, "build")
 
 SOURCES = [
@@ -76,6 +79,33 @@ def _compile(src, verbose):
     return obj, r.stderr
 
 
+def _build_glue(force):
+    import sysconfig
+
+    import torch
+
+    where = os.path.dirname(torch.__file__)
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI,
+           "-I", os.path.join(ROOT, "include"), "-I", sysconfig.get_paths()["include"],
+           "-isystem", os.path.join(where, "include"), "-isystem", os.path.join(where, "include", "torch", "csrc", "api", "include"),
+           "-isystem", os.path.join(os.path.dirname(os.path.dirname(_nvcc())) or "/usr/local/cuda", "include"),
+           GLUE_SRC, "-o", GLUE_OUT, "-L", HERE, "-l:libfa_b200.so", "-Wl,-rpath,$ORIGIN",
+           "-L", os.path.join(where, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python"]
+    h = hashlib.sha1((torch.__version__ + " ".join(cmd)).encode())
+    for p in (GLUE_SRC, os.path.join(ROOT, "include", "fa_b200.h")):
+        with open(p, "rb") as f:
+            h.update(f.read())
+    stamp = os.path.join(OBJ_DIR, "torch_glue.sha1")
+    if not force and os.path.exists(GLUE_OUT) and os.path.exists(stamp) and open(stamp).read() == h.hexdigest():
+        return
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("g++ failed for torch_glue.cpp:\n%s\n%s" % (r.stdout, r.stderr))
+    with open(stamp, "w") as f:
+        f.write(h.hexdigest())
+
+
 def build(force=False, verbose=False):
     os.makedirs(OBJ_DIR, exist_ok=True)
     if force:
@@ -94,6 +124,7 @@ def build(force=False, verbose=False):
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError("link failed:\n%s\n%s" % (r.stdout, r.stderr))
+    _build_glue(force)
     return OUT
 
 

@@ -42,57 +42,54 @@ class _Attention(torch.autograd.Function):
     @staticmethod
     def forward(ctx, packing, seq, dropout_p, softmax_scale, causal, window_size, return_softmax, deterministic, *tensors):
         # seq is None for padded batches, else (cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k)
-        varlen = seq is not None
-        q, k, v = (_unit_stride(t) for t in _split(packing, tensors, varlen))
+        q, k, v = _split(packing, tensors, seq is not None)
+        q, k, v = _unit_stride(q), _unit_stride(k), _unit_stride(v)
         if softmax_scale is None:
             softmax_scale = q.shape[-1] ** (-0.5)
         want_probs = return_softmax and dropout_p > 0
-        if varlen:
+        if seq is not None:
             cu_q, cu_k, max_q, max_k = seq
             out, q, k, v, out_padded, lse, s_dmask, rng_state = _ext.varlen_fwd(
                 q, k, v, None, cu_q, cu_k, max_q, max_k, dropout_p, softmax_scale, False, causal,
                 window_size[0], window_size[1], want_probs, None)
-            ctx.save_for_backward(q, k, v, out_padded, lse, cu_q, cu_k, rng_state)
-            ctx.max_seqlens = (max_q, max_k)
+            ctx.save_for_backward(q, k, v, out_padded, lse, rng_state, cu_q, cu_k)
+            max_seqlens = (max_q, max_k)
         else:
             out, q, k, v, out_padded, lse, s_dmask, rng_state = _ext.fwd(
                 q, k, v, None, dropout_p, softmax_scale, causal, window_size[0], window_size[1], want_probs, None)
             ctx.save_for_backward(q, k, v, out_padded, lse, rng_state)
-        ctx.packing, ctx.varlen, ctx.deterministic = packing, varlen, bool(deterministic)
-        ctx.dropout_p, ctx.softmax_scale, ctx.causal, ctx.window_size = dropout_p, softmax_scale, causal, window_size
+            max_seqlens = None
+        ctx.call = (packing, max_seqlens, dropout_p, softmax_scale, causal, window_size, bool(deterministic))
         return out if not return_softmax else (out, lse, s_dmask)
 
     @staticmethod
     def backward(ctx, dout, *unused):
-        if ctx.varlen:
-            q, k, v, out, lse, cu_q, cu_k, rng_state = ctx.saved_tensors
-        else:
-            q, k, v, out, lse, rng_state = ctx.saved_tensors
-        ax = 1 if ctx.varlen else 2
-        lead_q, lead_k = q.shape[:-2], k.shape[:-2]
+        packing, max_seqlens, dropout_p, softmax_scale, causal, window_size, deterministic = ctx.call
+        q, k, v, out, lse, rng_state, *cu = ctx.saved_tensors
         # one packed gradient tensor per packed input; dq/dk/dv are views into it
-        if ctx.packing == "qkv":
-            dqkv = torch.empty(lead_q + (3,) + q.shape[-2:], dtype=q.dtype, device=q.device)
+        ax = 1 if cu else 2
+        if packing == "qkv":
+            dqkv = torch.empty(q.shape[:-2] + (3,) + q.shape[-2:], dtype=q.dtype, device=q.device)
             dq, dk, dv = (dqkv.select(ax, i) for i in range(3))
             grads = (dqkv,)
-        elif ctx.packing == "kv":
+        elif packing == "kv":
             dq = torch.empty_like(q)
-            dkv = torch.empty(lead_k + (2,) + k.shape[-2:], dtype=k.dtype, device=k.device)
+            dkv = torch.empty(k.shape[:-2] + (2,) + k.shape[-2:], dtype=k.dtype, device=k.device)
             dk, dv = dkv.select(ax, 0), dkv.select(ax, 1)
             grads = (dq, dkv)
         else:
             dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
             grads = (dq, dk, dv)
-        dout, q, k, v, out = (_unit_stride(t) for t in (dout, q, k, v, out))
-        if ctx.varlen:
-            _ext.varlen_bwd(dout, q, k, v, out, lse, dq, dk, dv, cu_q, cu_k, ctx.max_seqlens[0], ctx.max_seqlens[1],
-                            ctx.dropout_p, ctx.softmax_scale, False, ctx.causal, ctx.window_size[0],
-                            ctx.window_size[1], None, rng_state, deterministic=ctx.deterministic)
+        dout, q, k, v, out = _unit_stride(dout), _unit_stride(q), _unit_stride(k), _unit_stride(v), _unit_stride(out)
+        if cu:
+            _ext.varlen_bwd(dout, q, k, v, out, lse, dq, dk, dv, cu[0], cu[1], max_seqlens[0], max_seqlens[1], dropout_p, softmax_scale,
+                            False, causal, window_size[0], window_size[1], None, rng_state, deterministic=deterministic)
         else:
-            _ext.bwd(dout, q, k, v, out, lse, dq, dk, dv, ctx.dropout_p, ctx.softmax_scale, ctx.causal,
-                     ctx.window_size[0], ctx.window_size[1], None, rng_state, deterministic=ctx.deterministic)
-        d = dout.shape[-1]  # the head dim may have been padded to a multiple of 8
-        grads = tuple(g[..., :d] for g in grads)
+            _ext.bwd(dout, q, k, v, out, lse, dq, dk, dv, dropout_p, softmax_scale, causal, window_size[0], window_size[1], None, rng_state,
+                     deterministic=deterministic)
+        d = dout.shape[-1]
+        if d != q.shape[-1]:  # the head dim was padded to a multiple of 8
+            grads = tuple(g[..., :d] for g in grads)
         return (None,) * 8 + grads
 
 

@@ -6,7 +6,8 @@ The reference's `flash_attn/flash_attn_interface.py` does `import flash_attn_2_c
 argument order, return lists, checks and error type (RuntimeError) of csrc/flash_attn/flash_api.cpp,
 on top of libfa_b200.so (hand-written sm_100a kernels, C ABI in include/fa_b200.h).  What the
 reference does with ATen in C++ — padding the head dim to a multiple of 8, allocating outputs and
-workspaces, RNG bookkeeping, the seqlen_q==1 grouped-query reshape — is done here with torch.
+workspaces, RNG bookkeeping, the seqlen_q==1 grouped-query reshape — is done here with torch; calls that need none of it but
+the allocations go through flash_attention_b200/csrc/torch_glue.cpp, which does the same natively (`_glue`).
 
 There is no fallback path: every function ends in a call into the CUDA library.
 """
@@ -18,6 +19,23 @@ import torch.nn.functional as F
 
 from flash_attention_b200 import _lib
 from flash_attention_b200._lib import FaBwdArgs, FaFwdArgs, FaKvcacheArgs, check, lib, ptr, tensor3
+
+
+
+class _GlueAtFirstUse:  # (the package must import before it is built)
+    def __getattr__(self, name):
+        global _glue
+        lib()
+        try:
+            from flash_attention_b200.csrc import _torch_glue
+        except ImportError as e:
+            raise ImportError("%s: build it with `python -m flash_attention_b200.csrc.build`; there is no fallback" % e) from e
+        _glue = _torch_glue
+        return getattr(_glue, name)
+
+
+_glue = _GlueAtFirstUse()
+
 
 __all__ = ["fwd", "varlen_fwd", "bwd", "varlen_bwd", "fwd_kvcache"]
 
@@ -152,6 +170,10 @@ def fwd(q, k, v, out_, p_dropout, softmax_scale, is_causal, window_size_left, wi
     q: (batch, seqlen_q, heads, d); k, v: (batch, seqlen_k, heads_k, d).
     Returns [out, q_padded, k_padded, v_padded, out_padded, softmax_lse, p, rng_state].
     """
+    if out_ is None and p_dropout == 0.0 and not return_softmax:
+        r = _glue.fwd(q, k, v, None, None, 0, 0, float(softmax_scale), bool(is_causal), int(window_size_left), int(window_size_right))
+        if r is not None:
+            return r
     dt = _dtype_code(q)
     _require(k.dtype == q.dtype, "query and key must have the same dtype")
     _require(v.dtype == q.dtype, "query and value must have the same dtype")
@@ -247,6 +269,11 @@ def varlen_fwd(q, k, v, out_, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seql
 
     q: (total_q, heads, d); k, v: (total_k, heads_k, d); cu_seqlens_*: (batch + 1) int32.
     """
+    if out_ is None and p_dropout == 0.0 and not return_softmax and not zero_tensors:
+        r = _glue.fwd(q, k, v, cu_seqlens_q, cu_seqlens_k, int(max_seqlen_q), int(max_seqlen_k), float(softmax_scale), bool(is_causal),
+                      int(window_size_left), int(window_size_right))
+        if r is not None:
+            return r
     dt = _dtype_code(q)
     _require(k.dtype == q.dtype, "query and key must have the same dtype")
     _require(v.dtype == q.dtype, "query and value must have the same dtype")
@@ -334,6 +361,11 @@ def _grad_out(given, shape, like, name):
 
 def _bwd_common(varlen, dout, q, k, v, out, softmax_lse, dq_, dk_, dv_, cu_q, cu_k, max_q, max_k, p_dropout,
                 softmax_scale, is_causal, wl_in, wr_in, rng_state, what, deterministic=False):
+    if p_dropout == 0.0:
+        r = _glue.bwd(dout, q, k, v, out, softmax_lse, dq_, dk_, dv_, cu_q, cu_k, int(max_q), int(max_k), float(softmax_scale),
+                      bool(is_causal), int(wl_in), int(wr_in), bool(deterministic))
+        if r is not None:
+            return r
     dt = _dtype_code(q)
     _require(k.dtype == q.dtype, "query and key must have the same dtype")
     _require(v.dtype == q.dtype, "query and value must have the same dtype")
@@ -456,6 +488,12 @@ def fwd_kvcache(q, kcache, vcache, k_, v_, seqlens_k_, rotary_cos_, rotary_sin_,
     (batch, pages_per_sequence) int32.  kcache / vcache are then pools (num_pages, page_block_size, heads_k, d);
     key j of sequence b is row j % page_block_size of page block_table[b, j // page_block_size].
     """
+    if out_ is None:
+        r = _glue.fwd_kvcache(q, kcache, vcache, k_, v_, seqlens_k_, rotary_cos_, rotary_sin_, cache_batch_idx_, float(softmax_scale),
+                              bool(is_causal), int(window_size_left), int(window_size_right), bool(is_rotary_interleaved), int(num_splits),
+                              block_table)
+        if r is not None:
+            return r
     dt = _dtype_code(q)
     _require(kcache.dtype == q.dtype, "query and key must have the same dtype")
     _require(vcache.dtype == q.dtype, "query and value must have the same dtype")
