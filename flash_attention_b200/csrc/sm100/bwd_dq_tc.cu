@@ -72,7 +72,8 @@ struct DqTcParams {
   CUtensorMap tq, tk, tv, tdo;
   FaBwdArgs a;
   StatusRef status;
-  int32_t head_group;
+  CtaOrder order;
+  FastDiv group;  // query heads per KV head
 };
 
 template <typename T>
@@ -117,9 +118,9 @@ __global__ void __launch_bounds__(kThreads, QCfg<DH, KN>::CTAS) bwd_dq_tc_kernel
     prefetch_tensormap(&P.tdo);
     prefetch_tensormap(&P.tv);
   }
-  const CtaItem item = UNEVEN ? cta_item(P.head_group) : CtaItem{(int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z};
+  const CtaItem item = UNEVEN ? cta_item(P.order) : CtaItem{(int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z};
   const int hq = item.head, b = item.batch;
-  const int hk = hq / (a.heads / a.heads_k);
+  const int hk = (int)P.group.div(hq);
   const SeqInfo si = seq_info(a.cu_seqlens_q, a.cu_seqlens_k, nullptr, nullptr, a.seqlen_q, a.seqlen_k,
                               a.use_mask_shift, a.mask_shift, b);
   // heavy query blocks (bottom rows of a causal mask see the most keys) are scheduled first
@@ -459,8 +460,10 @@ int launch_bwd_dq_tc(const FaBwdArgs& a, cudaStream_t st) {
   if (int rc = fa_host::raise_smem_limit(once[trim][uneven], reinterpret_cast<const void*>(kern), C::SMEM_BYTES, "bwd_dq_tc_kernel")) return rc;
   const int rows = a.d_seqlen > a.seqlen_q ? a.d_seqlen : a.seqlen_q;  // the padding rows of D are written too
   dim3 grid((rows + kM - 1) / kM, a.heads, a.batch);
-  P.head_group = fa_host::cta_head_group(uneven, (int64_t)a.seqlen_k * a.head_dim * 4 / (a.heads / a.heads_k),
+  P.group = fast_div(a.heads / a.heads_k);
+  const int head_group = fa_host::cta_head_group(uneven, (int64_t)a.seqlen_k * a.head_dim * 4 / (a.heads / a.heads_k),
                                          (int64_t)a.heads * a.batch);
+  P.order = cta_order(head_group, grid);
   kern<<<grid, kThreads, C::SMEM_BYTES, st>>>(P);
   return fa_host::check_launch("bwd_dq_tc_kernel");
 }

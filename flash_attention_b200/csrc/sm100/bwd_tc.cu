@@ -87,7 +87,8 @@ struct BwdTcParams {
   CUtensorMap tq, tk, tv, tdo;
   FaBwdArgs a;
   StatusRef status;
-  int32_t head_group;
+  CtaOrder order;
+  FastDiv group;  // query heads per KV head
 };
 
 template <typename T>
@@ -136,9 +137,9 @@ __global__ void __launch_bounds__(BCfg<DH, BQ>::THREADS, BCfg<DH, BQ>::CTAS) bwd
     prefetch_tensormap(&P.tdo);
     prefetch_tensormap(&P.tv);
   }
-  const CtaItem item = UNEVEN ? cta_item(P.head_group) : CtaItem{(int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z};
+  const CtaItem item = UNEVEN ? cta_item(P.order) : CtaItem{(int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z};
   const int nblk = item.block, hk = item.head, b = item.batch;
-  const int group = a.heads / a.heads_k;
+  const int group = (int)P.group.d;
   const SeqInfo si = seq_info(a.cu_seqlens_q, a.cu_seqlens_k, nullptr, nullptr, a.seqlen_q, a.seqlen_k,
                               a.use_mask_shift, a.mask_shift, b);
   const int n0 = nblk * kB;
@@ -555,8 +556,10 @@ int launch_bwd_tc(const FaBwdArgs& a, cudaStream_t st) {
   static fa_host::DeviceOnce once[2][2];
   if (int rc = fa_host::raise_smem_limit(once[trim][uneven], reinterpret_cast<const void*>(kern), C::SMEM_BYTES, "bwd_tc_kernel")) return rc;
   dim3 grid((a.seqlen_k + kB - 1) / kB, a.heads_k, a.batch);
-  P.head_group = fa_host::cta_head_group(uneven, (int64_t)a.seqlen_q * (a.heads / a.heads_k) * a.head_dim * 4,
+  P.group = fast_div(a.heads / a.heads_k);
+  const int head_group = fa_host::cta_head_group(uneven, (int64_t)a.seqlen_q * (a.heads / a.heads_k) * a.head_dim * 4,
                                          (int64_t)a.heads_k * a.batch);
+  P.order = cta_order(head_group, grid);
   kern<<<grid, C::THREADS, C::SMEM_BYTES, st>>>(P);
   return fa_host::check_launch("bwd_tc_kernel");
 }

@@ -69,7 +69,8 @@ struct WParams {
   CUtensorMap ta1, ta2, tb1, tb2;  // stationary tiles (128-row boxes), streamed tiles (64-row boxes)
   FaBwdArgs a;
   StatusRef status;
-  int32_t head_group;
+  CtaOrder order;
+  FastDiv group;  // query heads per KV head
 };
 
 template <typename T>
@@ -123,16 +124,16 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_wide_tc_kernel(const __grid_c
     prefetch_tensormap(&P.tb1);
     prefetch_tensormap(&P.tb2);
   }
-  const CtaItem item = cta_item(P.head_group);
+  const CtaItem item = cta_item(P.order);
   const int b = item.batch;
-  const int group = a.heads / a.heads_k;
+  const int group = (int)P.group.d;
   const SeqInfo si = seq_info(a.cu_seqlens_q, a.cu_seqlens_k, nullptr, nullptr, a.seqlen_q, a.seqlen_k,
                               a.use_mask_shift, a.mask_shift, b);
   // r0: first stationary row; [c_lo_blk, c_hi_blk): streamed 64-row blocks these rows can see
   int r0, blk_lo, blk_hi, iters, hq_fixed, hk;
   if (kRowsAreQueries) {
     hq_fixed = item.head;
-    hk = hq_fixed / group;
+    hk = (int)P.group.div(hq_fixed);
     r0 = ((int)gridDim.x - 1 - item.block) * kR;  // heavy query blocks of a causal mask first
     if (r0 >= si.sq) return;
     key_block_range(r0, kR, kN, si.sk, si.shift, a.window_left, a.window_right, blk_lo, blk_hi);
@@ -578,8 +579,10 @@ int launch_wide(const FaBwdArgs& a, cudaStream_t st) {
   dim3 grid(((PASS == PASS_DQ ? a.seqlen_q : a.seqlen_k) + kR - 1) / kR, PASS == PASS_DQ ? a.heads : a.heads_k, a.batch);
   const int group = a.heads / a.heads_k;
   const bool uneven = a.window_left >= 0 || a.window_right >= 0 || a.cu_seqlens_q;
-  P.head_group = PASS == PASS_DQ ? fa_host::cta_head_group(uneven, (int64_t)a.seqlen_k * a.head_dim * 4 / group, (int64_t)a.heads * a.batch)
+  P.group = fast_div(group);
+  const int head_group = PASS == PASS_DQ ? fa_host::cta_head_group(uneven, (int64_t)a.seqlen_k * a.head_dim * 4 / group, (int64_t)a.heads * a.batch)
                                  : fa_host::cta_head_group(uneven, (int64_t)a.seqlen_q * group * a.head_dim * 4, (int64_t)a.heads_k * a.batch);
+  P.order = cta_order(head_group, grid);
   kern<<<grid, kThreads, C::SMEM_BYTES, st>>>(P);
   return fa_host::check_launch("bwd_wide_tc_kernel");
 }
