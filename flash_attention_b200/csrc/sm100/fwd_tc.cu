@@ -1,17 +1,19 @@
 // Forward attention on the 5th-generation tensor cores (tcgen05 + TMEM + TMA), head dim <= 256.
 //
 // One CTA owns 256 query rows of one (batch, head) [and, with split-KV, one range of key blocks]: two
-// 128-row tiles that take turns on the tensor pipe (head dims above 128: one tile, because O alone
-// fills 256 TMEM columns; warps 4-7 idle).  CTAs are launched heaviest first (bottom rows of a causal
-// mask see the most keys).
-// Warp roles (384 threads):
+// 128-row tiles that take turns on the tensor pipe.  Or it owns one tile: two such CTAs share an SM where a tile has few key
+// blocks (one_tile), and one has it alone at head dims above 128, where O alone fills 256 TMEM columns.  CTAs are launched heaviest
+// first (bottom rows of a causal mask see the most keys).
+// Warp roles (384 threads; one tile: 256, without the second four):
 //   warps 0-3   softmax of tile 0  (one thread per query row; tcgen05.ld 32x32b gives a thread its row)
 //   warps 4-7   softmax of tile 1
-//   warp  8     TMA producer: Q tiles once, then K(j), V(j), K(j+1), ... through a ring of slots
-//   warp  9     MMA issuer: the warp stays converged, one elected lane issues every tcgen05.mma
-//   warp  10    owns the TMEM allocation
-//   warp  11    KV cache: clears the rows of the last V tile that hold no key
-// Registers: 168 a thread at launch, 4 to 8 bytes spilled.
+//   then        TMA producer: Q tiles once, then K(j), V(j), K(j+1), ... through a ring of slots
+//               MMA issuer: the warp stays converged, one elected lane issues every tcgen05.mma
+//               owner of the TMEM allocation
+//               KV cache: clears the rows of the last V tile that hold no key
+// V(j) and K(j+1) arrive on one barrier: a wait of the issuing warp costs 130 to 200 cycles even when there is nothing to wait for
+// (16 x 2048 x 16 x 128 causal 328 -> 325 us, 32 x 512 97.0 -> 95.5).
+// Registers: 168 (two CTAs per SM: 128) a thread at launch, 4 to 8 bytes spilled.
 // With grouped-query heads a tile's 128 rows are (positions x heads of the group), so that both tiles of a CTA end at the same
 // key block of a causal mask and a few tokens per sequence fill a tile (prefill of 4096 tokens, 32/8 heads: 179 -> 157 us, and
 // 137 with the CTA order of cta_item).  K and V may be a KV cache: lengths on the device, batch index, pages of 64 rows and up.
@@ -69,19 +71,26 @@ constexpr float kRescaleThreshold = 8.f;
 
 enum WaitCode { W_QFULL = 11, W_KVFULL = 12, W_KVEMPTY = 13, W_SFULL = 14, W_PFULL = 15, W_OFULL = 16, W_VTAIL = 17 };
 
-template <int DH>
+// NT: query tiles per CTA
+template <int DH, int NT>
 struct Cfg {
   static constexpr int NCHUNK = DH / 64;
   static constexpr int TILE_BYTES = NCHUNK * kChunkBytes;
-  // Head dims up to 128: two 128-row query tiles per CTA ping-pong on the tensor pipe.  Up to 256: O alone
-  // needs 256 TMEM columns and a tile is 64 KiB, so one query tile per CTA and a 2-slot (K, V) ring.
-  static constexpr int NT = DH > 128 ? 1 : 2;
-  static constexpr int STAGES = DH > 128 ? 2 : (DH == 128 ? 4 : 8);
+  // Head dims up to 128: one 128-row query tile and two CTAs per SM, or two tiles that ping-pong on the tensor pipe and share K
+  // and V.  Up to 256: O alone needs 256 TMEM columns and a tile is 64 KiB, so one tile and one CTA per SM, with a 2-slot (K, V) ring.
+  static constexpr int CTAS = NT == 1 && DH <= 128 ? 2 : 1;
+  static constexpr int WARP_PRODUCER = 4 * NT, WARP_MMA = 4 * NT + 1, WARP_TMEM = 4 * NT + 2, WARP_TAIL = 4 * NT + 3;
+  static constexpr int THREADS = 32 * (4 * NT + 4);
+  // a thread is launched with 128 (two CTAs), 168 or 255 registers: setmaxnreg only redistributes those
+  static constexpr int REGS = CTAS == 2 ? 200 : 216, REGS_OTHER = CTAS == 2 ? 56 : 64, REGS_LAUNCH = CTAS == 2 ? 128 : NT == 2 ? 168 : 255;
+  static_assert(128 * NT * REGS + 128 * REGS_OTHER <= THREADS * REGS_LAUNCH, "the registers of one CTA");
+  static constexpr int STAGES = DH == 64 ? (CTAS == 2 ? 4 : 8) : DH == 128 ? (CTAS == 2 ? 2 : 4) : 2;
   static constexpr int SMEM_TILES = (NT + STAGES) * TILE_BYTES;
   static constexpr int NBAR = 2 + 2 * STAGES + 10;
   static constexpr int SMEM_BYTES = SMEM_TILES + NBAR * 8 + 32 + 1024;  // + barriers, tmem ptr / abort block, align slack
-  static constexpr int TMEM_COLS = 512;
-  static constexpr int COL_S0 = 0, COL_S1 = 128, COL_O0 = 256, COL_O1 = 256 + DH;
+  static constexpr int TMEM_COLS = CTAS == 2 ? 256 : 512;
+  static constexpr int COL_S0 = 0, COL_S1 = 128, COL_O0 = CTAS == 2 ? 128 : 256, COL_O1 = COL_O0 + DH;
+  static_assert(CTAS * (SMEM_BYTES + 1024) <= 228 * 1024 && COL_O0 + NT * DH <= TMEM_COLS, "what the CTAs of an SM share");
 };
 
 struct FwdTcParams {
@@ -112,15 +121,15 @@ struct Fmt<__nv_bfloat16> {
 
 // GROUPED: tiles shared by heads and / or keys in a KV cache (the plain instance keeps its geometry as constants: read from
 // the parameters it took 436 us instead of 397 on 16 x 2048 x 16 x 128 causal)
-template <typename T, int DH, bool GROUPED, bool TRIM>
-__global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ FwdTcParams P) {
-  using C = Cfg<DH>;
+template <typename T, int DH, int NT, bool GROUPED, bool TRIM>
+__global__ void __launch_bounds__(Cfg<DH, NT>::THREADS, Cfg<DH, NT>::CTAS) fwd_tc_kernel(const __grid_constant__ FwdTcParams P) {
+  using C = Cfg<DH, NT>;
   const FaFwdArgs& a = P.a;
   extern __shared__ unsigned char smem_unaligned[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~uintptr_t(1023));
   const uint32_t s_base = smem_addr(smem);
   const uint32_t sQ = s_base;                          // NT tiles
-  const uint32_t sKV = s_base + C::NT * C::TILE_BYTES;  // STAGES slots
+  const uint32_t sKV = s_base + NT * C::TILE_BYTES;  // STAGES slots
   const uint32_t bar0 = s_base + C::SMEM_TILES;
   auto bar_qfull = [&](int t) { return bar0 + 8 * t; };
   auto bar_full = [&](int s) { return bar0 + 8 * (2 + s); };
@@ -134,7 +143,7 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + C::SMEM_TILES + C::NBAR * 8 + 4);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (threadIdx.x == 8 * 32) {  // the TMA unit fetches the three descriptors while the CTA sets itself up
+  if (threadIdx.x == C::WARP_PRODUCER * 32) {  // the TMA unit fetches the three descriptors while the CTA sets itself up
     prefetch_tensormap(&P.tq);
     prefetch_tensormap(&P.tk);
     prefetch_tensormap(&P.tv);
@@ -153,7 +162,7 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
                     : P.num_splits > 1    ? __shfl_sync(0xffffffffu, (int)P.splits.div(item.block), 0)
                                           : item.block;
   const int split = item.block - mrank * P.num_splits, mblk = P.row_blocks - 1 - mrank;
-  const int m_base = mblk * C::NT * tile_pos;
+  const int m_base = mblk * NT * tile_pos;
   if (m_base >= si.sq) return;  // uniform for the CTA
 
   // per-tile key block ranges
@@ -164,7 +173,7 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
     // tensor memory (32 sequences of 124 tokens in caches of 16384, 8/2 heads of 128, 5 parts: 17.9 -> 15.5 us).  Not in the
     // plain instance, whose lengths the host knows: it took 843 us instead of 836 on 16 x 2048, 32 heads of 64.
 #pragma unroll 1
-    for (int i = threadIdx.x; i < C::NT * kBM; i += 384) {
+    for (int i = threadIdx.x; i < NT * kBM; i += C::THREADS) {
       const int t = i / kBM, r = i % kBM, rp = (r * pack_inv) >> 16, row = m_base + t * tile_pos + rp;
       if (rp < tile_pos && row < si.sq)
         a.lse_accum[((int64_t)split * a.batch * a.heads + (int64_t)b * a.heads + h + r - rp * pack) * a.seqlen_q + row] = -INFINITY;
@@ -176,7 +185,7 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
 #pragma unroll
   for (int t = 0; t < 2; ++t) {
     const int m0 = m_base + t * tile_pos;
-    active[t] = t < C::NT && m0 < si.sq;
+    active[t] = t < NT && m0 < si.sq;
     if (active[t]) {
       key_block_range(m0, tile_pos, kBN, si.sk, si.shift, a.window_left, a.window_right, lo[t], hi[t]);
       if (P.num_splits > 1) {
@@ -217,23 +226,25 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
   auto page_at = [&](int key) { return a.block_table[(int64_t)b * a.block_table_stride + P.page.div(key)]; };
   auto page_of = [&](int key) { return key == page_key ? page_id : page_at(key); };
   // ring item idx: K of block J_lo + idx / 2 (idx even) or V (odd)
+  // V(j) and K(j + 1), which the MMA warp needs at the same time, arrive on one barrier, that of V's slot.
   auto load_kv = [&](int idx) {
     const int slot = idx % C::STAGES, j = J_lo + (idx >> 1);
+    const uint32_t bar = bar_full(idx > 0 && !(idx & 1) ? (idx - 1) % C::STAGES : slot);
     const CUtensorMap* tm = (idx & 1) ? &P.tv : &P.tk;
     const uint32_t dst = sKV + slot * C::TILE_BYTES;
     if (GROUPED && a.block_table) {  // one lookup per load; rows past the last key are not loaded page by page
       const int n_box = min((min(kBN, si.sk - j * kBN) + P.kv_box - 1) / P.kv_box, kBN / P.kv_box);
-      mbar_expect_tx(bar_full(slot), n_box * P.kv_box * nchunk * 128);
+      mbar_expect_tx(bar, n_box * P.kv_box * nchunk * 128);
       for (int i = 0; i < n_box; ++i) {
         const int key = j * kBN + i * P.kv_box;
         const int page = page_of(key);
         for (int c = 0; c < nchunk; ++c)
-          tma_load_4d(dst + c * kChunkBytes + i * P.kv_box * 128, tm, bar_full(slot), c * 64, key - (int)(P.page.div(key) * P.page.d), hk, page);
+          tma_load_4d(dst + c * kChunkBytes + i * P.kv_box * 128, tm, bar, c * 64, key - (int)(P.page.div(key) * P.page.d), hk, page);
       }
     } else {
-      mbar_expect_tx(bar_full(slot), nchunk * kChunkBytes);
+      mbar_expect_tx(bar, nchunk * kChunkBytes);
       for (int c = 0; c < nchunk; ++c)
-        tma_load_4d(dst + c * kChunkBytes, tm, bar_full(slot), c * 64, (int)si.k_row0 + j * kBN, hk, (int)si.k_batch);
+        tma_load_4d(dst + c * kChunkBytes, tm, bar, c * 64, (int)si.k_row0 + j * kBN, hk, (int)si.k_batch);
     }
   };
 
@@ -247,7 +258,7 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
       mbar_init(bar_ofull(t), 1);
     }
     for (int s = 0; s < C::STAGES; ++s) {
-      mbar_init(bar_full(s), 1);
+      mbar_init(bar_full(s), s & 1 ? 2 : 1);
       mbar_init(bar_empty(s), 1);
     }
     mbar_init(bar_vtail, 1);
@@ -259,11 +270,12 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
       // what S of the first tile needs goes first
       load_q(0);
       load_kv(0);
-      if (C::NT > 1) load_q(1);
+      if (NT > 1) load_q(1);
       load_kv(1);
+      if (nblk == 1) mbar_arrive(bar_full(1));  // no K behind the last V
     }
   }
-  if (warp == 10) {
+  if (warp == C::WARP_TMEM) {
     tmem_alloc(smem_addr(const_cast<uint32_t*>(tmem_ptr_smem)), C::TMEM_COLS);
     tmem_relinquish();
   }
@@ -274,10 +286,10 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
 
   const float scale_log2 = a.softmax_scale * kLog2e;
 
-  if (warp < 8) {
+  if (warp < 4 * NT) {
     // ------------------------------------------------------------------ softmax warpgroups
-    setmaxnreg_inc<216>();
-    const int t = warp >> 2;
+    if (C::REGS_LAUNCH < C::REGS) setmaxnreg_inc<C::REGS>();
+    const int t = NT > 1 ? warp >> 2 : 0;
     const int lo_t = t ? lo[1] : lo[0], hi_t = t ? hi[1] : hi[0];  // (indexing by t would put the arrays into local memory)
     const bool active_t = t ? active[1] : active[0];
     const int row_in_tile = (warp & 3) * 32 + lane;
@@ -532,8 +544,8 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
       }
     }
   } else {
-    setmaxnreg_dec<64>();
-    if (warp == 8) {
+    if (C::REGS_LAUNCH < C::REGS) setmaxnreg_dec<C::REGS_OTHER>();
+    if (warp == C::WARP_PRODUCER) {
       // ---------------------------------------------------------------- TMA producer
       if (lane == 0) {
         bool ok = true;
@@ -545,9 +557,10 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
           }
           ok = mbar_wait(bar_empty(slot), (round & 1) ^ 1, W_KVEMPTY, abort_flag);
           if (ok) load_kv(idx);
+          if (idx == 2 * nblk - 1) mbar_arrive(bar_full(slot));  // no K behind the last V
         }
       }
-    } else if (warp == 9) {
+    } else if (warp == C::WARP_MMA) {
       // ---------------------------------------------------------------- MMA issuer
       with_head_steps<DH, TRIM>(a.head_dim, [&](auto steps) {  // the whole warp runs the loop (see mma_ss_w); one elected lane issues
         constexpr uint32_t idesc_s = make_idesc(kBM, kBN, Fmt<T>::kIdesc, 0, 0);
@@ -561,7 +574,7 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
         const uint32_t d_lo = (uint32_t)d_base, d_hi = (uint32_t)(d_base >> 32);
         auto dsc = [&](uint32_t lo_add) { return ((uint64_t)d_hi << 32) | (uint64_t)(d_lo + lo_add); };
         constexpr uint32_t kMn = (uint32_t)((kChunkBytes - 16) >> 4) << 16;  // K-major -> MN-major (LBO = chunk stride)
-        constexpr uint32_t kTile16 = C::TILE_BYTES >> 4, oKV = (C::NT * C::TILE_BYTES) >> 4;
+        constexpr uint32_t kTile16 = C::TILE_BYTES >> 4, oKV = (NT * C::TILE_BYTES) >> 4;
         auto issue_s = [&](int t, int slot) {
           const uint32_t d = tmem + (t ? C::COL_S1 : C::COL_S0);
           const uint32_t a_lo = t ? kTile16 : 0u, b_lo = oKV + slot * kTile16;
@@ -592,7 +605,7 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
         if (nblk > 0) {
           // prologue: S_t(J_lo)
           ok = mbar_wait_w(bar_full(slot_of(0)), par_of(0), W_KVFULL, abort_flag);
-          for (int t = 0; t < C::NT && ok; ++t) {
+          for (int t = 0; t < NT && ok; ++t) {
             if (hi[t] > lo[t]) ok = mbar_wait_w(bar_qfull(t), 0, W_QFULL, abort_flag);
             if (!ok) break;
             tc_fence_after();
@@ -603,15 +616,14 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
             const int iv = 2 * (j - J_lo) + 1;  // ring index of V(j)
             const int ik = iv + 1;              // ring index of K(j+1)
             const bool more = j + 1 < J_hi;
-            ok = mbar_wait_w(bar_full(slot_of(iv)), par_of(iv), W_KVFULL, abort_flag);
-            if (ok && more) ok = mbar_wait_w(bar_full(slot_of(ik)), par_of(ik), W_KVFULL, abort_flag);
+            ok = mbar_wait_w(bar_full(slot_of(iv)), par_of(iv), W_KVFULL, abort_flag);  // and K(j+1)
             if (GROUPED && ok && j == j_tail) {  // V has landed: warp 11 clears its rows behind the last key
               if (lane == 0) mbar_arrive(bar_vtail_go);
               ok = mbar_wait_w(bar_vtail, 0, W_VTAIL, abort_flag);
             }
             if (!ok) break;
 #pragma unroll
-            for (int t = 0; t < C::NT; ++t) {
+            for (int t = 0; t < NT; ++t) {
               if (!ok) break;
               if (in_range(t, j)) {
                 const uint32_t par = (uint32_t)(p_iter[t] & 1);
@@ -625,20 +637,20 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
                 issue_pv_half(t, slot_of(iv), j == lo[t], 1);
                 ++p_iter[t];
               }
-              if (t == C::NT - 1) tc_commit_w(bar_empty(slot_of(iv)));
+              if (t == NT - 1) tc_commit_w(bar_empty(slot_of(iv)));
               if (more && in_range(t, j + 1)) issue_s(t, slot_of(ik));
-              if (more && t == C::NT - 1) tc_commit_w(bar_empty(slot_of(ik)));
+              if (more && t == NT - 1) tc_commit_w(bar_empty(slot_of(ik)));
             }
           }
         }
       });
-    } else if (GROUPED && warp == 11 && j_tail >= 0) {
+    } else if (GROUPED && warp == C::WARP_TAIL && j_tail >= 0) {
       // ---------------------------------------------------------------- zeroes the rows of the last V tile that hold no key
       // (The MMA warp says when: a wait of this warp's own on the slot's barrier would have to pass all its earlier phases.)
       const int iv = 2 * (j_tail - J_lo) + 1, slot = iv % C::STAGES;
       if (mbar_wait_w(bar_vtail_go, 0, W_VTAIL, abort_flag)) {
         const int first = si.sk - j_tail * kBN;
-        unsigned char* v = smem + (C::NT + slot) * C::TILE_BYTES + first * 128;
+        unsigned char* v = smem + (NT + slot) * C::TILE_BYTES + first * 128;
         for (int i = lane; i < (kBN - first) * 8; i += 32)
 #pragma unroll
           for (int c = 0; c < C::NCHUNK; ++c) *reinterpret_cast<uint4*>(v + c * kChunkBytes + i * 16) = make_uint4(0, 0, 0, 0);
@@ -660,7 +672,7 @@ __global__ void __launch_bounds__(384, 1) fwd_tc_kernel(const __grid_constant__ 
     }
     __syncthreads();
   }
-  if (warp == 10) tmem_dealloc(tmem, C::TMEM_COLS);
+  if (warp == C::WARP_TMEM) tmem_dealloc(tmem, C::TMEM_COLS);
 }
 
 // Heads of a KV head's group that share a query tile: the largest divisor of the group that leaves at least 120 of the
@@ -672,9 +684,9 @@ int pack_heads(int group) {
   return 1;
 }
 
-template <typename T, int DH>
+template <typename T, int DH, int NT>
 int launch_fwd_tc(const FaFwdArgs& a, int64_t kv_batches, cudaStream_t st) {
-  using C = Cfg<DH>;
+  using C = Cfg<DH, NT>;
   FwdTcParams P;
   P.a = a;
   const bool varlen = a.cu_seqlens_q != nullptr;
@@ -695,11 +707,11 @@ int launch_fwd_tc(const FaFwdArgs& a, int64_t kv_batches, cudaStream_t st) {
   P.num_splits = a.num_splits > 1 ? a.num_splits : 1;
   const bool grouped = P.pack > 1 || P.cache;
   const bool trim = head_trims<DH>(a.head_dim);
-  auto kern = trim ? (grouped ? fwd_tc_kernel<T, DH, true, true> : fwd_tc_kernel<T, DH, false, true>)
-                   : (grouped ? fwd_tc_kernel<T, DH, true, false> : fwd_tc_kernel<T, DH, false, false>);
+  auto kern = trim ? (grouped ? fwd_tc_kernel<T, DH, NT, true, true> : fwd_tc_kernel<T, DH, NT, false, true>)
+                   : (grouped ? fwd_tc_kernel<T, DH, NT, true, false> : fwd_tc_kernel<T, DH, NT, false, false>);
   static fa_host::DeviceOnce once[2][2];
   if (int rc = fa_host::raise_smem_limit(once[trim][grouped], reinterpret_cast<const void*>(kern), C::SMEM_BYTES, "fwd_tc_kernel")) return rc;
-  const int n_m = (a.seqlen_q + C::NT * P.tile_pos - 1) / (C::NT * P.tile_pos);
+  const int n_m = (a.seqlen_q + NT * P.tile_pos - 1) / (NT * P.tile_pos);
   dim3 grid(n_m * P.num_splits, a.heads / P.pack, a.batch);
   P.splits = fast_div(P.num_splits);
   P.group = fast_div(a.heads / a.heads_k);
@@ -708,7 +720,7 @@ int launch_fwd_tc(const FaFwdArgs& a, int64_t kv_batches, cudaStream_t st) {
   const int head_group = fa_host::cta_head_group(a.window_left >= 0 || a.window_right >= 0 || a.cu_seqlens_q, (int64_t)a.seqlen_k * a.head_dim * 4 / (a.heads / P.pack / a.heads_k),
                                          (int64_t)a.heads / P.pack * a.batch);
   P.order = cta_order(head_group, grid);
-  kern<<<grid, 384, C::SMEM_BYTES, st>>>(P);
+  kern<<<grid, C::THREADS, C::SMEM_BYTES, st>>>(P);
   return fa_host::check_launch("fwd_tc_kernel");
 }
 
@@ -732,13 +744,39 @@ static bool fwd_tc_takes(const FaFwdArgs& a, int64_t kv_batches) {
   return encode_tiled_fn() != nullptr;
 }
 
+// One tile per CTA and two CTAs per SM, or two tiles per CTA and one.  What a CTA does outside its key blocks (about 9000 cycles) runs
+// under the blocks of the other one, and no tile waits for the longer one beside it; but K and V are loaded for each tile, and nothing
+// keeps two CTAs' softmax phases apart: a pair of blocks takes 5 to 9 % longer.  So: few blocks per tile.  Measured, one tile / two
+// tiles, us, 16 heads: causal, head dim 128: 32 x 512 80 / 94, 8 x 1024 57 / 65, 16 x 2048 318 / 323, 8 x 3072 333 / 327, 1 x 32768 (32/8
+// heads) 7327 / 6693; head dim 64: 32 heads, 16 x 2048 528 / 572, 8 x 3072 298 / 313, 8 x 4096 463 / 475; window of 512, 16384 tokens
+// 122 / 141; packed 65536 tokens of 128 to 4096 845 / 898.  Where the tiles of a CTA end together anyway the line is lower:
+// no mask, head dim 128: 32 x 512 94 / 95, 16 x 1024 150 / 144, 64: 77 / 82, 126 / 125; shared tiles (32/8 heads, causal) 4 x 700 28.8 / 31.1,
+// 4 x 1536 101.6 / 100.8, 2 x 2048 82.7 / 80.5.  KV caches, whose lengths differ: 64 x 128 tokens, capacity 1024 65 / 77; 32 x 200, 2048, 64
+// 143 / 157; 4 x 128, 8192 in 2 parts 75.5 / 72.7.
+static bool one_tile(const FaFwdArgs& a, int64_t kv_batches) {
+  const int pack = pack_heads(a.heads / a.heads_k);
+  if (a.seqlen_q <= kBM / pack) return true;  // one tile is all there is
+  const bool varlen = a.cu_seqlens_q != nullptr;
+  const double sq = varlen ? (double)a.total_q / a.batch : a.seqlen_q, sk = varlen ? (double)a.total_k / a.batch : a.seqlen_k;
+  double keys = sk;  // of a row, on average
+  if (a.window_right >= 0) keys = (sq <= sk ? sk - sq / 2 : sk * sk / (2 * sq)) + a.window_right;
+  if (a.window_left >= 0 && keys > (double)a.window_left + a.window_right + 1) keys = (double)a.window_left + a.window_right + 1;
+  if (keys > sk) keys = sk;
+  const double blocks = keys / kBN / (a.num_splits > 1 ? a.num_splits : 1);
+  const bool cache = kv_batches > 0, uneven = a.window_left >= 0 || a.window_right >= 0 || varlen;
+  return blocks <= (cache || (uneven && pack == 1 && a.head_dim <= 64) ? 16.5 : uneven && pack == 1 ? 8.5 : 4.5);
+}
+
+template <typename T>
+static int fwd_tc_dispatch(const FaFwdArgs& a, int64_t kv_batches, cudaStream_t st) {
+  if (a.head_dim > 128) return launch_fwd_tc<T, 256, 1>(a, kv_batches, st);
+  const bool one = one_tile(a, kv_batches);
+  if (a.head_dim > 64) return one ? launch_fwd_tc<T, 128, 1>(a, kv_batches, st) : launch_fwd_tc<T, 128, 2>(a, kv_batches, st);
+  return one ? launch_fwd_tc<T, 64, 1>(a, kv_batches, st) : launch_fwd_tc<T, 64, 2>(a, kv_batches, st);
+}
+
 static int fwd_tc_run(const FaFwdArgs& a, int64_t kv_batches, cudaStream_t st) {
-  const bool bf = a.dtype == FA_DTYPE_BF16;
-  if (a.head_dim <= 64)
-    return bf ? launch_fwd_tc<__nv_bfloat16, 64>(a, kv_batches, st) : launch_fwd_tc<__half, 64>(a, kv_batches, st);
-  if (a.head_dim <= 128)
-    return bf ? launch_fwd_tc<__nv_bfloat16, 128>(a, kv_batches, st) : launch_fwd_tc<__half, 128>(a, kv_batches, st);
-  return bf ? launch_fwd_tc<__nv_bfloat16, 256>(a, kv_batches, st) : launch_fwd_tc<__half, 256>(a, kv_batches, st);
+  return a.dtype == FA_DTYPE_BF16 ? fwd_tc_dispatch<__nv_bfloat16>(a, kv_batches, st) : fwd_tc_dispatch<__half>(a, kv_batches, st);
 }
 
 bool fwd_tc_eligible(const FaFwdArgs& a) { return fwd_tc_takes(a, 0); }
