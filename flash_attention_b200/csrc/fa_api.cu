@@ -26,6 +26,7 @@ bool fwd_tc_eligible(const FaFwdArgs& a);
 int fwd_tc(const FaFwdArgs& a, cudaStream_t st);
 bool fwd_tc_cache_eligible(const FaFwdArgs& a, int64_t kv_batches);
 int fwd_tc_cache(const FaFwdArgs& a, int64_t kv_batches, cudaStream_t st);
+int fwd_tc_cache_splits(int batch, int heads, int heads_k, int seqlen_q, int capacity, int head_dim, int num_sms);
 bool bwd_tc_eligible(const FaBwdArgs& a);
 int bwd_tc_main(const FaBwdArgs& a, cudaStream_t st);
 // fused single-token decode
@@ -388,18 +389,6 @@ static bool cache_on_tensor_cores(const FaKvcacheArgs& a) {
   return !fa_host::env_flag("FA_B200_FORCE_GENERIC") && fa::fwd_tc_cache_eligible(cache_fwd_args(a, 1), a.batch_cache);
 }
 
-// Splits of a multi-token call on the tensor-core kernel.  The lengths are on the device, so the plan knows the capacity
-// only: enough parts for about two rounds of CTAs over the SMs, so that a long sequence next to short ones does not set
-// the time alone, but no part under 4 key blocks of the capacity.
-static int cache_tc_splits(const FaKvcacheArgs& a, int num_sms) {
-  const int group = a.heads / a.heads_k, rows = a.head_dim > 128 ? 128 : 256;
-  const int64_t ctas = (int64_t)a.batch * a.heads_k * (((int64_t)a.seqlen_q * group + rows - 1) / rows);
-  int64_t s = (2 * num_sms + ctas - 1) / ctas;
-  const int64_t most = (a.seqlen_cache + 511) / 512;
-  s = s < most ? s : most;
-  return (int)(s < 1 ? 1 : s > 128 ? 128 : s);
-}
-
 extern "C" {
 
 int fa_kvcache_plan(const FaKvcacheArgs* a, int32_t num_sms, int64_t* lse_accum_bytes, int64_t* out_accum_bytes) {
@@ -410,7 +399,8 @@ int fa_kvcache_plan(const FaKvcacheArgs* a, int32_t num_sms, int64_t* lse_accum_
     splits = fa::decode_plan(*a, num_sms);
   } else {
     splits = a->num_splits;
-    if (splits == 0 && cache_on_tensor_cores(*a)) splits = cache_tc_splits(*a, num_sms);
+    if (splits == 0 && cache_on_tensor_cores(*a))
+      splits = fa::fwd_tc_cache_splits(a->batch, a->heads, a->heads_k, a->seqlen_q, a->seqlen_cache, a->head_dim, num_sms);
     if (splits == 0) splits = splits_by_wave_efficiency(a->batch, a->heads, a->seqlen_q, a->seqlen_cache, a->head_dim, num_sms);
   }
   if (splits < 1) splits = 1;

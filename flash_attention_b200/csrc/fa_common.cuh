@@ -69,6 +69,7 @@ struct FastDiv {
   __device__ __forceinline__ uint32_t div(uint32_t n) const { return (__umulhi(n, mul) + n) >> shift; }
 };
 static inline FastDiv fast_div(int64_t d) {
+  if (d < 1) d = 1;  // (a launch with nothing to do)
   FastDiv f;
   f.d = (uint32_t)d;
   f.shift = 0;

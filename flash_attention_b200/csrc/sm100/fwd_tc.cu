@@ -753,6 +753,7 @@ static bool fwd_tc_takes(const FaFwdArgs& a, int64_t kv_batches) {
 // no mask, head dim 128: 32 x 512 94 / 95, 16 x 1024 150 / 144, 64: 77 / 82, 126 / 125; shared tiles (32/8 heads, causal) 4 x 700 28.8 / 31.1,
 // 4 x 1536 101.6 / 100.8, 2 x 2048 82.7 / 80.5.  KV caches, whose lengths differ: 64 x 128 tokens, capacity 1024 65 / 77; 32 x 200, 2048, 64
 // 143 / 157; 4 x 128, 8192 in 2 parts 75.5 / 72.7.
+constexpr double kOneTileUneven = 16.5;  // key blocks of a tile
 static bool one_tile(const FaFwdArgs& a, int64_t kv_batches) {
   const int pack = pack_heads(a.heads / a.heads_k);
   if (a.seqlen_q <= kBM / pack) return true;  // one tile is all there is
@@ -764,7 +765,7 @@ static bool one_tile(const FaFwdArgs& a, int64_t kv_batches) {
   if (keys > sk) keys = sk;
   const double blocks = keys / kBN / (a.num_splits > 1 ? a.num_splits : 1);
   const bool cache = kv_batches > 0, uneven = a.window_left >= 0 || a.window_right >= 0 || varlen;
-  return blocks <= (cache || (uneven && pack == 1 && a.head_dim <= 64) ? 16.5 : uneven && pack == 1 ? 8.5 : 4.5);
+  return blocks <= (cache || (uneven && pack == 1 && a.head_dim <= 64) ? kOneTileUneven : uneven && pack == 1 ? 8.5 : 4.5);
 }
 
 template <typename T>
@@ -781,6 +782,35 @@ static int fwd_tc_run(const FaFwdArgs& a, int64_t kv_batches, cudaStream_t st) {
 
 bool fwd_tc_eligible(const FaFwdArgs& a) { return fwd_tc_takes(a, 0); }
 int fwd_tc(const FaFwdArgs& a, cudaStream_t st) { return fwd_tc_run(a, 0, st); }
+
+// Parts for several tokens per sequence against a KV cache of which only the capacity is known here: the count with the least
+// estimated time, in us.  A CTA takes 6 and 1.65 per key block for two tiles, 1.55 for one tile that has its SM alone, 1.7 for one of
+// two on an SM (head dims above 128: 2.25); rounds of CTAs count half whole and half by their share, because the lengths differ and a
+// CTA that has fewer keys makes room; the merge takes 4, 0.1 per part and what writing and reading the fp32 rows takes at 3 TB/s.
+// On 15 caches of 1 to 32 sequences and 1024 to 32768 rows, full, ragged and nearly empty, with up to 12 counts each, it is 6 % off
+// the best count on average and 43 % at most (nearly empty caches: one part is best there).  Two rounds of CTAs whatever the
+// lengths, before: 19 % and 76 %.  4 x 128 tokens, 32/8 heads of 128, full caches of 8192 112 -> 80 us; 512 tokens, one of 32768 292 -> 231.
+int fwd_tc_cache_splits(int batch, int heads, int heads_k, int seqlen_q, int capacity, int head_dim, int num_sms) {
+  const int group = heads / heads_k, pack = pack_heads(group), tile_pos = kBM / pack, blocks = (capacity + kBN - 1) / kBN;
+  const double rows = (double)batch * heads * seqlen_q;
+  int best = 1;
+  double best_time = 0;
+  for (int s = 1; s <= 128 && s <= (blocks > 1 ? blocks : 1); ++s) {
+    const int per = (blocks + s - 1) / s;
+    const bool one = head_dim > 128 || seqlen_q <= tile_pos || (double)blocks / s <= kOneTileUneven;
+    const int64_t pos = (int64_t)tile_pos * (one ? 1 : 2);
+    const double ctas = (double)batch * heads_k * (group / pack) * (double)((seqlen_q + pos - 1) / pos) * s;
+    const bool pair = one && head_dim <= 128 && ctas > num_sms;
+    const double block_us = head_dim > 128 ? 2.25 : !one ? 1.65 : pair ? 1.7 : 1.55;
+    const double rounds = ctas / (pair ? 2 * num_sms : num_sms), whole = (double)(int64_t)(rounds + 0.999999);
+    const double t = (6 + block_us * per) * (rounds <= 1 ? 1 : 0.5 * rounds + 0.5 * whole) + (s > 1 ? 4 + s * (0.1 + rows * head_dim * 8 / 3e6) : 0);
+    if (s == 1 || t < best_time) {
+      best_time = t;
+      best = s;
+    }
+  }
+  return best;
+}
 
 // Several tokens per sequence against a KV cache (4 x 128 tokens, 32/8 heads, pages of 256: 469 us on the any-shape kernel,
 // 62 + 13 us merge here).  From 17 rows (tokens x heads of a group) on, where the decode kernel's 16 end: 20 rows, batch 8,
