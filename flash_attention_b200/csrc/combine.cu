@@ -13,17 +13,33 @@ struct CombineParams {
   float* lse;  // may be NULL
   int64_t out_sb, out_ss, out_sh;
   int32_t n_parts, B, H, S, D, lse_pitch;
+  FastDiv by_s, by_h;  // rows of a head, heads
 };
 
 // G: groups of 32 parts, one part per lane.  One group is an instance of its own, without the choice among groups and with two
-// steps of the walk in flight, four with more groups (16384 rows of 128 in 5 parts: 10.9 us, 11.6 with four groups for all;
-// 2048 rows in 64 parts: 12.6 us, 16.6 with two steps in flight).
-template <typename T, int G>
+// steps of the walk in flight, four with more groups (before PRE: 16384 rows of 128 in 5 parts 10.9 us, 11.6 with four groups for
+// all; 2048 rows in 64 parts 12.6 us, 16.6 with two steps in flight).
+// PRE: the rows of the first four parts are on their way before it is known which of them have keys (32 rows in 18 parts: 4.0 -> 3.0
+// us, 1024 in 8: 3.0 -> 2.5, 16384 in 5: 10.2 -> 9.9; with fewer parts and many rows the registers cost more than the wait: 16384 in
+// 2 parts 7.0 without, 7.7 with).
+template <typename T, int G, bool PRE>
 __global__ void __launch_bounds__(128) combine_kernel(const CombineParams p) {
   const int lane = threadIdx.x & 31;
   const int64_t rows = (int64_t)p.B * p.H * p.S;
   const int64_t row = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
   if (row >= rows) return;
+  auto load = [&](int s, float4(&x)[2]) {
+    const float* src = p.out_parts + ((int64_t)s * rows + row) * p.D;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int c = lane * 4 + i * 128;
+      x[i] = s < p.n_parts && c < p.D ? *reinterpret_cast<const float4*>(src + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  };
+  float4 pre[4][2];  // (an empty part's row, which nobody may have written, is dropped below)
+  if constexpr (PRE)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) load(k, pre[k]);
   float l[G];
   uint32_t live[G];  // parts with keys (+inf is not an LSE of theirs)
   float mx = -INFINITY;
@@ -46,10 +62,10 @@ __global__ void __launch_bounds__(128) combine_kernel(const CombineParams p) {
   const bool nan = sum != sum && mx != INFINITY;
   const bool empty = !nan && (!(sum > 0.f) || mx == -INFINITY);
   const float lse = empty || nan ? INFINITY : logf(sum) + mx;
-  const int s_idx = (int)(row % p.S);
-  const int64_t bh = row / p.S;
-  const int h = (int)(bh % p.H), b = (int)(bh / p.H);
-  if (lane == 0 && p.lse) p.lse[bh * p.lse_pitch + s_idx] = lse;
+  // (two 64-bit divisions per row were a third of its instructions; 2^31 rows would be parts of 10^12 bytes)
+  const uint32_t bh = p.by_s.div((uint32_t)row), b = p.by_h.div(bh);
+  const int s_idx = (int)((uint32_t)row - bh * p.S), h = (int)(bh - b * p.H);
+  if (lane == 0 && p.lse) p.lse[(int64_t)bh * p.lse_pitch + s_idx] = lse;
   T* o = reinterpret_cast<T*>(p.out) + b * p.out_sb + s_idx * p.out_ss + h * p.out_sh;
   // head_dim <= 256: at most two 4-column groups per lane
   float4 acc[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
@@ -79,11 +95,22 @@ __global__ void __launch_bounds__(128) combine_kernel(const CombineParams p) {
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       w[k] = __shfl_sync(0xffffffffu, wsel, (s0 + k) & 31);
-      const float* src = p.out_parts + ((int64_t)(s0 + k) * rows + row) * p.D;
+      const bool on = lsel >> k & 1;
+      if (PRE && s0 == 0) {
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int c = lane * 4 + i * 128;
-        x[k][i] = (lsel >> k & 1) && c < p.D ? *reinterpret_cast<const float4*>(src + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int i = 0; i < 2; ++i) x[k][i] = on ? pre[k][i] : make_float4(0.f, 0.f, 0.f, 0.f);
+      } else if (PRE || G > 1) {  // (a branch is the faster form here, a select below)
+        if (on)
+          load(s0 + k, x[k]);
+        else
+          x[k][0] = x[k][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+      } else {
+        const float* src = p.out_parts + ((int64_t)(s0 + k) * rows + row) * p.D;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int c = lane * 4 + i * 128;
+          x[k][i] = on && c < p.D ? *reinterpret_cast<const float4*>(src + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
       }
     }
 #pragma unroll
@@ -110,11 +137,13 @@ __global__ void __launch_bounds__(128) combine_kernel(const CombineParams p) {
 
 int combine(const float* out_parts, const float* lse_parts, const FaTensor& out, float* lse, int lse_pitch, int n_parts,
             int B, int H, int S, int D, int dtype, cudaStream_t st) {
-  CombineParams p{out_parts, lse_parts, out.ptr, lse, out.stride_b, out.stride_s, out.stride_h, n_parts, B, H, S, D, lse_pitch};
+  CombineParams p{out_parts, lse_parts, out.ptr, lse, out.stride_b, out.stride_s, out.stride_h, n_parts, B, H, S, D, lse_pitch, fast_div(S), fast_div(H)};
   int64_t rows = (int64_t)B * H * S;
   unsigned grid = (unsigned)((rows + 3) / 4);
-  auto kern = dtype == FA_DTYPE_BF16 ? (n_parts <= 32 ? combine_kernel<__nv_bfloat16, 1> : combine_kernel<__nv_bfloat16, 4>)
-                                     : (n_parts <= 32 ? combine_kernel<__half, 1> : combine_kernel<__half, 4>);
+  const bool bf = dtype == FA_DTYPE_BF16, pre = n_parts >= 4 || rows <= 4096;
+  auto kern = n_parts > 32 ? (bf ? combine_kernel<__nv_bfloat16, 4, false> : combine_kernel<__half, 4, false>)
+              : pre        ? (bf ? combine_kernel<__nv_bfloat16, 1, true> : combine_kernel<__half, 1, true>)
+                           : (bf ? combine_kernel<__nv_bfloat16, 1, false> : combine_kernel<__half, 1, false>);
   kern<<<grid, 128, 0, st>>>(p);
   return fa_host::check_launch("combine_kernel");
 }
