@@ -35,7 +35,6 @@ constexpr int kN = 64;                   // streamed rows per block
 constexpr int kDH = 256;                 // padded head dim
 constexpr int kChunkA = kR * 128;        // [128 rows][64 x 16-bit]
 constexpr int kChunkB = kN * 128;        // [64 rows][64 x 16-bit]
-constexpr int kTileA = 4 * kChunkA, kTileB = 4 * kChunkB;
 constexpr int kThreads = 384;
 constexpr int kWarpProducer = 8, kWarpMma = 9, kWarpTmem = 10, kWarpMmaX1 = 11;
 constexpr int kRegsCompute = 192, kRegsOther = 88;
@@ -45,13 +44,17 @@ enum Pass { PASS_DV = 0, PASS_DK = 1, PASS_DQ = 2 };
 enum WWait { W_W_ALIGN = 60, W_W_A = 61, W_W_B_FULL = 62, W_W_B_EMPTY = 63, W_W_X1 = 64, W_W_X2 = 65, W_W_W = 66,
              W_W_DONE = 67, W_W_READ = 68 };
 
-template <int PASS>
+// TRIM: head dims up to 192, tiles of three chunks
+template <int PASS, bool TRIM>
 struct WCfg {
+  static constexpr int kTileA = (TRIM ? 3 : 4) * kChunkA, kTileB = (TRIM ? 3 : 4) * kChunkB;
   static constexpr int NA = PASS == PASS_DV ? 1 : 2;
   // passes dK / dQ: B1 is held from X1(j) (issued a block early) to the last product of block j, B2 only by X2(j);
   // pass dV: B1 (Q) only by X1(j), B2 (dO) from its arrival to the last product of block j
-  static constexpr int NS1 = 2;
-  static constexpr int NS2 = PASS == PASS_DV ? 3 : 1;
+  // What smaller tiles leave goes to deeper rings: with one slot for B2 its next tile is loaded after X2(j) and X2(j+1) waits for it
+  // (8 x 2048 tokens, no mask, whole backward in us: 12 heads of 160 1255 -> 1080, 10 of 192 1117 -> 981).
+  static constexpr int NS1 = TRIM ? 3 : 2;
+  static constexpr int NS2 = TRIM ? (PASS == PASS_DV ? 4 : 2) : (PASS == PASS_DV ? 3 : 1);
   static constexpr int OFF_A = 0;
   static constexpr int OFF_B1 = NA * kTileA;
   static constexpr int OFF_B2 = OFF_B1 + NS1 * kTileB;
@@ -97,7 +100,8 @@ struct Walk {
 
 template <typename T, int PASS, bool TRIM>
 __global__ void __launch_bounds__(kThreads, 1) bwd_wide_tc_kernel(const __grid_constant__ WParams P) {
-  using C = WCfg<PASS>;
+  using C = WCfg<PASS, TRIM>;
+  constexpr int kTileA = C::kTileA, kTileB = C::kTileB;
   constexpr int NS1 = C::NS1, NS2 = C::NS2;
   constexpr bool kRowsAreQueries = PASS == PASS_DQ;
   const FaBwdArgs& a = P.a;
@@ -552,9 +556,9 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_wide_tc_kernel(const __grid_c
   if (warp == kWarpTmem) tmem_dealloc(tmem, C::TMEM_COLS);
 }
 
-template <typename T, int PASS>
+template <typename T, int PASS, bool TRIM>
 int launch_wide(const FaBwdArgs& a, cudaStream_t st) {
-  using C = WCfg<PASS>;
+  using C = WCfg<PASS, TRIM>;
   WParams P;
   P.a = a;
   const bool varlen = a.cu_seqlens_q != nullptr;
@@ -571,11 +575,10 @@ int launch_wide(const FaBwdArgs& a, cudaStream_t st) {
   } else {
     P.ta1 = tk, P.ta2 = tv, P.tb1 = tq, P.tb2 = tdo;
   }
-  const bool trim = head_trims<kDH>(a.head_dim);
-  auto kern = trim ? bwd_wide_tc_kernel<T, PASS, true> : bwd_wide_tc_kernel<T, PASS, false>;
+  auto kern = bwd_wide_tc_kernel<T, PASS, TRIM>;
   P.status = status_ref(true);
-  static fa_host::DeviceOnce once[2];
-  if (int rc = fa_host::raise_smem_limit(once[trim], reinterpret_cast<const void*>(kern), C::SMEM_BYTES, "bwd_wide_tc_kernel")) return rc;
+  static fa_host::DeviceOnce once;
+  if (int rc = fa_host::raise_smem_limit(once, reinterpret_cast<const void*>(kern), C::SMEM_BYTES, "bwd_wide_tc_kernel")) return rc;
   dim3 grid(((PASS == PASS_DQ ? a.seqlen_q : a.seqlen_k) + kR - 1) / kR, PASS == PASS_DQ ? a.heads : a.heads_k, a.batch);
   const int group = a.heads / a.heads_k;
   const bool uneven = a.window_left >= 0 || a.window_right >= 0 || a.cu_seqlens_q;
@@ -587,14 +590,14 @@ int launch_wide(const FaBwdArgs& a, cudaStream_t st) {
   return fa_host::check_launch("bwd_wide_tc_kernel");
 }
 
-template <typename T>
+template <typename T, bool TRIM>
 int run_wide(const FaBwdArgs& a, int parts, cudaStream_t st) {
   int rc = 0;
   if (parts & 2) {
-    rc = launch_wide<T, PASS_DV>(a, st);
-    if (!rc) rc = launch_wide<T, PASS_DK>(a, st);
+    rc = launch_wide<T, PASS_DV, TRIM>(a, st);
+    if (!rc) rc = launch_wide<T, PASS_DK, TRIM>(a, st);
   }
-  if (!rc && (parts & 1)) rc = launch_wide<T, PASS_DQ>(a, st);
+  if (!rc && (parts & 1)) rc = launch_wide<T, PASS_DQ, TRIM>(a, st);
   return rc;
 }
 
@@ -603,7 +606,9 @@ int run_wide(const FaBwdArgs& a, int parts, cudaStream_t st) {
 // dV, dK (parts & 2) and dQ (parts & 1) of a backward pass with 128 < head_dim <= 256 (softmax_d must hold
 // rowsum(dO o O)).
 int bwd_wide_tc_main(const FaBwdArgs& a, int parts, cudaStream_t st) {
-  return a.dtype == FA_DTYPE_BF16 ? run_wide<__nv_bfloat16>(a, parts, st) : run_wide<__half>(a, parts, st);
+  const bool bf = a.dtype == FA_DTYPE_BF16;
+  if (head_trims<kDH>(a.head_dim)) return bf ? run_wide<__nv_bfloat16, true>(a, parts, st) : run_wide<__half, true>(a, parts, st);
+  return bf ? run_wide<__nv_bfloat16, false>(a, parts, st) : run_wide<__half, false>(a, parts, st);
 }
 
 }  // namespace fa
