@@ -111,7 +111,7 @@ EXPORTS = (
     "fa_fwd", "fa_bwd", "fa_fwd_kvcache", "fa_fwd_num_splits", "fa_kvcache_plan", "fa_bwd_workspace_bytes",
     "fa_combine", "fa_last_error", "fa_build_info", "fa_device_status", "fa_abi_struct_size",
     "fa_fwd_kvcache_noalloc", "fa_noalloc_scratch_bytes", "fa_merge_partial", "fa_rotary",
-    "fa_selftest_wait_timeout", "fa_selftest_device_once", "fa_last_path",
+    "fa_selftest_wait_timeout", "fa_selftest_device_once", "fa_last_path", "fa_last_forward_tiles",
 )
 
 _lib = None
@@ -152,6 +152,7 @@ def lib():
         L.fa_last_error.restype = C.c_char_p
         L.fa_build_info.restype = C.c_char_p
         L.fa_last_path.restype = C.c_char_p
+        L.fa_last_forward_tiles.restype = C.c_int
         L.fa_device_status.restype = C.c_int
         L.fa_selftest_wait_timeout.argtypes = [c_i64, c_vp]
         L.fa_selftest_wait_timeout.restype = C.c_int
@@ -173,6 +174,11 @@ def last_error():
 def last_path():
     """Kernels launched by this process's last fa_fwd / fa_bwd / fa_fwd_kvcache call (any thread)."""
     return lib().fa_last_path().decode()
+
+
+def last_forward_tiles():
+    """Query tiles per CTA (1 or 2) of the last launch of the tensor-core forward."""
+    return lib().fa_last_forward_tiles()
 
 
 def check(status, what):

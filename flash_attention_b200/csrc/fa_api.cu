@@ -24,6 +24,7 @@ int kvcache_prep(const FaKvcacheArgs& a, int q_follows_rows, cudaStream_t st);
 // tcgen05 kernels (sm100/)
 bool fwd_tc_eligible(const FaFwdArgs& a);
 int fwd_tc(const FaFwdArgs& a, cudaStream_t st);
+int fwd_tc_last_tiles();
 bool fwd_tc_cache_eligible(const FaFwdArgs& a, int64_t kv_batches);
 int fwd_tc_cache(const FaFwdArgs& a, int64_t kv_batches, cudaStream_t st);
 int fwd_tc_cache_splits(int batch, int heads, int heads_k, int seqlen_q, int capacity, int head_dim, int num_sms);
@@ -166,6 +167,8 @@ extern "C" {
 const char* fa_last_error(void) { return fa_host::g_err; }
 
 const char* fa_last_path(void) { return g_last_path; }
+
+int fa_last_forward_tiles(void) { return fa::fwd_tc_last_tiles(); }
 
 const char* fa_build_info(void) {
   return "libfa_b200 arch=sm_100a kernels=fwd_tc(tcgen05+TMA),bwd_dkdv_tc(tcgen05+TMA),bwd_dq_tc(tcgen05+TMA),bwd_wide_tc(tcgen05+TMA),decode_splitkv(TMA),"

@@ -768,10 +768,14 @@ static bool one_tile(const FaFwdArgs& a, int64_t kv_batches) {
   return blocks <= (cache || (uneven && pack == 1 && a.head_dim <= 64) ? kOneTileUneven : uneven && pack == 1 ? 8.5 : 4.5);
 }
 
+static volatile int g_last_tiles = 0;
+int fwd_tc_last_tiles() { return g_last_tiles; }
+
 template <typename T>
 static int fwd_tc_dispatch(const FaFwdArgs& a, int64_t kv_batches, cudaStream_t st) {
+  const bool one = a.head_dim > 128 || one_tile(a, kv_batches);
+  g_last_tiles = one ? 1 : 2;
   if (a.head_dim > 128) return launch_fwd_tc<T, 256, 1>(a, kv_batches, st);
-  const bool one = one_tile(a, kv_batches);
   if (a.head_dim > 64) return one ? launch_fwd_tc<T, 128, 1>(a, kv_batches, st) : launch_fwd_tc<T, 128, 2>(a, kv_batches, st);
   return one ? launch_fwd_tc<T, 64, 1>(a, kv_batches, st) : launch_fwd_tc<T, 64, 2>(a, kv_batches, st);
 }

@@ -265,6 +265,8 @@ const char* fa_last_error(void);
    (whichever thread made it) launched, e.g. "fwd_tc", "fwd_generic+combine", "bwd_tc+bwd_dq_tc", "bwd_wide_tc", "decode+combine"
    (no counterpart in the reference; tests use it to pin a case to the kernel it is meant to cover). */
 const char* fa_last_path(void);
+/* Query tiles per CTA of this process's last launch of the "fwd_tc" kernel: 1, 2, or 0 before the first (for tests, as fa_last_path). */
+int fa_last_forward_tiles(void);
 /* Compile-time facts: "sm_100a", kernel list, build flags. */
 const char* fa_build_info(void);
 /* Device-side status word of the tensor-core and decode kernels: 0 = ok, otherwise the code of the
