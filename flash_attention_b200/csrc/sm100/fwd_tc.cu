@@ -747,25 +747,37 @@ static bool fwd_tc_takes(const FaFwdArgs& a, int64_t kv_batches) {
 // One tile per CTA and two CTAs per SM, or two tiles per CTA and one.  What a CTA does outside its key blocks (about 9000 cycles) runs
 // under the blocks of the other one, and no tile waits for the longer one beside it; but K and V are loaded for each tile, and nothing
 // keeps two CTAs' softmax phases apart: a pair of blocks takes 5 to 9 % longer.  So: few blocks per tile.  Measured, one tile / two
-// tiles, us, 16 heads: causal, head dim 128: 32 x 512 80 / 94, 8 x 1024 57 / 65, 16 x 2048 318 / 323, 8 x 3072 333 / 327, 1 x 32768 (32/8
-// heads) 7327 / 6693; head dim 64: 32 heads, 16 x 2048 528 / 572, 8 x 3072 298 / 313, 8 x 4096 463 / 475; window of 512, 16384 tokens
-// 122 / 141; packed 65536 tokens of 128 to 4096 845 / 898.  Where the tiles of a CTA end together anyway the line is lower:
-// no mask, head dim 128: 32 x 512 94 / 95, 16 x 1024 150 / 144, 64: 77 / 82, 126 / 125; shared tiles (32/8 heads, causal) 4 x 700 28.8 / 31.1,
-// 4 x 1536 101.6 / 100.8, 2 x 2048 82.7 / 80.5.  KV caches, whose lengths differ: 64 x 128 tokens, capacity 1024 65 / 77; 32 x 200, 2048, 64
-// 143 / 157; 4 x 128, 8192 in 2 parts 75.5 / 72.7.
-constexpr double kOneTileUneven = 16.5;  // key blocks of a tile
+// tiles, us, by key blocks of a tile on average:
+// causal, window or packed, tiles of one head: head dim 64 560 / 580 (12 blocks), 910 / 927 (16), 1030 / 1033 (20), 982 / 969 (24), 1673 / 1619
+// (32); 128 201 / 212 (6), 312 / 320 (8), 346 / 346 (10), 326 / 324 (12), 541 / 521 (16); 96 505 / 524 (16); window of 512, 16384 tokens 122 / 141;
+// packed 65536 tokens of 128 to 4096 845 / 898.  Where the tiles of a CTA end together anyway the line is lower: no mask, head dim 128 67 / 74 (3),
+// 92 / 93 (4), 113 / 114 (6), 146 / 139 (8), 64 75 / 81 (4), 94 / 100 (6), 124 / 123 (8), 196 / 189 (12); shared tiles (32/8 heads of 128, causal) 33 / 34
+// (3), 105 / 106 (4), 100 / 100 (6), 81 / 79 (8), 160 / 152 (12).
+// KV caches, of which only the capacity is known here, one tile against two, by blocks of a part.  Under 2.5 rounds of one-tile CTAs,
+// head dim 128 -15 to +3 % (4), -8 to +2 % (8), -2 to +5 % (12), -3 to +7 % (16), 64 with tiles of one head -12 to -6 % (8), -2 to +6 % (12),
+// with shared ones -3 to +5 % (8), +2 to +9 % (12); more rounds 128 -3 to +5 % (12), +1 to +7 % (16), 96 -1 to +5 % (16), 64 -6 to +2 % (16).  An odd
+// number of tiles leaves the last two-tile CTA of a sequence with one: 300 rows, 10 blocks, 128 41 / 45, 326 x 4 rows, 13 blocks, 64 53 / 56.
+// Rows that fill one tile at most: two CTAs on an SM are 12 to 38 % faster than one after the other.  But a CTA that has its SM alone
+// gets nothing from sharing it and wants the longer ring of the two-tile form: head dim 128 -1 to +2 % (8), -2 to +14 % (12), +5 to +17 %
+// (16), +10 to +19 % (32), 64 -2 to +3 % (16), -2 to +4 % (32).
+static bool one_tile_form(int64_t ctas, int row_tiles, bool cache, bool uneven, int pack, int head_dim, double blocks, int num_sms) {
+  const bool small = head_dim <= 64, even = row_tiles % 2 == 0;
+  if (row_tiles <= 1) return ctas > num_sms || blocks <= (small ? 16.5 : 10.5);
+  if (!cache) return blocks <= (!uneven || pack > 1 ? 4.5 : small ? 16.5 : 8.5);
+  if (ctas >= 5 * num_sms) return blocks <= (head_dim <= 96 ? 16.5 : 12.5);
+  return blocks <= (small ? (!even ? 16.5 : pack == 1 ? 12.5 : 8.5) : head_dim <= 96 ? 16.5 : even ? 8.5 : 12.5);
+}
 static bool one_tile(const FaFwdArgs& a, int64_t kv_batches) {
-  const int pack = pack_heads(a.heads / a.heads_k);
-  if (a.seqlen_q <= kBM / pack) return true;  // one tile is all there is
+  const int pack = pack_heads(a.heads / a.heads_k), parts = a.num_splits > 1 ? a.num_splits : 1;
   const bool varlen = a.cu_seqlens_q != nullptr;
   const double sq = varlen ? (double)a.total_q / a.batch : a.seqlen_q, sk = varlen ? (double)a.total_k / a.batch : a.seqlen_k;
   double keys = sk;  // of a row, on average
   if (a.window_right >= 0) keys = (sq <= sk ? sk - sq / 2 : sk * sk / (2 * sq)) + a.window_right;
   if (a.window_left >= 0 && keys > (double)a.window_left + a.window_right + 1) keys = (double)a.window_left + a.window_right + 1;
   if (keys > sk) keys = sk;
-  const double blocks = keys / kBN / (a.num_splits > 1 ? a.num_splits : 1);
-  const bool cache = kv_batches > 0, uneven = a.window_left >= 0 || a.window_right >= 0 || varlen;
-  return blocks <= (cache || (uneven && pack == 1 && a.head_dim <= 64) ? kOneTileUneven : uneven && pack == 1 ? 8.5 : 4.5);
+  const int pos = kBM / pack, row_tiles = (int)(((int64_t)a.seqlen_q + pos - 1) / pos);
+  return one_tile_form((int64_t)a.batch * (a.heads / pack) * row_tiles * parts, row_tiles, kv_batches > 0,
+                       a.window_left >= 0 || a.window_right >= 0 || varlen, pack, a.head_dim, keys / kBN / parts, fa_host::sm_count());
 }
 
 static volatile int g_last_tiles = 0;
@@ -791,17 +803,22 @@ int fwd_tc(const FaFwdArgs& a, cudaStream_t st) { return fwd_tc_run(a, 0, st); }
 // estimated time, in us.  A CTA takes 6 and 1.65 per key block for two tiles, 1.55 for one tile that has its SM alone, 1.7 for one of
 // two on an SM (head dims above 128: 2.25); rounds of CTAs count half whole and half by their share, because the lengths differ and a
 // CTA that has fewer keys makes room; the merge takes 4, 0.1 per part and what writing and reading the fp32 rows takes at 3 TB/s.
-// On 15 caches of 1 to 32 sequences and 1024 to 32768 rows, full, ragged and nearly empty, with up to 12 counts each, it is 6 % off
-// the best count on average and 43 % at most (nearly empty caches: one part is best there).  Two rounds of CTAs whatever the
-// lengths, before: 19 % and 76 %.  4 x 128 tokens, 32/8 heads of 128, full caches of 8192 112 -> 80 us; 512 tokens, one of 32768 292 -> 231.
+// 178 calls (55 caches of 1 to 63 sequences and 1024 to 32768 rows, each full, ragged and nearly empty; every count from 1 to 12, then 16,
+// 20, 24 and 32): 4.7 % off the best count on average, 67 % at most (nearly empty caches: one part is best there), and 22 % faster on average than two
+// rounds of CTAs whatever the lengths (36 % off the best).  Six calls are 2 to 31 % slower than with those: two nearly empty
+// caches (31 and 17 %), 11 full sequences that are 1.2 rounds in one part (11 %), three ragged ones (2 to 16 %).  The merge of 16384 rows takes 7 us in 2 parts, less than is
+// charged here; charged as 4 to 6 TB/s the count is half a percent further off, because more parts also make ragged lengths less even.
+// 4 x 128 tokens, 32/8 heads of 128, full caches of 8192 112 -> 80 us; 512 tokens, one of 32768 292 -> 231.
 int fwd_tc_cache_splits(int batch, int heads, int heads_k, int seqlen_q, int capacity, int head_dim, int num_sms) {
   const int group = heads / heads_k, pack = pack_heads(group), tile_pos = kBM / pack, blocks = (capacity + kBN - 1) / kBN;
+  const int row_tiles = (int)(((int64_t)seqlen_q + tile_pos - 1) / tile_pos);
   const double rows = (double)batch * heads * seqlen_q;
   int best = 1;
   double best_time = 0;
   for (int s = 1; s <= 128 && s <= (blocks > 1 ? blocks : 1); ++s) {
     const int per = (blocks + s - 1) / s;
-    const bool one = head_dim > 128 || seqlen_q <= tile_pos || (double)blocks / s <= kOneTileUneven;
+    const bool one = head_dim > 128 || one_tile_form((int64_t)batch * heads_k * (group / pack) * row_tiles * s, row_tiles, true, true, pack, head_dim,
+                                                     (double)blocks / s, num_sms);
     const int64_t pos = (int64_t)tile_pos * (one ? 1 : 2);
     const double ctas = (double)batch * heads_k * (group / pack) * (double)((seqlen_q + pos - 1) / pos) * s;
     const bool pair = one && head_dim <= 128 && ctas > num_sms;
