@@ -76,9 +76,10 @@ bool int32_vector(const Tensor& t, c10::Device dev, int64_t n) {
 }
 
 // fwd / varlen_fwd: [out, q, k, v, out, softmax_lse, None, rng_state]
-py::object fwd(const Tensor& q, const Tensor& k, const Tensor& v, const MaybeTensor& cu_q, const MaybeTensor& cu_k, int64_t max_q,
+// varlen: which of the two was called; packed operands without their offsets are an error, not a padded batch
+py::object fwd(bool varlen, const Tensor& q, const Tensor& k, const Tensor& v, const MaybeTensor& cu_q, const MaybeTensor& cu_k, int64_t max_q,
                int64_t max_k, double scale, bool causal, int64_t wl, int64_t wr) {
-  const bool varlen = cu_q.has_value();
+  if (cu_q.has_value() != varlen || cu_k.has_value() != varlen) return py::none();
   if (!takes(q) || q.dim() != (varlen ? 3 : 4) || getenv("FA_B200_FWD_SPLITS")) return py::none();
   const c10::Device dev = q.device();
   for (const Tensor* t : {&k, &v})
@@ -88,7 +89,7 @@ py::object fwd(const Tensor& q, const Tensor& k, const Tensor& v, const MaybeTen
   if (varlen) {
     total_q = q.size(0), total_k = k.size(0);
     batch = cu_q->numel() - 1, sq = max_q, sk = max_k;
-    if (!cu_k || !int32_vector(*cu_q, dev, batch + 1) || !int32_vector(*cu_k, dev, batch + 1) || total_q <= 0 || total_k <= 0) return py::none();
+    if (!int32_vector(*cu_q, dev, batch + 1) || !int32_vector(*cu_k, dev, batch + 1) || total_q <= 0 || total_k <= 0) return py::none();
     if (!has_shape(k, {total_k, heads_k, d}) || !has_shape(v, {total_k, heads_k, d})) return py::none();
   } else {
     batch = q.size(0), sq = q.size(1), sk = k.size(1);
@@ -138,10 +139,10 @@ py::object fwd(const Tensor& q, const Tensor& k, const Tensor& v, const MaybeTen
 }
 
 // bwd / varlen_bwd: [dq, dk, dv, softmax_d]
-py::object bwd(const Tensor& dout, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& out, const Tensor& lse,
+py::object bwd(bool varlen, const Tensor& dout, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& out, const Tensor& lse,
                const MaybeTensor& dq_, const MaybeTensor& dk_, const MaybeTensor& dv_, const MaybeTensor& cu_q, const MaybeTensor& cu_k,
                int64_t max_q, int64_t max_k, double scale, bool causal, int64_t wl, int64_t wr, bool deterministic) {
-  const bool varlen = cu_q.has_value();
+  if (cu_q.has_value() != varlen || cu_k.has_value() != varlen) return py::none();
   if (!takes(q) || q.dim() != (varlen ? 3 : 4) || !dq_ || !dk_ || !dv_) return py::none();
   const c10::Device dev = q.device();
   const Tensor &dq = *dq_, &dk = *dk_, &dv = *dv_;
@@ -152,7 +153,7 @@ py::object bwd(const Tensor& dout, const Tensor& q, const Tensor& k, const Tenso
   if (varlen) {
     total_q = q.size(0), total_k = k.size(0);
     batch = cu_q->numel() - 1, sq = max_q, sk = max_k;
-    if (!cu_k || !int32_vector(*cu_q, dev, batch + 1) || !int32_vector(*cu_k, dev, batch + 1) || total_q <= 0 || total_k <= 0) return py::none();
+    if (!int32_vector(*cu_q, dev, batch + 1) || !int32_vector(*cu_k, dev, batch + 1) || total_q <= 0 || total_k <= 0) return py::none();
     if (!has_shape(k, {total_k, heads_k, d})) return py::none();
   } else {
     batch = q.size(0), sq = q.size(1), sk = k.size(1);

@@ -171,7 +171,7 @@ def fwd(q, k, v, out_, p_dropout, softmax_scale, is_causal, window_size_left, wi
     Returns [out, q_padded, k_padded, v_padded, out_padded, softmax_lse, p, rng_state].
     """
     if out_ is None and p_dropout == 0.0 and not return_softmax:
-        r = _glue.fwd(q, k, v, None, None, 0, 0, float(softmax_scale), bool(is_causal), int(window_size_left), int(window_size_right))
+        r = _glue.fwd(False, q, k, v, None, None, 0, 0, float(softmax_scale), bool(is_causal), int(window_size_left), int(window_size_right))
         if r is not None:
             return r
     dt = _dtype_code(q)
@@ -270,7 +270,7 @@ def varlen_fwd(q, k, v, out_, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seql
     q: (total_q, heads, d); k, v: (total_k, heads_k, d); cu_seqlens_*: (batch + 1) int32.
     """
     if out_ is None and p_dropout == 0.0 and not return_softmax and not zero_tensors:
-        r = _glue.fwd(q, k, v, cu_seqlens_q, cu_seqlens_k, int(max_seqlen_q), int(max_seqlen_k), float(softmax_scale), bool(is_causal),
+        r = _glue.fwd(True, q, k, v, cu_seqlens_q, cu_seqlens_k, int(max_seqlen_q), int(max_seqlen_k), float(softmax_scale), bool(is_causal),
                       int(window_size_left), int(window_size_right))
         if r is not None:
             return r
@@ -362,7 +362,7 @@ def _grad_out(given, shape, like, name):
 def _bwd_common(varlen, dout, q, k, v, out, softmax_lse, dq_, dk_, dv_, cu_q, cu_k, max_q, max_k, p_dropout,
                 softmax_scale, is_causal, wl_in, wr_in, rng_state, what, deterministic=False):
     if p_dropout == 0.0:
-        r = _glue.bwd(dout, q, k, v, out, softmax_lse, dq_, dk_, dv_, cu_q, cu_k, int(max_q), int(max_k), float(softmax_scale),
+        r = _glue.bwd(varlen, dout, q, k, v, out, softmax_lse, dq_, dk_, dv_, cu_q, cu_k, int(max_q), int(max_k), float(softmax_scale),
                       bool(is_causal), int(wl_in), int(wr_in), bool(deterministic))
         if r is not None:
             return r
