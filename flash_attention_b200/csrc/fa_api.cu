@@ -189,6 +189,8 @@ int fa_selftest_device_once(const int32_t* devices, int32_t n, int32_t* needed) 
   return 0;
 }
 
+int64_t fa_selftest_fast_div(int64_t n, int64_t divisor) { return (int64_t)fa::fast_div(divisor).div((uint32_t)n); }
+
 int fa_abi_struct_size(int32_t which) {
   switch (which) {
     case 0: return (int)sizeof(FaTensor);

@@ -65,11 +65,19 @@ __device__ __forceinline__ bool visible(int i, int j, int sk, int shift, int wl,
 // compiler's own division is a chain of some forty instructions, about 200 cycles, and three to eight of them stood in front of a CTA's
 // first load: 32 x 512 tokens, 16 heads of 128 causal, forward 97.0 -> 93.1 us; 16 x 2048, 32 heads of 64 causal, backward 1284 -> 1222.
 struct FastDiv {
-  uint32_t d, mul, shift;  // n / d = (mulhi(n, mul) + n) >> shift for n < 2^31
-  __device__ __forceinline__ uint32_t div(uint32_t n) const { return (__umulhi(n, mul) + n) >> shift; }
+  uint32_t d, mul, shift;  // n / d = (mulhi(n, mul) + n) >> shift, the sum in 33 bits: all n and d of 32 bits
+  __host__ __device__ __forceinline__ uint32_t div(uint32_t n) const {
+#ifdef __CUDA_ARCH__
+    const uint32_t hi = __umulhi(n, mul);
+#else
+    const uint32_t hi = (uint32_t)(((uint64_t)n * mul) >> 32);
+#endif
+    return (uint32_t)(((uint64_t)hi + n) >> shift);
+  }
 };
 static inline FastDiv fast_div(int64_t d) {
   if (d < 1) d = 1;  // (a launch with nothing to do)
+  if (d > 0xffffffffll) d = 0xffffffffll;  // (CTAs are counted in 32 bits)
   FastDiv f;
   f.d = (uint32_t)d;
   f.shift = 0;

@@ -285,6 +285,8 @@ int fa_device_status(void);
    have configured its device. */
 int fa_selftest_wait_timeout(int64_t limit_cycles, fa_stream_t stream);
 int fa_selftest_device_once(const int32_t* devices, int32_t n, int32_t* needed);
+/* n / divisor (both below 2^32) by the multiplication that the kernels use for divisors known at launch (host only). */
+int64_t fa_selftest_fast_div(int64_t n, int64_t divisor);
 
 #ifdef __cplusplus
 }
