@@ -329,22 +329,15 @@ __host__ __device__ constexpr uint32_t make_idesc(int M, int N, int ab_format, i
 // TRIM is an instance of the kernel of its own for the same reason (all in one: 128 1.4 %, 256 9 % longer).
 template <int DH, bool TRIM, typename F>
 __device__ __forceinline__ void with_head_steps(int head_dim, F&& f) {
-  if (!TRIM)
+  if constexpr (!TRIM) {
     f(std::integral_constant<int, DH / 16>{});
-  else if (DH == 64 && head_dim <= 32)
-    f(std::integral_constant<int, 2>{});
-  else if (DH == 64 && head_dim <= 48)
-    f(std::integral_constant<int, 3>{});
-  else if (DH == 128 && head_dim <= 80)
-    f(std::integral_constant<int, 5>{});
-  else if (DH == 128 && head_dim <= 96)
-    f(std::integral_constant<int, 6>{});
-  else if (DH == 256 && head_dim <= 160)
-    f(std::integral_constant<int, 10>{});
-  else if (DH == 256 && head_dim <= 192)
-    f(std::integral_constant<int, 12>{});
-  else
-    f(std::integral_constant<int, DH / 16>{});
+  } else {  // (head_trims: at most three quarters of DH)
+    constexpr int kLess = DH == 64 ? 2 : DH == 128 ? 5 : 10, kMore = DH / 16 * 3 / 4;
+    if (head_dim <= kLess * 16)
+      f(std::integral_constant<int, kLess>{});
+    else
+      f(std::integral_constant<int, kMore>{});
+  }
 }
 // chunks of a tile of DH columns (a tile of up to 128 columns is always loaded whole: its last chunk holds data)
 template <int DH, bool TRIM>
