@@ -66,6 +66,7 @@ struct WCfg {
   static constexpr int COL_X1 = 0, COL_X2 = 64, COL_W = 128, COL_OUT = 256;  // W: two 32-column buffers
   static constexpr int TMEM_COLS = 512;
   static_assert(SMEM_BYTES <= 232448, "shared memory of one CTA");
+  static_assert(kR * kDH * 2 <= OFF_STATS, "the rows of the result are staged over the tiles");
 };
 
 struct WParams {
@@ -388,7 +389,8 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_wide_tc_kernel(const __grid_c
             }
           }
         } else {
-          // 16-bit rows over the first stationary tile (every MMA is done), 16-byte pieces swizzled
+          // 16-bit rows, 16-byte pieces swizzled, over the stationary tiles (the first alone is smaller in the trimmed instance) and, in its
+          // pass dV, the first ring slot: every load was waited for by a product and every MMA is done
 #pragma unroll
           for (int i = 0; i < 32; i += 8) {
             uint4 v;
