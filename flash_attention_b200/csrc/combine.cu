@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(128) combine_kernel(const CombineParams p) {
   const bool nan = sum != sum && mx != INFINITY;
   const bool empty = !nan && (!(sum > 0.f) || mx == -INFINITY);
   const float lse = empty || nan ? INFINITY : logf(sum) + mx;
-  // (two 64-bit divisions per row were a third of its instructions; 2^31 rows would be parts of 10^12 bytes)
+  // (two 64-bit divisions per row were a third of its instructions; combine() checks that a row's number has 32 bits)
   const uint32_t bh = p.by_s.div((uint32_t)row), b = p.by_h.div(bh);
   const int s_idx = (int)((uint32_t)row - bh * p.S), h = (int)(bh - b * p.H);
   if (lane == 0 && p.lse) p.lse[(int64_t)bh * p.lse_pitch + s_idx] = lse;
@@ -73,8 +73,8 @@ __global__ void __launch_bounds__(128) combine_kernel(const CombineParams p) {
 #pragma unroll
   for (int i = 0; i < G; ++i) wgt[i] = nan ? sum : empty ? 0.f : __expf(l[i] - lse);
   // Bound by the latency of the loads: four parts are in flight at a time (16 parts of 2048 x 128: 9.4 us, 11.5 us with one
-  // at a time).  Empty parts, those past the last one among them, are not read: nobody may have written them.  The walk ends
-  // behind the last part with keys (2048 rows of 128, 64 parts, 4 of them with keys: 8.9 -> 3.5 us; a test of every four parts
+  // at a time).  Empty parts, those past the last one among them, are not read, or dropped where PRE has read them: nobody
+  // may have written them.  The walk ends behind the last part with keys (2048 rows of 128, 64 parts, 4 of them with keys: 8.9 -> 3.5 us; a test of every four parts
   // in the loop instead: 4.6, and 16.2 where all have keys).
   constexpr int kSteps = G == 1 ? 2 : 4;
   int end = 0;
@@ -139,6 +139,7 @@ int combine(const float* out_parts, const float* lse_parts, const FaTensor& out,
             int B, int H, int S, int D, int dtype, cudaStream_t st) {
   CombineParams p{out_parts, lse_parts, out.ptr, lse, out.stride_b, out.stride_s, out.stride_h, n_parts, B, H, S, D, lse_pitch, fast_div(S), fast_div(H)};
   int64_t rows = (int64_t)B * H * S;
+  FA_REQUIRE(rows < (1ll << 32), "too many rows");
   unsigned grid = (unsigned)((rows + 3) / 4);
   const bool bf = dtype == FA_DTYPE_BF16, pre = n_parts >= 4 || rows <= 4096;
   auto kern = n_parts > 32 ? (bf ? combine_kernel<__nv_bfloat16, 4, false> : combine_kernel<__half, 4, false>)

@@ -204,13 +204,14 @@ int fa_abi_struct_size(int32_t which) {
 
 int fa_fwd_num_splits(int32_t batch, int32_t heads, int32_t seqlen_q, int32_t seqlen_k, int32_t head_dim,
                       int32_t num_sms) {
-  // For the tensor-core kernel (a work item is 256 query rows, 128 above head dim 128, and walks 128-key blocks): the
-  // split count with the least estimated time, in us.  The terms are fitted to 362 shapes of head dim 64 to 256, 8 to 2048
-  // query rows and 128 to 32768 keys, each timed with up to 17 counts (one B200, 1965 MHz): a round of CTAs takes 6 and 1.75
-  // (d <= 64), 2 (d <= 128) or 2.25 per key block, the merge 4, 0.15 per part and what writing and reading the parts' fp32
-  // rows takes at 5 TB/s.  The count it finds is 0.5 % off the best one on average and 7 % at most.  With 2 per block for all
-  // head dims, 5 for the merge and nothing per part: 0.8 % and 20 %; with splits_by_wave_efficiency: 7 % and a factor
-  // of 2.3.  (82 x 7511, 2 heads of 256: 1 part 125 us, 59 parts 33.5, 20 parts 24.7.)  A mask is not looked at.
+  // For the tensor-core kernel: the split count with the least estimated time, in us, for work items of 256 query rows (128 above head
+  // dim 128) that walk 128-key blocks: a round of them takes 6 and 1.75 (d <= 64), 2 (d <= 128) or 2.25 per key block, the merge 4, 0.15
+  // per part and what writing and reading the parts' fp32 rows takes at 5 TB/s.  The terms were fitted to 362 shapes of head dim 64 to 256, 8 to
+  // 2048 query rows and 128 to 32768 keys on a kernel with 256-row CTAs only (0.5 % off the best count on average, 7 % at most; with 2 per block for all
+  // head dims, 5 for the merge and nothing per part 0.8 % and 20 %; with splits_by_wave_efficiency 7 % and a factor of 2.3).  Many parts now run as
+  // 128-row CTAs, two per SM; measured again so on 60 such shapes with up to 25 counts each: 1.4 % off the best count on average, 14 % at most
+  // (1 x 114 x 7739, 8/2 heads of 128: 21 parts 19.9 us, 16 parts 17.5), and no call slower than before, so the terms are the same.
+  // (82 x 7511, 2 heads of 256: 1 part 125 us, 59 parts 33.5, 20 parts 24.7.)  A mask is not looked at.
   if (num_sms <= 0) num_sms = fa_host::sm_count();
   const int rows = head_dim > 128 ? 128 : 256;
   const int64_t ctas = (int64_t)batch * heads * ((seqlen_q + rows - 1) / rows);

@@ -617,7 +617,7 @@ __global__ void __launch_bounds__(Cfg<DH, NT>::THREADS, Cfg<DH, NT>::CTAS) fwd_t
             const int ik = iv + 1;              // ring index of K(j+1)
             const bool more = j + 1 < J_hi;
             ok = mbar_wait_w(bar_full(slot_of(iv)), par_of(iv), W_KVFULL, abort_flag);  // and K(j+1)
-            if (GROUPED && ok && j == j_tail) {  // V has landed: warp 11 clears its rows behind the last key
+            if (GROUPED && ok && j == j_tail) {  // V has landed: WARP_TAIL clears its rows behind the last key
               if (lane == 0) mbar_arrive(bar_vtail_go);
               ok = mbar_wait_w(bar_vtail, 0, W_VTAIL, abort_flag);
             }
