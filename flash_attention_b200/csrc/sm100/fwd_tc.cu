@@ -156,18 +156,22 @@ __global__ void __launch_bounds__(Cfg<DH, NT>::THREADS, Cfg<DH, NT>::CTAS) fwd_t
                         a.seqlen_k, a.use_mask_shift, a.mask_shift, b, GROUPED ? a.seqused_k_extra : 0);
   if (cache) si.sk = min(si.sk, a.seqlen_k);
   // heaviest blocks (largest row index under a causal mask) first; with split-KV the splits of a row block are neighbours
-  // (Shuffles as in cta_item, but for the plain instance of head dim 128, where it was 1 to 2 % faster to keep the block ranges in
-  // ordinary registers: 8 x 3072 tokens, 16 heads causal 326 us, 332 with.)
-  const int mrank = !GROUPED && DH == 128 ? (int)P.splits.div(item.block)
-                    : P.num_splits > 1    ? __shfl_sync(0xffffffffu, (int)P.splits.div(item.block), 0)
-                                          : item.block;
-  const int split = item.block - mrank * P.num_splits, mblk = P.row_blocks - 1 - mrank;
+  // (Shuffles as in cta_item, but where it was faster to keep the block ranges in ordinary registers: the plain instances of two tiles, whose
+  // warps compare every block against them, and of head dim 128.  1 x 2048 x 16384 tokens, 16 heads causal: 128 228.9 us, 240.2 with; 64 209.7,
+  // 213.8.  Trimmed, 8192 tokens: no mask, 80 433, 445 in ordinary registers.  One tile: the test of num_splits costs more than a multiplication,
+  // 16 x 2048 x 128 85.0, 85.4 with it.)
+  constexpr bool kPlainTwo = !GROUPED && NT == 2 && !TRIM;
+  const int mrank = kPlainTwo                 ? (P.num_splits > 1 ? (int)P.splits.div(item.block) : item.block)
+                    : !GROUPED && DH == 128 ? (int)P.splits.div(item.block)
+                    : P.num_splits > 1      ? __shfl_sync(0xffffffffu, (int)P.splits.div(item.block), 0)
+                                            : item.block;
+  const int split = kPlainTwo && P.num_splits <= 1 ? 0 : item.block - mrank * P.num_splits, mblk = P.row_blocks - 1 - mrank;
   const int m_base = mblk * NT * tile_pos;
   if (m_base >= si.sq) return;  // uniform for the CTA
 
   // per-tile key block ranges
-  const int blocks_per_split =
-      P.num_splits > 1 ? __shfl_sync(0xffffffffu, (int)P.splits.div((max(si.sk, 0) + kBN - 1) / kBN + P.num_splits - 1), 0) : 0;
+  auto part_blocks = [&] { return (int)P.splits.div((max(si.sk, 0) + kBN - 1) / kBN + P.num_splits - 1); };
+  const int blocks_per_split = kPlainTwo ? part_blocks() : P.num_splits > 1 ? __shfl_sync(0xffffffffu, part_blocks(), 0) : 0;
   if (GROUPED && P.num_splits > 1 && split * blocks_per_split * kBN >= si.sk) {
     // A part behind the last key (most of them where short sequences stand in a large cache) only says so: no barriers, no
     // tensor memory (32 sequences of 124 tokens in caches of 16384, 8/2 heads of 128, 5 parts: 17.9 -> 15.5 us).  Not in the
