@@ -752,10 +752,11 @@ static bool fwd_tc_takes(const FaFwdArgs& a, int64_t kv_batches) {
 // under the blocks of the other one, and no tile waits for the longer one beside it; but K and V are loaded for each tile, and nothing
 // keeps two CTAs' softmax phases apart: a pair of blocks takes 5 to 9 % longer.  So: few blocks per tile.  Measured, one tile / two
 // tiles, us, by key blocks of a tile on average:
-// causal, window or packed, tiles of one head: head dim 64 560 / 580 (12 blocks), 910 / 927 (16), 1030 / 1033 (20), 982 / 969 (24), 1673 / 1619
-// (32); 128 201 / 212 (6), 312 / 320 (8), 346 / 346 (10), 326 / 324 (12), 541 / 521 (16); 96 505 / 524 (16); window of 512, 16384 tokens 122 / 141;
-// packed 65536 tokens of 128 to 4096 845 / 898.  Where the tiles of a CTA end together anyway the line is lower: no mask, head dim 128 67 / 74 (3),
-// 92 / 93 (4), 113 / 114 (6), 146 / 139 (8), 64 75 / 81 (4), 94 / 100 (6), 124 / 123 (8), 196 / 189 (12); shared tiles (32/8 heads of 128, causal) 33 / 34
+// causal, window or packed, tiles of one head: head dim 64 40 / 42 (8 blocks), 166 / 172 (12), 66 / 63 (16), 124 / 119 (16), 982 / 969 (24),
+// 1673 / 1619 (32); 128 201 / 212 (6), 312 / 320 (8), 346 / 346 (10), 326 / 324 (12), 541 / 521 (16); 96 505 / 524 (16); window of 512, 16384 tokens
+// 122 / 141; packed 65536 tokens of 128 to 4096 845 / 898.  Where the tiles of a CTA end together anyway the line is lower: no mask, head dim 128 67 / 74 (3),
+// 92 / 93 (4), 113 / 114 (6), 146 / 139 (8), 64 75 / 81 (4), 94 / 100 (6), 124 / 123 (8), 196 / 189 (12), but where all CTAs
+// fit two to an SM, and not one, 128 11.5 / 11.4 (2), 16.4 / 15.0 (4), 64 9.6 / 9.8 (2), 13.9 / 12.8 (4); shared tiles (32/8 heads of 128, causal) 33 / 34
 // (3), 105 / 106 (4), 100 / 100 (6), 81 / 79 (8), 160 / 152 (12).
 // KV caches, of which only the capacity is known here, one tile against two, by blocks of a part.  Under 2.5 rounds of one-tile CTAs,
 // head dim 128 -15 to +3 % (4), -8 to +2 % (8), -2 to +5 % (12), -3 to +7 % (16), 64 with tiles of one head -12 to -6 % (8), -2 to +6 % (12),
@@ -767,7 +768,8 @@ static bool fwd_tc_takes(const FaFwdArgs& a, int64_t kv_batches) {
 static bool one_tile_form(int64_t ctas, int row_tiles, bool cache, bool uneven, int pack, int head_dim, double blocks, int num_sms) {
   const bool small = head_dim <= 64, even = row_tiles % 2 == 0;
   if (row_tiles <= 1) return ctas > num_sms || blocks <= (small ? 16.5 : 10.5);
-  if (!cache) return blocks <= (!uneven || pack > 1 ? 4.5 : small ? 16.5 : 8.5);
+  if (!cache && !uneven) return blocks <= (ctas > num_sms && ctas <= 2 * num_sms ? 2.5 : 4.5);
+  if (!cache) return blocks <= (pack > 1 ? 4.5 : small ? 14 : 8.5);
   if (ctas >= 5 * num_sms) return blocks <= (head_dim <= 96 ? 16.5 : 12.5);
   return blocks <= (small ? (!even ? 16.5 : pack == 1 ? 12.5 : 8.5) : head_dim <= 96 ? 16.5 : even ? 8.5 : 12.5);
 }

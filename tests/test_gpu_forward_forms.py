@@ -20,7 +20,7 @@ def _check(q, k, v, tiles, **kw):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("heads,heads_k", [(40, 40), (80, 10)])  # enough heads for one part; own tiles and shared ones
+@pytest.mark.parametrize("heads,heads_k", [(60, 60), (80, 10)])  # enough heads for one part; own tiles and shared ones
 @pytest.mark.parametrize("d", [8, 32, 48, 56, 64, 72, 80, 96, 104, 128])
 @pytest.mark.parametrize("sk,tiles", [(576, 1), (640, 2), (777, 2)])  # 4.5 blocks: the line without a mask
 def test_no_mask(d, heads, heads_k, sk, tiles, dtype):
@@ -28,8 +28,15 @@ def test_no_mask(d, heads, heads_k, sk, tiles, dtype):
     _check(q, k, v, tiles)
 
 
+@pytest.mark.parametrize("sk,tiles", [(320, 1), (321, 2)])  # 240 one-tile CTAs, two to an SM: 2.5 blocks
+@pytest.mark.parametrize("d", [64, 80, 128])
+def test_no_mask_two_to_an_sm(d, sk, tiles):
+    q, k, v, _ = make_qkv(2, 300, sk, 40, 40, d, torch.bfloat16, seed=d)
+    _check(q, k, v, tiles)
+
+
 @pytest.mark.parametrize("sq,sk,d,tiles,causal,window", [
-    (300, 2600, 64, 2, True, (-1, -1)), (300, 2600, 40, 2, True, (-1, -1)), (300, 2200, 64, 1, True, (-1, -1)), (300, 2200, 32, 1, True, (-1, -1)),
+    (300, 2600, 64, 2, True, (-1, -1)), (300, 2600, 40, 2, True, (-1, -1)), (300, 1900, 64, 1, True, (-1, -1)), (300, 1900, 32, 1, True, (-1, -1)), (300, 2000, 64, 2, True, (-1, -1)),
     (300, 2600, 64, 2, False, (2300, 0)), (300, 2600, 48, 2, False, (2200, 100)), (300, 2600, 64, 1, False, (1500, 0)),
     (300, 1400, 128, 2, True, (-1, -1)), (300, 1400, 80, 2, True, (-1, -1)), (300, 1200, 128, 1, True, (-1, -1)), (300, 1200, 96, 1, True, (-1, -1)),
     (300, 1400, 128, 2, False, (1000, 200)), (300, 1400, 72, 2, False, (1200, 0)), (300, 1400, 128, 1, False, (900, 0)),
