@@ -758,6 +758,9 @@ static bool fwd_tc_takes(const FaFwdArgs& a, int64_t kv_batches) {
 // 92 / 93 (4), 113 / 114 (6), 146 / 139 (8), 64 75 / 81 (4), 94 / 100 (6), 124 / 123 (8), 196 / 189 (12), but where all CTAs
 // fit two to an SM, and not one, 128 11.5 / 11.4 (2), 16.4 / 15.0 (4), 64 9.6 / 9.8 (2), 13.9 / 12.8 (4); shared tiles (32/8 heads of 128, causal) 33 / 34
 // (3), 105 / 106 (4), 100 / 100 (6), 81 / 79 (8), 160 / 152 (12).
+// A packed batch of very unequal lengths goes by the length its work belongs to (work_length): 16384 + 128 x 64 tokens causal, 16 heads of 128 2426
+// / 1749, 2 x 8192 + 64 x 128 868 / 702, 16/4 heads 879 / 689; lengths from 128 to 4096, where the tails are uneven, 486 / 520, and 16/4 heads, 8 x 2048
+// + 100 x 100 tokens, 322 / 277.
 // KV caches, of which only the capacity is known here, one tile against two, by blocks of a part.  Under 2.5 rounds of one-tile CTAs,
 // head dim 128 -15 to +3 % (4), -8 to +2 % (8), -2 to +5 % (12), -3 to +7 % (16), 64 with tiles of one head -12 to -6 % (8), -2 to +6 % (12),
 // with shared ones -3 to +5 % (8), +2 to +9 % (12); more rounds 128 -3 to +5 % (12), +1 to +7 % (16), 96 -1 to +5 % (16), 64 -6 to +2 % (16).  An odd
@@ -765,25 +768,35 @@ static bool fwd_tc_takes(const FaFwdArgs& a, int64_t kv_batches) {
 // Rows that fill one tile at most: two CTAs on an SM are 12 to 38 % faster than one after the other.  But a CTA that has its SM alone
 // gets nothing from sharing it and wants the longer ring of the two-tile form: head dim 128 -1 to +2 % (8), -2 to +14 % (12), +5 to +17 %
 // (16), +10 to +19 % (32), 64 -2 to +3 % (16), -2 to +4 % (32).
-static bool one_tile_form(int64_t ctas, int row_tiles, bool cache, bool uneven, int pack, int head_dim, double blocks, int num_sms) {
+static bool one_tile_form(int64_t ctas, int row_tiles, bool cache, bool uneven, bool skewed, int pack, int head_dim, double blocks, int num_sms) {
   const bool small = head_dim <= 64, even = row_tiles % 2 == 0;
   if (row_tiles <= 1) return ctas > num_sms || blocks <= (small ? 16.5 : 10.5);
   if (!cache && !uneven) return blocks <= (ctas > num_sms && ctas <= 2 * num_sms ? 2.5 : 4.5);
-  if (!cache) return blocks <= (pack > 1 ? 4.5 : small ? 14 : 8.5);
+  if (!cache) return blocks <= (pack > 1 ? (skewed ? 2.5 : 4.5) : small || skewed ? 14 : 8.5);
   if (ctas >= 5 * num_sms) return blocks <= (head_dim <= 96 ? 16.5 : 12.5);
   return blocks <= (small ? (!even ? 16.5 : pack == 1 ? 12.5 : 8.5) : head_dim <= 96 ? 16.5 : even ? 8.5 : 12.5);
+}
+// Length of the sequence that a row's work belongs to, on average over the work of a packed batch, from what the host knows: between the least
+// that one sequence of the maximum makes it and that maximum.  (16384 + 128 x 64 tokens: 13390, in truth 10965; 4 x 4096 + 32 x 256: 2189, 2816; evenly
+// from 128 to 4096: 3021, 2816.)
+static double work_length(double total, double batch, double longest) {
+  if (longest > total) longest = total;
+  if (batch <= 1 || longest * batch <= total) return total / batch;
+  const double rest = total - longest;
+  return sqrt((longest * longest + rest * rest / (batch - 1)) / total * longest);
 }
 static bool one_tile(const FaFwdArgs& a, int64_t kv_batches) {
   const int pack = pack_heads(a.heads / a.heads_k), parts = a.num_splits > 1 ? a.num_splits : 1;
   const bool varlen = a.cu_seqlens_q != nullptr;
-  const double sq = varlen ? (double)a.total_q / a.batch : a.seqlen_q, sk = varlen ? (double)a.total_k / a.batch : a.seqlen_k;
+  const double sq = varlen ? work_length(a.total_q, a.batch, a.seqlen_q) : a.seqlen_q, sk = varlen ? work_length(a.total_k, a.batch, a.seqlen_k) : a.seqlen_k;
   double keys = sk;  // of a row, on average
   if (a.window_right >= 0) keys = (sq <= sk ? sk - sq / 2 : sk * sk / (2 * sq)) + a.window_right;
   if (a.window_left >= 0 && keys > (double)a.window_left + a.window_right + 1) keys = (double)a.window_left + a.window_right + 1;
   if (keys > sk) keys = sk;
   const int pos = kBM / pack, row_tiles = (int)(((int64_t)a.seqlen_q + pos - 1) / pos);
   return one_tile_form((int64_t)a.batch * (a.heads / pack) * row_tiles * parts, row_tiles, kv_batches > 0,
-                       a.window_left >= 0 || a.window_right >= 0 || varlen, pack, a.head_dim, keys / kBN / parts, fa_host::sm_count());
+                       a.window_left >= 0 || a.window_right >= 0 || varlen, varlen && sk * a.batch > 1.2 * a.total_k, pack, a.head_dim,
+                       keys / kBN / parts, fa_host::sm_count());
 }
 
 static volatile int g_last_tiles = 0;
@@ -823,7 +836,7 @@ int fwd_tc_cache_splits(int batch, int heads, int heads_k, int seqlen_q, int cap
   double best_time = 0;
   for (int s = 1; s <= 128 && s <= (blocks > 1 ? blocks : 1); ++s) {
     const int per = (blocks + s - 1) / s;
-    const bool one = head_dim > 128 || one_tile_form((int64_t)batch * heads_k * (group / pack) * row_tiles * s, row_tiles, true, true, pack, head_dim,
+    const bool one = head_dim > 128 || one_tile_form((int64_t)batch * heads_k * (group / pack) * row_tiles * s, row_tiles, true, true, false, pack, head_dim,
                                                      (double)blocks / s, num_sms);
     const int64_t pos = (int64_t)tile_pos * (one ? 1 : 2);
     const double ctas = (double)batch * heads_k * (group / pack) * (double)((seqlen_q + pos - 1) / pos) * s;

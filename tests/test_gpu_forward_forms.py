@@ -74,3 +74,21 @@ def test_packed(heads, heads_k, d, tiles, lens_q, lens_k, causal):
         if lens_q[i]:
             ref, low = oracle_fwd_bwd(qs[i][None], ks[i][None], vs[i][None], None, causal=causal)
             assert_within(o[None], ref[0], low[0], what="sequence %d" % i)
+
+
+@pytest.mark.parametrize("heads,heads_k,d,tiles,lens", [
+    (4, 4, 64, 2, (4200, 60, 40, 33)), (4, 4, 64, 2, (33, 60, 4200, 1, 0)), (4, 4, 128, 2, (70, 4000, 200)), (4, 4, 80, 1, (2600, 60, 50, 40)), (8, 2, 128, 2, (900, 20, 30)),
+    (8, 2, 64, 1, (600, 500, 550)), (4, 4, 128, 1, (2600, 60, 50, 40)), (4, 4, 128, 2, (2300, 2300)),
+])
+def test_packed_unequal(heads, heads_k, d, tiles, lens):
+    """Few long sequences among short ones go by the long ones."""
+    g = torch.Generator().manual_seed(d)
+    q = torch.randn(sum(lens), heads, d, generator=g).half().cuda()
+    k, v = (torch.randn(sum(lens), heads_k, d, generator=g).half().cuda() for _ in range(2))
+    cu = torch.tensor([0, *lens], dtype=torch.int32).cumsum(0).int().cuda()
+    out = fa.flash_attn_varlen_func(q, k, v, cu, cu, max(lens), max(lens), causal=True)
+    assert _lib.last_path() == "fwd_tc" and _lib.last_forward_tiles() == tiles
+    for i, (o, qs, ks, vs) in enumerate(zip(out.split(lens), q.split(lens), k.split(lens), v.split(lens))):
+        if lens[i]:
+            ref, low = oracle_fwd_bwd(qs[None], ks[None], vs[None], None, causal=True)
+            assert_within(o[None], ref[0], low[0], what="sequence %d" % i)
