@@ -61,7 +61,7 @@ struct WCfg {
   static constexpr int OFF_STATS = OFF_B2 + NS2 * kTileB;  // per compute warp: 32 LSE + 32 D of the streamed columns
   static constexpr int STATS_BYTES = PASS == PASS_DQ ? 0 : 8 * 64 * 4;
   static constexpr int OFF_BAR = OFF_STATS + STATS_BYTES;
-  static constexpr int NBAR = 2 * NS1 + 2 * NS2 + 8;
+  static constexpr int NBAR = 2 * NS1 + 2 * NS2 + 9;
   static constexpr int SMEM_BYTES = OFF_BAR + NBAR * 8 + 32;
   static constexpr int COL_X1 = 0, COL_X2 = 64, COL_W = 128, COL_OUT = 256;  // W: two 32-column buffers
   static constexpr int TMEM_COLS = 512;
@@ -116,9 +116,12 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_wide_tc_kernel(const __grid_c
   auto bar_b2_full = [&](int st) { return bar0 + 8 * (2 * NS1 + st); };
   auto bar_b2_empty = [&](int st) { return bar0 + 8 * (2 * NS1 + NS2 + st); };
   constexpr int kB0 = 2 * NS1 + 2 * NS2;
-  const uint32_t bar_x1 = bar0 + 8 * kB0, bar_x1read = bar0 + 8 * (kB0 + 1), bar_a1 = bar0 + 8 * (kB0 + 2), bar_a2 = bar0 + 8 * (kB0 + 7),
-                 bar_x2 = bar0 + 8 * (kB0 + 3), bar_x2read = bar0 + 8 * (kB0 + 4), bar_w = bar0 + 8 * (kB0 + 5),
-                 bar_done = bar0 + 8 * (kB0 + 6);
+  const uint32_t bar_x1 = bar0 + 8 * kB0, bar_x1read = bar0 + 8 * (kB0 + 1), bar_a1 = bar0 + 8 * (kB0 + 2), bar_a2 = bar0 + 8 * (kB0 + 5),
+                 bar_x2 = bar0 + 8 * (kB0 + 3), bar_x2read = bar0 + 8 * (kB0 + 4), bar_done = bar0 + 8 * (kB0 + 6);
+  // One per buffer of W: the compute warps may hand over W(j+1) as soon as product j-1 is complete, which can be before the issuing warp
+  // looks for W(j).  With one barrier for both that phase would be over, its parity that of the next one, and every wait would give up.  The next
+  // phase of the same buffer needs product j, which is issued after the look.
+  auto bar_w = [&](int j) { return bar0 + 8 * (kB0 + 7 + (j & 1)); };
   volatile uint32_t* tmem_ptr_smem = reinterpret_cast<volatile uint32_t*>(smem + C::OFF_BAR + C::NBAR * 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + C::OFF_BAR + C::NBAR * 8 + 4);
 
@@ -172,7 +175,8 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_wide_tc_kernel(const __grid_c
     mbar_init(bar_a2, 1);
     mbar_init(bar_x2, 1);
     mbar_init(bar_x2read, 8);
-    mbar_init(bar_w, 8);
+    mbar_init(bar_w(0), 8);
+    mbar_init(bar_w(1), 8);
     mbar_init(bar_done, 1);
     fence_barrier_init();
     fence_proxy_async();
@@ -352,7 +356,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_wide_tc_kernel(const __grid_c
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(bar_w);
+      if (lane == 0) mbar_arrive(bar_w(it));
     }
     // ---- epilogue: the accumulator (times softmax_scale for dQ and dK) goes to its tensor
     if (ok && iters > 0) ok = mbar_wait(bar_done, 0, W_W_DONE, abort_flag);
@@ -527,7 +531,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_wide_tc_kernel(const __grid_c
               tc_commit_w(bar_x2);
               tc_commit_w(bar_b2_empty(n2));
             }
-            ok = mbar_wait_w(bar_w, j & 1, W_W_W, abort_flag);
+            ok = mbar_wait_w(bar_w(j), (j >> 1) & 1, W_W_W, abort_flag);
             if (ok && PASS == PASS_DV) ok = mbar_wait_w(bar_b2_full(j % NS2), (j / NS2) & 1, W_W_B_FULL, abort_flag);
             if (!ok) break;
             tc_fence_after();
