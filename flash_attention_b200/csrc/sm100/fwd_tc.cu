@@ -761,6 +761,10 @@ static bool fwd_tc_takes(const FaFwdArgs& a, int64_t kv_batches) {
 // A packed batch of very unequal lengths goes by the length its work belongs to (work_length): 16384 + 128 x 64 tokens causal, 16 heads of 128 2426
 // / 1749, 2 x 8192 + 64 x 128 868 / 702, 16/4 heads 879 / 689; lengths from 128 to 4096, where the tails are uneven, 486 / 520, and 16/4 heads, 8 x 2048
 // + 100 x 100 tokens, 322 / 277.
+// Rows that are not whole 32-byte sectors (head dims 72, 88, 104, 120) make loads dearer, and one tile loads K and V twice: causal 88 98 / 93 (8),
+// 104 77 / 71 (6), 196 / 172 (8), 26.3 / 24.4 (4), 120 67 / 62 (6), with shared tiles 104 36 / 32 (4); no mask 32 / 29 (4), 72 29 / 27 (4); two to an
+// SM 104 13.6 / 11.5 (2), 40 11.8 / 10.3 (2); caches 104 -3 to +1 % (4), +1 to +16 % (8), shared tiles +1 to +13 % (4); rows that fill one tile, an SM each,
+// 104 +2 to +8 % (4), +8 to +12 % (6).
 // KV caches, of which only the capacity is known here, one tile against two, by blocks of a part.  Under 2.5 rounds of one-tile CTAs,
 // head dim 128 -15 to +3 % (4), -8 to +2 % (8), -2 to +5 % (12), -3 to +7 % (16), 64 with tiles of one head -12 to -6 % (8), -2 to +6 % (12),
 // with shared ones -3 to +5 % (8), +2 to +9 % (12); more rounds 128 -3 to +5 % (12), +1 to +7 % (16), 96 -1 to +5 % (16), 64 -6 to +2 % (16).  An odd
@@ -769,9 +773,10 @@ static bool fwd_tc_takes(const FaFwdArgs& a, int64_t kv_batches) {
 // gets nothing from sharing it and wants the longer ring of the two-tile form: head dim 128 -1 to +2 % (8), -2 to +14 % (12), +5 to +17 %
 // (16), +10 to +19 % (32), 64 -2 to +3 % (16), -2 to +4 % (32).
 static bool one_tile_form(int64_t ctas, int row_tiles, bool cache, bool uneven, bool skewed, int pack, int head_dim, double blocks, int num_sms) {
-  const bool small = head_dim <= 64, even = row_tiles % 2 == 0;
-  if (row_tiles <= 1) return ctas > num_sms || blocks <= (small ? 16.5 : 10.5);
-  if (!cache && !uneven) return blocks <= (ctas > num_sms && ctas <= 2 * num_sms ? 2.5 : 4.5);
+  const bool small = head_dim <= 64, even = row_tiles % 2 == 0, cut = head_dim % 16 != 0;
+  if (row_tiles <= 1) return ctas > num_sms || blocks <= (small ? 16.5 : cut ? 3.5 : 10.5);
+  if (!cache && !uneven) return blocks <= (ctas > num_sms && ctas <= 2 * num_sms ? (cut ? 1.5 : 2.5) : cut && !small ? 2.5 : 4.5);
+  if (cut && !small) return blocks <= (pack > 1 ? 2.5 : 5.5);
   if (!cache) return blocks <= (pack > 1 ? (skewed ? 2.5 : 4.5) : small || skewed ? 14 : 8.5);
   if (ctas >= 5 * num_sms) return blocks <= (head_dim <= 96 ? 16.5 : 12.5);
   return blocks <= (small ? (!even ? 16.5 : pack == 1 ? 12.5 : 8.5) : head_dim <= 96 ? 16.5 : even ? 8.5 : 12.5);

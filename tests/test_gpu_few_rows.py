@@ -16,7 +16,7 @@ if torch.cuda.is_available():
 @pytest.mark.parametrize("batch,sq,heads,heads_k,d,parts,sk,tiles", [
     (4, 18, 16, 8, 96, 4, 8300, 2), (4, 18, 16, 8, 96, 9, 10240, 1), (4, 18, 16, 8, 128, 4, 5000, 1), (1, 128, 8, 8, 128, 12, 17000, 2),
     (2, 31, 8, 4, 128, 1, 1409, 2), (2, 31, 8, 4, 128, 1, 1280, 1), (2, 31, 8, 4, 80, 3, 4300, 2), (1, 20, 4, 2, 64, 2, 4500, 2),
-    (1, 20, 4, 2, 40, 2, 4500, 2), (1, 20, 4, 2, 64, 2, 4000, 1), (1, 128, 2, 2, 128, 1, 1, 1), (2, 33, 6, 6, 192, 2, 5000, 1),
+    (1, 20, 4, 2, 40, 2, 4500, 2), (1, 20, 4, 2, 64, 2, 4000, 1), (1, 128, 2, 2, 128, 1, 1, 1), (2, 31, 8, 4, 88, 2, 1100, 2), (2, 31, 8, 4, 104, 2, 896, 1), (2, 33, 6, 6, 192, 2, 5000, 1),
 ])
 @pytest.mark.parametrize("causal", [False, True])
 def test_parts(batch, sq, heads, heads_k, d, parts, sk, tiles, causal, monkeypatch):
@@ -33,7 +33,7 @@ def test_parts(batch, sq, heads, heads_k, d, parts, sk, tiles, causal, monkeypat
 @pytest.mark.parametrize("batch,new,heads,heads_k,d,parts,cap,tiles", [
     (4, 40, 8, 8, 128, 1, 1400, 2), (4, 40, 8, 8, 128, 1, 1280, 1), (40, 40, 8, 8, 128, 1, 1400, 1), (4, 40, 4, 4, 64, 1, 2200, 2),
     (2, 129, 8, 8, 128, 1, 1250, 2), (2, 129, 8, 8, 128, 1, 1000, 1), (2, 120, 8, 2, 64, 2, 2300, 2), (2, 140, 4, 4, 64, 2, 2300, 1),
-    (2, 140, 4, 4, 96, 1, 2300, 2), (2, 140, 4, 4, 96, 2, 3000, 1), (2, 300, 8, 8, 128, 1, 1500, 1), (2, 300, 8, 8, 128, 1, 1900, 2),
+    (2, 140, 4, 4, 96, 1, 2300, 2), (2, 140, 4, 4, 96, 2, 3000, 1), (2, 300, 8, 8, 128, 1, 1500, 1), (2, 300, 8, 8, 128, 1, 1900, 2), (2, 140, 4, 4, 104, 1, 900, 2), (2, 140, 4, 4, 72, 1, 700, 1), (2, 140, 8, 2, 120, 1, 500, 2),
 ])
 @pytest.mark.parametrize("page", [0, 64])
 def test_cache(batch, new, heads, heads_k, d, parts, cap, tiles, page):

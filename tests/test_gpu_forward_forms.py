@@ -22,8 +22,9 @@ def _check(q, k, v, tiles, **kw):
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("heads,heads_k", [(60, 60), (80, 10)])  # enough heads for one part; own tiles and shared ones
 @pytest.mark.parametrize("d", [8, 32, 48, 56, 64, 72, 80, 96, 104, 128])
-@pytest.mark.parametrize("sk,tiles", [(576, 1), (640, 2), (777, 2)])  # 4.5 blocks: the line without a mask
-def test_no_mask(d, heads, heads_k, sk, tiles, dtype):
+@pytest.mark.parametrize("blocks,more", [(4.5, 0), (4.5, 1), (4.5, 200)])  # the line without a mask; 2.5 where rows are not whole sectors
+def test_no_mask(d, heads, heads_k, blocks, more, dtype):
+    sk, tiles = int((2.5 if d in (72, 104) else blocks) * 128) + more, 2 if more else 1
     q, k, v, _ = make_qkv(2, 300, sk, heads, heads_k, d, dtype, seed=d)
     _check(q, k, v, tiles)
 
@@ -40,6 +41,7 @@ def test_no_mask_two_to_an_sm(d, sk, tiles):
     (300, 2600, 64, 2, False, (2300, 0)), (300, 2600, 48, 2, False, (2200, 100)), (300, 2600, 64, 1, False, (1500, 0)),
     (300, 1400, 128, 2, True, (-1, -1)), (300, 1400, 80, 2, True, (-1, -1)), (300, 1200, 128, 1, True, (-1, -1)), (300, 1200, 96, 1, True, (-1, -1)),
     (300, 1400, 128, 2, False, (1000, 200)), (300, 1400, 72, 2, False, (1200, 0)), (300, 1400, 128, 1, False, (900, 0)),
+    (300, 900, 104, 2, True, (-1, -1)), (300, 800, 88, 1, True, (-1, -1)), (300, 900, 120, 2, False, (700, 20)), (300, 900, 112, 1, True, (-1, -1)),
     (1111, 2500, 96, 2, True, (-1, -1)), (257, 4100, 56, 2, True, (-1, -1)),
 ])
 def test_masked(sq, sk, d, tiles, causal, window):
