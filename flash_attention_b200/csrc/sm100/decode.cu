@@ -349,20 +349,21 @@ __global__ void __launch_bounds__(160, 2) decode_kernel(const __grid_constant__ 
     pa[2] = Pack<T>::two(s[1][0], s[1][1]);
     pa[3] = Pack<T>::two(s[1][2], s[1][3]);
     const int vrow = warp * 16 + (lane & 7) + ((lane >> 3) & 1) * 8;
-    uint32_t seen = 0;
 #pragma unroll
     for (int dt = 0; dt < D / 16; ++dt) {
       uint32_t bb[4];
       const int c16 = (dt * 2 + (lane >> 4)) & 7;
       ldsm_x4_t(bb, swz(sV + (dt / 4) * C::BOX_BYTES, vrow, c16));
-      seen ^= bb[3];
       mma16816<T>(o_acc[2 * dt], pa, bb[0], bb[1]);
       mma16816<T>(o_acc[2 * dt + 1], pa, bb[2], bb[3]);
     }
     __syncwarp();
-    // The slot is given back once the last pieces of V are in registers: the address of the arrival depends on them.  Without that the
+    // The slot is given back once all of V has gone into the products: the address of the arrival depends on each.  Without that the
     // last ldmatrix of a tile could still be on its way when the next tile landed (45 sequences of 640 to 2560 keys, 16/4 heads of 64, two
     // tokens: the last 16 columns of one KV head's rows were wrong in one call of 20 to 60).
+    uint32_t seen = 0;
+#pragma unroll
+    for (int dt = 0; dt < D / 16; ++dt) seen |= __float_as_uint(o_acc[2 * dt + 1][0]);
     if (lane == 0) mbar_arrive(bar_empty(slot) + (seen & P.zero));
   }
 
